@@ -238,7 +238,7 @@ def _stage_kernels(cfg):
     """The kernel that does the work of each timed stage for a launch config."""
     return {
         "day_shadow_kernel": "day_sweep_tma_kernel" if cfg.sweep_window else "day_shadow_kernel",
-        "day_gvf_kernel": "day_gvf_hv_kernel" if cfg.gvf_hours == 1 else "day_gvf_kernel",
+        "day_gvf_kernel": "day_gvf_walk_kernel" if cfg.gvf_hours == 1 else "day_gvf_kernel",
         "day_tables_kernel": "day_tables_kernel",
         "patch_gemm_kernel": "patch_gemm_pipe_kernel",  # the combined sums of <= 24 hours
         "day_radiation_kernel": "day_radiation_kernel",

@@ -93,11 +93,14 @@ typedef struct SolweigScene {
        value of the three rasters is exactly representable in float32 (the
        hourly shadow sweep then loads one 16-byte sample per step); NULL otherwise */
     const void* geo32;
-    /* optional statics of the batched day's hour-vectorized GVF (1 m walk, no
-       water), from solweig_gvf_statics: walk-length codes [4][pixels] and the
-       albedo-without-shadow GVF [pixels]; NULL: the day walks them itself */
+    /* optional statics of the ground view factors (first 1, second 2 to 22, no
+       water), from solweig_gvf_walks: walk-length codes [4][pixels], the
+       albedo-without-shadow GVF [pixels] and (16-byte aligned) the walk words
+       of the batched day; a day without gvf_nosh or gvf_walks prepares them in
+       its work buffer */
     const uint32_t* gvf_hits;
     const float* gvf_nosh;
+    const uint32_t* gvf_walks;
 } SolweigScene;
 
 /* Per-patch constants of the sky-vault layout (host arrays, copied per call). */
@@ -412,14 +415,23 @@ int solweig_day_batched_timed(const SolweigScene* scene, const SolweigSkyLayout*
                               const int32_t* gvf_dxdy, int first_steps, int second_steps,
                               void* work, int64_t work_bytes, const SolweigDayConfig* config,
                               void* stream, float* stage_ms);
-/* The scene statics of the batched day's hour-vectorized GVF (no
- * counterpart in the reference): for the 1 m walk (first_steps 1,
- * second_steps 22) of a scene without water, the walk length of every GVF
- * direction (the first building step; device uint32 [4][pixels], 5
- * directions of 6 bits per word) and the albedo-without-shadow GVF (device
- * float32 [pixels]), which depend only on the ground bits and the albedo.
- * Set scene->gvf_hits / gvf_nosh to them and every later day skips that
- * walk; the results are identical. */
+/* The scene statics of the ground view factors (no counterpart in the
+ * reference): for walks of 2 to 22 steps with first_steps 1 in a scene without
+ * water, what depends only on the ground bits, the walls and the albedo.
+ *   walks  device uint32 [words], 16-byte aligned, words at least
+ *          solweig_gvf_walk_words(rows, cols): per (pixel, direction) the wall
+ *          pixels met, the samples read, whether the last one repeats to the
+ *          end (the walk left the raster) and whether the pixel's own wall
+ *          faces away, in the batched day's tile order
+ *   hits   device uint32 [4][pixels] or NULL: samples read (5 bits) and the
+ *          repeat flag, 5 directions of 6 bits per word
+ *   nosh   device float32 [pixels]: albedo-without-shadow GVF
+ * Set scene->gvf_walks / gvf_nosh to them and every later day skips that walk;
+ * the results are identical.  solweig_gvf_statics gives hits and nosh alone,
+ * for the 1 m walk (second_steps 22). */
+int64_t solweig_gvf_walk_words(int rows, int cols);
+int solweig_gvf_walks(const SolweigScene* scene, const int32_t* gvf_dxdy, int first_steps, int second_steps,
+                      uint32_t* hits, uint32_t* walks, int64_t words, float* nosh, void* stream);
 int solweig_gvf_statics(const SolweigScene* scene, const int32_t* gvf_dxdy, int first_steps, int second_steps,
                         uint32_t* hits, float* nosh, void* stream);
 /* Byte offsets inside the batched-day work buffer: quads [H][px] float4,

@@ -135,12 +135,14 @@ def day_launches(scene, config, sweep_parts=1):
     """Kernel launches of one batched day for this scene and launch shapes,
     with the sweep stage issued in ``sweep_parts`` hour ranges: per range the
     ray exits, the ceilings and the sweep; once the height dilation (and the
-    tile maxima of the window sweep); then the GVF (the hour-vectorized
-    kernel or the per-hour one), weights, two splits (sky and vegetation
+    tile maxima of the window sweep); then the GVF (sample codes and the walk
+    kernel, or the per-hour kernel), weights, two splits (sky and vegetation
     weights), tables, contraction and radiation."""
     c = int(not config.no_ceiling)
+    walk = int(config.gvf_hours == 1 and scene.first_steps == 1 and 2 <= scene.second_steps <= 22
+               and not scene.struct.has_water)
     win = int(config.sweep_window != 0 and scene.geo32 is not None and not scene.struct.has_water)
-    return sweep_parts * (2 + c) + c + win + 7
+    return sweep_parts * (2 + c) + c + win + walk + 7
 
 
 class ChosenDay(BatchedDay):

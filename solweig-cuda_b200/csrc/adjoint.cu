@@ -671,9 +671,10 @@ struct GradWork {
     long long total;
 };
 
-GradWork grad_work_layout(long long px, int nhours) {
+GradWork grad_work_layout(int rows, int cols, int nhours) {
     GradWork g{};
-    const DayWork d = day_work_layout(px, nhours, false);
+    const long long px = (long long)rows * cols;
+    const DayWork d = day_work_layout(rows, cols, nhours, false);
     long long o = d.total;
     g.day_total = d.total;
     g.quads1 = o; o = align256(o + 16LL * px * nhours);
@@ -699,7 +700,7 @@ using namespace solweig;
 
 extern "C" int64_t solweig_day_grad_work_bytes(int rows, int cols, int nhours) {
     if (rows <= 0 || cols <= 0 || nhours <= 0) return 0;
-    return grad_work_layout((long long)rows * cols, nhours).total;
+    return grad_work_layout(rows, cols, nhours).total;
 }
 
 // Shared forward of the gradient entry points: masks, parameter quads, GVF,
@@ -718,8 +719,8 @@ static int grad_prepare(const SolweigScene* scene, const SolweigSkyLayout* layou
     SOLWEIG_CHECK_ARG(first_steps == 1 && second_steps == 22 && gvf_dxdy,
                       "solweig_day_grad: only the 1 m GVF walk (first=1, second=22)");
     const long long px = (long long)S.rows * S.cols;
-    gw = grad_work_layout(px, nhours);
-    dw = day_work_layout(px, nhours, false);
+    gw = grad_work_layout(S.rows, S.cols, nhours);
+    dw = day_work_layout(S.rows, S.cols, nhours, false);
     SOLWEIG_CHECK_ARG(work_bytes >= gw.total, "solweig_day_grad: work buffer of %lld bytes, need %lld",
                       (long long)work_bytes, gw.total);
     SOLWEIG_CHECK_ARG(((uintptr_t)work & 255) == 0, "solweig_day_grad: work buffer not 256-byte aligned");

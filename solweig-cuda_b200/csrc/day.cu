@@ -13,12 +13,13 @@
 //                           (day_sweep_tma_kernel with sweep_window = 1 / 2:
 //                           the same sweep on TMA-staged shared-memory windows
 //                           with the warp-vote exit, sweep_tma.cuh)
-//  2 day_gvf_hv_kernel      32 x 32 tiles, every daytime hour per block (4 per
-//                           shared-memory pass): all-direction GVF (Lup,
-//                           albedo) + the pixel's shadow, the hour-independent
-//                           albedo-without-shadow GVF once per day
-//                           (day_gvf_kernel, grid.z = hour, for other walk
-//                           lengths and water scenes)
+//  2 gvf_codes_kernel,      the tiles' distinct samples, then
+//    day_gvf_walk_kernel    32 x 32 tiles, four daytime hours per
+//                           block along the scene's walk words:
+//                           all-direction GVF (Lup, albedo) + the pixel's
+//                           shadow, the hour-independent albedo-without-shadow
+//                           GVF once per day (day_gvf_kernel, grid.z = hour,
+//                           for walks of more than 22 steps and water scenes)
 //  3 day_weights_kernel     per-hour patch weights (luminance, luminance*cos*omega)
 //  4 split_bf16_kernel      weights (and 0.03 x the weights) -> BF16 hi/lo
 //                           pairs in the canonical K-major shared-memory
@@ -53,17 +54,49 @@ using namespace solweig;
 
 extern "C" int64_t solweig_day_batched_work_bytes(int rows, int cols, int nhours, int has_water) {
     if (rows <= 0 || cols <= 0 || nhours <= 0) return 0;
-    return day_work_layout((long long)rows * cols, nhours, has_water != 0).total;
+    return day_work_layout(rows, cols, nhours, has_water != 0).total;
 }
 
 extern "C" int solweig_day_batched_layout(int rows, int cols, int nhours, int has_water, int64_t* offsets) {
     SOLWEIG_CHECK_ARG(offsets && rows > 0 && cols > 0 && nhours > 0, "solweig_day_batched_layout: bad arguments");
-    const DayWork w = day_work_layout((long long)rows * cols, nhours, has_water != 0);
+    const DayWork w = day_work_layout(rows, cols, nhours, has_water != 0);
     const long long v[11] = {w.quads, w.lup_first, w.gvf, w.nosh, w.sums, w.wf32, w.bw, w.tables, w.error,
                              w.tilemax, w.total};
     for (int i = 0; i < 11; ++i) offsets[i] = v[i];
     return SOLWEIG_OK;
 }
+
+namespace {
+
+int launch_gvf_walks(const SolweigScene& S, const int32_t* gvf_dxdy, int second, uint32_t* hits, uint32_t* walks,
+                     float* nosh, cudaStream_t st) {
+    GvfTable<kWkMaxSteps> tab;
+    fill_day_table(tab, gvf_dxdy, second, kWkMaxWidth);
+    const size_t smem = gvf_walks_smem_bytes();
+    set_smem_attr((const void*)gvf_walks_kernel, smem);
+    dim3 grid(blocks_for(S.cols, kWkTile), blocks_for(S.rows, kWkTile));
+    gvf_walks_kernel<<<grid, kWkPixels, smem, st>>>(S, second, tab, hits, walks, nosh);
+    SOLWEIG_CHECK_LAUNCH("gvf_walks_kernel");
+    return SOLWEIG_OK;
+}
+
+// Shared by the two entry points: `second` of solweig_gvf_statics is fixed.
+int gvf_scene_walks(const char* name, const SolweigScene* scene, const int32_t* gvf_dxdy, int second, uint32_t* hits,
+                    uint32_t* walks, float* nosh, void* stream) {
+    SOLWEIG_CHECK_ARG(!scene->has_water, "%s: scenes with water walk per hour", name);
+    SOLWEIG_CHECK_ARG(scene->rows > 0 && scene->cols > 0 && scene->flags && scene->alb && scene->walls &&
+                          scene->gvf_face,
+                      "%s: bad scene", name);
+    for (int j = 0; j < SOLWEIG_GVF_DIRECTIONS; ++j)
+        for (int m = 0; m < second; ++m) {
+            const int32_t* o = gvf_dxdy + 2 * (j * second + m);
+            SOLWEIG_CHECK_ARG(o[0] >= -m && o[0] <= m && o[1] >= -m && o[1] <= m,
+                              "%s: GVF offset (%d, %d) at step %d", name, o[0], o[1], m);
+        }
+    return launch_gvf_walks(*scene, gvf_dxdy, second, hits, walks, nosh, as_stream(stream));
+}
+
+}  // namespace
 
 extern "C" int solweig_gvf_statics(const SolweigScene* scene, const int32_t* gvf_dxdy, int first_steps,
                                    int second_steps, uint32_t* hits, float* nosh, void* stream) {
@@ -71,19 +104,24 @@ extern "C" int solweig_gvf_statics(const SolweigScene* scene, const int32_t* gvf
     SOLWEIG_CHECK_ARG(first_steps == 1 && second_steps == 22,
                       "solweig_gvf_statics: only the 1 m walk (first 1, second 22), not %d/%d", first_steps,
                       second_steps);
-    SOLWEIG_CHECK_ARG(!scene->has_water, "solweig_gvf_statics: scenes with water walk per hour");
-    SOLWEIG_CHECK_ARG(scene->rows > 0 && scene->cols > 0 && scene->flags && scene->alb,
-                      "solweig_gvf_statics: bad scene");
-    const SolweigScene& S = *scene;
-    GvfTable<22> tab;
-    fill_day_table(tab, gvf_dxdy, 22, kHvPitch);
-    cudaStream_t st = as_stream(stream);
-    const size_t smem = gvf_statics_smem_bytes();
-    set_smem_attr((const void*)gvf_statics_kernel, smem);
-    dim3 grid(blocks_for(S.cols, kHvTile), blocks_for(S.rows, kHvTile));
-    gvf_statics_kernel<<<grid, dim3(kHvTile, kHvTile), smem, st>>>(S, tab, hits, nosh);
-    SOLWEIG_CHECK_LAUNCH("gvf_statics_kernel");
-    return SOLWEIG_OK;
+    return gvf_scene_walks("solweig_gvf_statics", scene, gvf_dxdy, second_steps, hits, nullptr, nosh, stream);
+}
+
+extern "C" int64_t solweig_gvf_walk_words(int rows, int cols) {
+    return rows > 0 && cols > 0 ? walk_words(rows, cols) : 0;
+}
+
+extern "C" int solweig_gvf_walks(const SolweigScene* scene, const int32_t* gvf_dxdy, int first_steps,
+                                 int second_steps, uint32_t* hits, uint32_t* walks, int64_t words, float* nosh,
+                                 void* stream) {
+    SOLWEIG_CHECK_ARG(scene && gvf_dxdy && walks && nosh, "solweig_gvf_walks: null argument");
+    SOLWEIG_CHECK_ARG(first_steps == 1 && second_steps >= 2 && second_steps <= kWkMaxSteps,
+                      "solweig_gvf_walks: walks of 2 to %d steps with first 1, not %d/%d", kWkMaxSteps, first_steps,
+                      second_steps);
+    SOLWEIG_CHECK_ARG(words >= walk_words(scene->rows, scene->cols), "solweig_gvf_walks: %lld words, need %lld",
+                      (long long)words, walk_words(scene->rows, scene->cols));
+    SOLWEIG_CHECK_ARG(((uintptr_t)walks & 15) == 0, "solweig_gvf_walks: walk words not 16-byte aligned");
+    return gvf_scene_walks("solweig_gvf_walks", scene, gvf_dxdy, second_steps, hits, walks, nosh, stream);
 }
 
 extern "C" int solweig_patch_sums(const uint32_t* masks, int64_t pixels, int patches, const float* weights,
@@ -150,7 +188,7 @@ int day_batched_impl(const SolweigScene* scene, const SolweigSkyLayout* layout, 
                           first_steps >= 1 && first_steps <= second_steps,
                       "solweig_day_batched: GVF steps first=%d second=%d", first_steps, second_steps);
     const long long px = (long long)S.rows * S.cols;
-    const DayWork w = day_work_layout(px, nhours, S.has_water != 0);
+    const DayWork w = day_work_layout(S.rows, S.cols, nhours, S.has_water != 0);
     SOLWEIG_CHECK_ARG(work_bytes >= w.total, "solweig_day_batched: work buffer of %lld bytes, need %lld",
                       (long long)work_bytes, w.total);
     SOLWEIG_CHECK_ARG(((uintptr_t)work & 255) == 0, "solweig_day_batched: work buffer not 256-byte aligned");
@@ -268,21 +306,46 @@ int day_batched_impl(const SolweigScene* scene, const SolweigSkyLayout* layout, 
         return SOLWEIG_OK;
     }
     // kDayRest (the error flag was cleared by the sweep part of hour 0)
-    cudaMemsetAsync(nosh, 0, 4 * px, st);
-    if (first_steps == 1 && second_steps == 22) {
+    DayWalkArgs wa;
+    wa.second = second_steps;
+    wa.halo = second_steps - 1;
+    wa.width = kWkTile + 2 * wa.halo;
+    // The walk-word kernel: walks of 2 to 22 steps from the pixel itself (pixels
+    // of 0.98 m and more), no water (whose first direction reads another Lup);
+    // the per-hour kernel takes the rest (0.996 against 0.202 ms per 517 x 389
+    // px day at 2 m).
+    if (cfg.gvf_hours == 1 && !S.has_water && first_steps == 1 && second_steps >= 2 && second_steps <= kWkMaxSteps &&
+        walk_offsets(gvf_dxdy, second_steps, wa.width, &wa.at)) {
+        uint32_t* walks = reinterpret_cast<uint32_t*>(wb + w.walks);
+        const bool statics = S.gvf_walks && S.gvf_nosh && ((uintptr_t)S.gvf_walks & 15) == 0;
+        if (!statics) {
+            const int rc = launch_gvf_walks(S, gvf_dxdy, second_steps, nullptr, walks, nosh, st);
+            if (rc) return rc;
+        }
+        wa.magic = (uint32_t)((0x100000000ull + wa.width - 1) / wa.width);
+        wa.walks = statics ? S.gvf_walks : walks;
+        // the samples' codes (4 B per pixel and pass) and the tiles' values live
+        // in the patch-sum region (16 B per pixel-hour), free until the contraction
+        const int passes = (nhours + kWkHours - 1) / kWkHours;
+        uint32_t* codes = reinterpret_cast<uint32_t*>(sums);
+        unsigned long long* dict = reinterpret_cast<unsigned long long*>(wb + w.dict);
+        wa.codes = codes;
+        wa.dict = dict;
+        const dim3 grid(blocks_for(S.cols, kWkTile), blocks_for(S.rows, kWkTile), passes);
+        gvf_codes_kernel<<<grid, kWkCodeThreads, 0, st>>>(
+            S.rows, S.cols, hours, nhours, quads, codes, dict, gvf, statics ? S.gvf_nosh : nullptr, nosh);
+        SOLWEIG_CHECK_LAUNCH("gvf_codes_kernel");
+        const size_t smem = day_walk_smem_bytes(wa.width);
+        set_smem_attr((const void*)day_gvf_walk_kernel, smem);
+        day_gvf_walk_kernel<<<grid, kWkThreads, smem, st>>>(S, hours, nhours, wa, quads, gvf);
+        SOLWEIG_CHECK_LAUNCH("day_gvf_walk_kernel");
+    } else if (first_steps == 1 && second_steps == 22) {
+        cudaMemsetAsync(nosh, 0, 4 * px, st);
         GvfTable<22> tab;
         fill_day_table(tab, gvf_dxdy, 22, pitch);
-        const bool hv = cfg.gvf_hours == 1 && !S.has_water;
-        if (!hv) {
-            launch_day_gvf<1, 22, 22>(cfg.gvf_rows, S, hours, nhours, ga, tab, quads, lup_first, gvf, nosh, st);
-        } else {
-            const size_t smem = hv_smem_bytes();
-            set_smem_attr((const void*)day_gvf_hv_kernel, smem);
-            dim3 grid(blocks_for(S.cols, kHvTile), blocks_for(S.rows, kHvTile));
-            day_gvf_hv_kernel<<<grid, dim3(kHvTile, kHvTile), smem, st>>>(S, hours, nhours, tab, quads, gvf, nosh);
-            SOLWEIG_CHECK_LAUNCH("day_gvf_hv_kernel");
-        }
+        launch_day_gvf<1, 22, 22>(cfg.gvf_rows, S, hours, nhours, ga, tab, quads, lup_first, gvf, nosh, st);
     } else {
+        cudaMemsetAsync(nosh, 0, 4 * px, st);
         GvfTable<SOLWEIG_GVF_MAX_STEPS> tab;
         fill_day_table(tab, gvf_dxdy, second_steps, pitch);
         launch_day_gvf<0, 0, SOLWEIG_GVF_MAX_STEPS>(cfg.gvf_rows, S, hours, nhours, ga, tab, quads, lup_first, gvf,
@@ -411,7 +474,7 @@ extern "C" int solweig_day_batched_timed(const SolweigScene* scene, const Solwei
 extern "C" int solweig_day_batched_error(const void* work, int rows, int cols, int nhours, int has_water,
                                          int* out_device, void* stream) {
     SOLWEIG_CHECK_ARG(work && out_device, "solweig_day_batched_error: null argument");
-    const DayWork w = day_work_layout((long long)rows * cols, nhours, has_water != 0);
+    const DayWork w = day_work_layout(rows, cols, nhours, has_water != 0);
     cudaMemcpyAsync(out_device, static_cast<const char*>(work) + w.error, sizeof(int), cudaMemcpyDeviceToDevice,
                     as_stream(stream));
     return SOLWEIG_OK;

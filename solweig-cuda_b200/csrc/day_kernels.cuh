@@ -5,7 +5,7 @@
 #include <cuda_bf16.h>
 
 #include "ceiling.cuh"
-#include "gvf_fields.cuh"
+#include "gvf_walk.cuh"
 #include "hour.cuh"
 #include "radiation.cuh"
 #include "sweep_tma.cuh"
@@ -259,16 +259,6 @@ struct DayGvfArgs {
     int first, second, halo;
 };
 
-// Tiles of the hour-vectorized GVF kernel: 32 x 32 pixels, halo 21 (the 1 m
-// walk, second = 22).  A tile is interior when its halo lies inside the raster.
-constexpr int kHvTile = 32, kHvHalo = 21, kHvPitch = kHvTile + 2 * kHvHalo;
-static_assert(kHvTile == 32, "the hour-vectorized GVF maps its 32 warps to 8 x 4 pieces of a 32 x 32 tile");
-
-__host__ __device__ __forceinline__ bool hv_tile_interior(int rows, int cols, int tr, int tc) {
-    const int row0 = tr * kHvTile - kHvHalo, col0 = tc * kHvTile - kHvHalo;
-    return row0 >= 0 && col0 >= 0 && row0 + kHvPitch <= rows && col0 + kHvPitch <= cols;
-}
-
 // gvf[z][0] = Lup GVF (ambient added), gvf[z][1] = albedo GVF, gvf[z][2] = shadow.
 // nosh = albedo-without-shadow GVF: the same for every hour (walk geometry and
 // albedo only), so every daytime launch writes the same values.
@@ -352,334 +342,6 @@ __global__ void __launch_bounds__(32 * TY) day_gvf_kernel(SolweigScene S, const 
     gvf[(3 * z + 1) * n + p] = alb / 18.f;
     gvf[(3 * z + 2) * n + p] = own.x;
     nosh[p] = nsh / 18.f;
-}
-
-// Hour-vectorized GVF for interior 32 x 32 tiles (the 1 m walk: first = 1,
-// second = 22), all daytime hours of the day in one block.  The walk length
-// of every direction (first building step) and the albedo-without-shadow
-// plane depend only on the ground bits and the albedo, so they are computed
-// once; then per pass of kHvCh daytime hours the tile is staged as
-// (Lup, albedo*shadow) pairs plus the sunlit-wall bits of those hours, and
-// every walked sample is one pair of 16-byte shared loads serving all kHvCh
-// hours.  The sunlit-wall statistics need only the first step at which each
-// hour's bit appears: seen at step f < hit means n_sun = second - f (the
-// steps after a building hit keep counting, as in gvf_direction_fixed).
-// Same recurrences as gvf_direction_fixed and the same float32 sums along
-// the walk, except albedo*shadow, which is rounded once per sample here
-// instead of fused into the sum; the per-direction weights are applied as
-// fused multiply-adds (a few ulp from the per-hour kernel's order).
-//
-// Border tiles (halo reaching outside the raster) stage zeros outside and
-// follow the per-hour walk's edge rule: a walk whose first step leaves the
-// raster sees no ground (hit = 0); one that leaves at step L > 0 repeats its
-// last sample (step L - 1) for the remaining second - L steps and never hits.
-// Per direction the kernel keeps `lim` (samples read) and a frozen-tail bit
-// (then hit = second, else hit = lim): 6 bits, 5 directions per word.
-//
-// Shared memory: the two (Lup, albedo*shadow) float4 planes, one byte per
-// pixel of bits (ground during the walk-length pass, then the pass hours'
-// sunlit-wall bits 0..3) and the daytime hour list; the albedo of the
-// walk-length pass lives in the second float4 plane before the first hour
-// pass overwrites it.  A warp's byte loads (8 x 4 pixels, rows 74 bytes
-// apart) touch distinct banks: one wavefront.
-constexpr int kHvN = kHvPitch * kHvPitch;
-constexpr int kHvCh = 4;
-constexpr int kHvThreads = kHvTile * kHvTile;
-constexpr int kHvBitsBytes = (kHvN + 15) & ~15;
-
-size_t hv_smem_bytes() { return (size_t)kHvN * 2 * sizeof(float4) + kHvBitsBytes + 64 * sizeof(int); }
-
-// The hour-independent part of the hour-vectorized GVF for the pixel at tile
-// offset `own` (tile staged with its ground bits and albedo): the walk-length
-// code of every direction (5 per word: lim, frozen-tail bit) and the
-// albedo-without-shadow GVF sum (before / 18).  Shared by day_gvf_hv_kernel
-// and gvf_statics_kernel.
-__device__ __forceinline__ float hv_static_walks(const uint8_t* bits, const float* albs, int own, bool own_ground,
-                                                 bool interior, int r, int c, int rows, int cols,
-                                                 const GvfTable<22>& tab, uint32_t (&hits)[4]) {
-    constexpr int FIRST = 1, SECOND = 22;
-    constexpr float albedo_b = 0.2f;
-    constexpr float inv_first = 1.f / FIRST, inv_first1 = 1.f / (FIRST + 1);
-    constexpr float inv_second = 1.f / SECOND;
-    const float ob = own_ground ? 1.f : 0.f;
-    float nsh = 0.f;
-#pragma unroll
-    for (int w = 0; w < 4; ++w) hits[w] = 0u;
-    for (int j = 0; j < SOLWEIG_GVF_DIRECTIONS; ++j) {
-        int hit = 0, lim = 0;
-        float s_alb = 0.f, n_alb = 0.f;
-        if (own_ground) {
-            hit = lim = SECOND;
-            for (int m = 0; m < SECOND; ++m) {
-                if (!interior) {
-                    const int2 o = tab.offs[j * SECOND + m];
-                    if (!in_raster(r + o.x, c + o.y, rows, cols)) {
-                        if (m == 0) {
-                            hit = lim = 0;
-                        } else {  // frozen tail: step m and the rest repeat step m - 1
-                            lim = m;
-                            const float al = albs[own + tab.delta[j * SECOND + m - 1]];
-                            s_alb += al;
-                            s_alb += (SECOND - 1 - m) * al;
-                        }
-                        break;
-                    }
-                }
-                const int off = own + tab.delta[j * SECOND + m];
-                if (!(bits[off] & 1u)) {
-                    hit = lim = m;
-                    break;
-                }
-                s_alb += albs[off];
-                if (m + 1 == FIRST) n_alb = s_alb;
-            }
-        }
-        hits[j / 5] |= ((uint32_t)lim | (hit > lim ? 32u : 0u)) << (6 * (j % 5));
-        const int n_wall = SECOND - hit;
-        const int n_wall_first = FIRST > hit ? FIRST - hit : 0;
-        const float nosh1 = n_wall_first > 0 ? ((float)n_wall_first * albedo_b + n_alb) * inv_first1 : n_alb * inv_first;
-        const float nosh2 = n_wall > 0 ? ((float)n_wall * albedo_b + s_alb) * inv_second : s_alb * inv_second;
-        nsh += (nosh1 * 0.5f + nosh2 * 0.4f) * (1.f / 0.9f);
-    }
-    nsh *= ob;
-    nsh += 18.f * (albs[own] * (1.f - ob));
-    return nsh;
-}
-
-__global__ void __launch_bounds__(kHvThreads, 1) day_gvf_hv_kernel(SolweigScene S, const SolweigHour* __restrict__ hours,
-                                                                  int nhours, GvfTable<22> tab,
-                                                                  const float4* __restrict__ quads,
-                                                                  float* __restrict__ gvf, float* __restrict__ nosh) {
-    constexpr int FIRST = 1, SECOND = 22;
-    const int tr = blockIdx.y, tc = blockIdx.x;
-    const bool interior = hv_tile_interior(S.rows, S.cols, tr, tc);
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    float4* LA = reinterpret_cast<float4*>(smem_raw);  // Lup, albsh of pass hours 0, 1
-    float4* LB = LA + kHvN;                            // pass hours 2, 3
-    uint8_t* bits = reinterpret_cast<uint8_t*>(LB + kHvN);    // ground bit, then sunlit-wall bits
-    float* albs = reinterpret_cast<float*>(LB);                // albedo (walk-length pass only)
-    int* dayh = reinterpret_cast<int*>(bits + kHvBitsBytes);   // daytime hour indices
-    __shared__ int nday;
-    const int tid = threadIdx.y * kHvTile + threadIdx.x;
-    const long long n = (long long)S.rows * S.cols;
-    const int row0 = tr * kHvTile - kHvHalo, col0 = tc * kHvTile - kHvHalo;
-    if (tid == 0) {
-        int k = 0;
-        for (int h = 0; h < nhours && k < 64; ++h)
-            if (hours[h].daytime) dayh[k++] = h;
-        nday = k;
-    }
-    __syncthreads();
-    const int nd = nday;
-    if (nd == 0) return;
-    const bool statics = S.gvf_hits != nullptr && S.gvf_nosh != nullptr;
-    if (!statics) {
-        const float4* q0 = quads + (long long)dayh[0] * n;
-        for (int i = tid; i < kHvN; i += kHvThreads) {
-            const int rr = row0 + i / kHvPitch, cc = col0 + i % kHvPitch;
-            const bool in = interior || in_raster(rr, cc, S.rows, S.cols);
-            const float4 q = in ? q0[(long long)rr * S.cols + cc] : make_float4(0.f, 0.f, 0.f, 0.f);
-            bits[i] = (uint8_t)(__float_as_int(q.w) & kQuadGround);
-            albs[i] = q.z;
-        }
-        __syncthreads();
-    }
-    // each warp walks an 8 x 4 (columns x rows) piece of the tile: walk lengths
-    // of nearby pixels are alike in both directions (24% fewer warp steps than
-    // a row of 32 on the synthetic city), and a warp's shared loads still take
-    // 4 wavefronts (rows of the piece 296 words, 8 banks, apart)
-    const int lw = tid >> 5, ll = tid & 31;
-    const int tx = (lw & 3) * 8 + (ll & 7), ty = (lw >> 2) * 4 + (ll >> 3);
-    const int r = tr * kHvTile + ty, c = tc * kHvTile + tx;
-    const bool valid = r < S.rows && c < S.cols;  // partial tiles at the far edges
-    const long long p = valid ? (long long)r * S.cols + c : 0;
-    const int own = (ty + kHvHalo) * kHvPitch + tx + kHvHalo;
-    // the ground bit of the sweep's quads is the scene's (flags bit 0)
-    const bool own_ground = valid && (statics ? (S.flags[p] & 1) != 0 : (bits[own] & 1u) != 0);
-    const float ob = own_ground ? 1.f : 0.f;
-    const uint32_t face = valid ? S.gvf_face[p] : 0u;
-    constexpr float albedo_b = 0.2f;
-    constexpr float inv_first = 1.f / FIRST, inv_first1 = 1.f / (FIRST + 1);
-    constexpr float inv_second = 1.f / SECOND, inv_second1 = 1.f / (SECOND + 1);
-    // walk lengths and the static plane: prepared with the scene
-    // (gvf_statics_kernel) or walked here from the first daytime hour's quads
-    uint32_t hits[4] = {0u, 0u, 0u, 0u};
-    if (statics) {
-        if (valid) {
-#pragma unroll
-            for (int w = 0; w < 4; ++w) hits[w] = S.gvf_hits[(long long)w * n + p];
-            nosh[p] = S.gvf_nosh[p];
-        }
-    } else {
-        const float nsh = hv_static_walks(bits, albs, own, own_ground, interior, r, c, S.rows, S.cols, tab, hits);
-        if (valid) nosh[p] = nsh / 18.f;
-    }
-    const double ambient_e = valid ? kSBC * (double)S.emis[p] : 0.0;
-
-    for (int g0 = 0; g0 < nd; g0 += kHvCh) {
-        const int nc = nd - g0 < kHvCh ? nd - g0 : kHvCh;
-        __syncthreads();  // the previous pass no longer reads the tile
-        for (int i = tid; i < kHvN; i += kHvThreads) {
-            const int rr = row0 + i / kHvPitch, cc = col0 + i % kHvPitch;
-            const bool in = interior || in_raster(rr, cc, S.rows, S.cols);
-            const long long pix = in ? (long long)rr * S.cols + cc : 0;
-            float v[2 * kHvCh];
-            uint32_t b = 0u;
-#pragma unroll
-            for (int k = 0; k < kHvCh; ++k) {
-                if (k < nc && in) {
-                    const float4 q = quads[(long long)dayh[g0 + k] * n + pix];
-                    v[2 * k] = q.y;
-                    v[2 * k + 1] = q.z * q.x;
-                    b |= (((uint32_t)__float_as_int(q.w) & kQuadSunwall) ? 1u : 0u) << k;
-                } else {
-                    v[2 * k] = v[2 * k + 1] = 0.f;
-                }
-            }
-            LA[i] = make_float4(v[0], v[1], v[2], v[3]);
-            LB[i] = make_float4(v[4], v[5], v[6], v[7]);
-            bits[i] = (uint8_t)b;
-        }
-        __syncthreads();
-        float lw[kHvCh];
-#pragma unroll
-        for (int k = 0; k < kHvCh; ++k) {
-            if (k < nc) {
-                const SolweigHour& hh = hours[dayh[g0 + k]];
-                lw[k] = (float)(kSBC * 0.9 * pow4(hh.tgwall + hh.ta + 273.15) - kSBC * 0.9 * pow4(hh.ta + 273.15));
-            } else {
-                lw[k] = 0.f;
-            }
-        }
-        float lup_t[kHvCh], alb_t[kHvCh];
-#pragma unroll
-        for (int k = 0; k < kHvCh; ++k) lup_t[k] = alb_t[k] = 0.f;
-        if (own_ground) {
-#pragma unroll 1
-            for (int j = 0; j < SOLWEIG_GVF_DIRECTIONS; ++j) {
-                const uint32_t code = (hits[j / 5] >> (6 * (j % 5))) & 63u;
-                const int lim = (int)(code & 31u);
-                const int hit = (code & 32u) ? SECOND : lim;
-                float sl[kHvCh], sa[kHvCh], l0[kHvCh], a0[kHvCh];
-#pragma unroll
-                for (int k = 0; k < kHvCh; ++k) sl[k] = sa[k] = l0[k] = a0[k] = 0.f;
-                // Per hour k (byte k of both words): seen = a sunlit wall met so far,
-                // cnt = steps before the first one (branch-free: each step adds
-                // the not-yet-seen bytes), so f = cnt_k when seen_k.
-                uint32_t seen = 0u, cnt = 0u;
-#pragma unroll
-                for (int m = 0; m < SECOND; ++m) {
-                    if (m < lim) {
-                        const int off = own + tab.delta[j * SECOND + m];
-                        const float4 A = LA[off], B = LB[off];
-                        const uint32_t b = bits[off];
-                        sl[0] += A.x; sa[0] += A.y; sl[1] += A.z; sa[1] += A.w;
-                        sl[2] += B.x; sa[2] += B.y; sl[3] += B.z; sa[3] += B.w;
-                        seen |= (b * 0x00204081u) & 0x01010101u;  // bit k -> byte k
-                        cnt += ~seen & 0x01010101u;
-                        if (m + 1 == FIRST) {
-#pragma unroll
-                            for (int k = 0; k < kHvCh; ++k) {
-                                l0[k] = sl[k];
-                                a0[k] = sa[k];
-                            }
-                        }
-                    }
-                }
-                if (hit > lim) {
-                    // frozen tail (border tiles): step lim and the rest repeat step lim - 1,
-                    // whose sunlit-wall bits are already counted
-                    const int last = own + tab.delta[j * SECOND + lim - 1];
-                    const float4 A = LA[last], B = LB[last];
-                    const float rest = (float)(SECOND - 1 - lim);
-                    const float tl[kHvCh] = {A.x, A.z, B.x, B.z}, ta_[kHvCh] = {A.y, A.w, B.y, B.w};
-#pragma unroll
-                    for (int k = 0; k < kHvCh; ++k) {
-                        sl[k] += tl[k];
-                        sa[k] += ta_[k];
-                        sl[k] += rest * tl[k];
-                        sa[k] += rest * ta_[k];
-                    }
-                }
-                const bool fj = (face >> j) & 1u;
-                // Per hour, with f the first step showing a sunlit wall (FIRST = 1):
-                //   near = (f == 0 < hit): lup1 = (lw + l0) / 2, else l0;
-                //   far  = (f < hit):      lup2 = ((SECOND - f) lw + sl) / (SECOND + 1), else sl / SECOND,
-                //          the wall term dropped when f == 0 on a self-shadowed face (fj);
-                //   lup_t += (0.5 lup1 + 0.4 lup2) / 0.9  (the same for the albedos with albedo_b),
-                // as two fused multiply-adds with the selected weights.
-#pragma unroll
-                for (int k = 0; k < kHvCh; ++k) {
-                    const int f = (seen >> (8 * k)) & 1u ? (int)((cnt >> (8 * k)) & 0xFFu) : 31;
-                    const bool sun_far = f < hit;
-                    const bool sun_near = sun_far && f == 0;
-                    const float wn = (sun_far && !(sun_near && fj)) ? (float)(SECOND - f) : 0.f;
-                    const float en = sun_near ? 1.f : 0.f;
-                    const float c1 = sun_near ? (inv_first1 * 0.5f / 0.9f) : (inv_first * 0.5f / 0.9f);
-                    const float c2 = sun_far ? (inv_second1 * 0.4f / 0.9f) : (inv_second * 0.4f / 0.9f);
-                    lup_t[k] = fmaf(c1, fmaf(en, lw[k], l0[k]), lup_t[k]);
-                    lup_t[k] = fmaf(c2, fmaf(wn, lw[k], sl[k]), lup_t[k]);
-                    alb_t[k] = fmaf(c1, fmaf(en, albedo_b, a0[k]), alb_t[k]);
-                    alb_t[k] = fmaf(c2, fmaf(wn, albedo_b, sa[k]), alb_t[k]);
-                }
-            }
-        }
-        const float4 oA = LA[own], oB = LB[own];
-        const float own_lup[4] = {oA.x, oA.z, oB.x, oB.z};
-        const float own_albsh[4] = {oA.y, oA.w, oB.y, oB.w};
-#pragma unroll
-        for (int k = 0; k < kHvCh; ++k) {
-            if (k < nc && valid) {
-                const int h = dayh[g0 + k];
-                const SolweigHour& hh = hours[h];
-                const float lt = lup_t[k] + 18.f * (own_lup[k] * (1.f - ob));
-                const float at = alb_t[k] + 18.f * (own_albsh[k] * (1.f - ob));
-                const double ambient = ambient_e * pow4(hh.ta + 273.15);
-                gvf[(3LL * h) * n + p] = (float)((double)(lt / 18.f) + ambient);
-                gvf[(3LL * h + 1) * n + p] = at / 18.f;
-                gvf[(3LL * h + 2) * n + p] = quads[(long long)h * n + p].x;
-            }
-        }
-    }
-}
-
-// Scene statics of the hour-vectorized GVF (1 m walk, no water): per pixel
-// the walk-length codes [4][px] and the albedo-without-shadow GVF [px], from
-// the scene's ground bits and albedo -- what day_gvf_hv_kernel would walk
-// from the first daytime hour's quads each day.  32 x 32 tiles, 1024 threads.
-size_t gvf_statics_smem_bytes() { return (size_t)kHvBitsBytes + (size_t)kHvN * sizeof(float); }
-
-__global__ void __launch_bounds__(kHvThreads, 1) gvf_statics_kernel(SolweigScene S, GvfTable<22> tab,
-                                                                   uint32_t* __restrict__ hits_out,
-                                                                   float* __restrict__ nosh_out) {
-    const int tr = blockIdx.y, tc = blockIdx.x;
-    const bool interior = hv_tile_interior(S.rows, S.cols, tr, tc);
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    float* albs = reinterpret_cast<float*>(smem_raw);
-    uint8_t* bits = reinterpret_cast<uint8_t*>(albs + kHvN);
-    const int tid = threadIdx.y * kHvTile + threadIdx.x;
-    const long long n = (long long)S.rows * S.cols;
-    const int row0 = tr * kHvTile - kHvHalo, col0 = tc * kHvTile - kHvHalo;
-    for (int i = tid; i < kHvN; i += kHvThreads) {
-        const int rr = row0 + i / kHvPitch, cc = col0 + i % kHvPitch;
-        const bool in = interior || in_raster(rr, cc, S.rows, S.cols);
-        const long long q = in ? (long long)rr * S.cols + cc : 0;
-        bits[i] = in ? (uint8_t)(S.flags[q] & 1) : (uint8_t)0;
-        albs[i] = in ? S.alb[q] : 0.f;
-    }
-    __syncthreads();
-    const int lw = tid >> 5, ll = tid & 31;
-    const int tx = (lw & 3) * 8 + (ll & 7), ty = (lw >> 2) * 4 + (ll >> 3);
-    const int r = tr * kHvTile + ty, c = tc * kHvTile + tx;
-    if (r >= S.rows || c >= S.cols) return;
-    const long long p = (long long)r * S.cols + c;
-    const int own = (ty + kHvHalo) * kHvPitch + tx + kHvHalo;
-    const bool own_ground = (bits[own] & 1u) != 0;
-    uint32_t hits[4];
-    const float nsh = hv_static_walks(bits, albs, own, own_ground, interior, r, c, S.rows, S.cols, tab, hits);
-#pragma unroll
-    for (int w = 0; w < 4; ++w) hits_out[(long long)w * n + p] = hits[w];
-    nosh_out[p] = nsh / 18.f;
 }
 
 // ------------------------------------------------------------- kernels 3, 4, 5
@@ -1353,11 +1015,12 @@ __global__ void __launch_bounds__(THREADS, 2048 / THREADS) day_radiation_kernel(
 inline long long align256(long long x) { return (x + 255) & ~255LL; }
 
 struct DayWork {
-    long long quads, lup_first, gvf, nosh, sums, wf32, bw, tables, error, tilemax, total;
+    long long quads, lup_first, gvf, nosh, sums, wf32, bw, tables, error, tilemax, walks, dict, total;
 };
 
-DayWork day_work_layout(long long px, int nhours, bool water) {
+DayWork day_work_layout(int rows, int cols, int nhours, bool water) {
     DayWork w{};
+    const long long px = (long long)rows * cols;
     const int ncols = 2 * nhours;
     const int nb = (ncols + 15) / 16 * 16;
     long long o = 0;
@@ -1375,6 +1038,10 @@ DayWork day_work_layout(long long px, int nhours, bool water) {
     // per 16 x 16 tile maxima of the heights (ceil(rows/16) * ceil(cols/16)
     // floats, bounded here from the pixel count alone: <= px/256 + (rows + cols)/16 + 1)
     w.tilemax = o; o = align256(o + 4LL * (px / 256 + (px + 1) / 16 + 4));
+    // GVF walk words, for scenes that come without them, and the tiles' distinct samples
+    w.walks = o; o = align256(o + (water ? 0 : 4LL * walk_words(rows, cols)));
+    w.dict = o;
+    o = align256(o + (water ? 0 : walk_words(rows, cols) / kWkTileWords * 8 * kWkDictKeys * ((nhours + 3) / kWkHours)));
     w.total = o;
     return w;
 }

@@ -540,21 +540,27 @@ class Scene:
         return self
 
     def _gvf_statics(self, st):
-        """The hour-independent part of the batched day's GVF (walk length of
-        every direction, albedo-without-shadow plane) for the 1 m walk of a
-        scene without water, prepared once here (``solweig_gvf_statics``) so
-        the days skip that walk; other scenes leave the pointers NULL."""
-        self.gvf_hits = self.gvf_nosh = None
-        if self.first_steps != 1 or self.second_steps != 22 or self.has_water:
+        """The hour-independent part of the ground view factors (walk words and
+        lengths of every direction, albedo-without-shadow plane) for walks of
+        2 to 22 steps in a scene without water, prepared once here
+        (``solweig_gvf_walks``) so the days skip that walk; other scenes leave
+        the pointers NULL."""
+        self.gvf_hits = self.gvf_nosh = self.gvf_walks = None
+        if self.first_steps != 1 or not 2 <= self.second_steps <= 22 or self.has_water:
             return
         dev = self.dsm.device
+        L = _lib.lib()
         self.gvf_hits = torch.empty((4,) + self.shape, dtype=torch.int32, device=dev)
         self.gvf_nosh = torch.empty(self.shape, dtype=torch.float32, device=dev)
-        _lib.check(_lib.lib().solweig_gvf_statics(
+        self.gvf_walks = torch.empty(int(L.solweig_gvf_walk_words(self.rows, self.cols)), dtype=torch.int32,
+                                     device=dev)
+        _lib.check(L.solweig_gvf_walks(
             ctypes.byref(self.struct), self.gvf_host_ptr, self.first_steps, self.second_steps,
-            device_ptr(self.gvf_hits), device_ptr(self.gvf_nosh), st), "solweig_gvf_statics")
+            device_ptr(self.gvf_hits), device_ptr(self.gvf_walks), self.gvf_walks.numel(),
+            device_ptr(self.gvf_nosh), st), "solweig_gvf_walks")
         self.struct.gvf_hits = self.gvf_hits.data_ptr()
         self.struct.gvf_nosh = self.gvf_nosh.data_ptr()
+        self.struct.gvf_walks = self.gvf_walks.data_ptr()
 
     def _make_struct(self):
         s = _lib.SolweigScene()

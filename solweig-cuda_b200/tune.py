@@ -6,7 +6,7 @@ The search space is :class:`_lib.SolweigDayConfig`:
   windows, fixed 16 x 16 tiles), or the raster sweep with a shadow block
   (columns x rows) of 32x8, 64x4, 16x16, 32x4, 128x2
 * GVF: tile rows per block of the per-hour kernel: 4, 8, 16 (32 columns,
-  halo of ``second`` - 1), or the hour-vectorized kernel on 32 x 32 tiles
+  halo of ``second`` - 1), or the walk-word kernel on 32 x 32 tiles
 * radiation block: 128 or 256 pixels
 * patch-contraction CTAs per SM: 1 or 2
 

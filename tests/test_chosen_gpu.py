@@ -407,3 +407,54 @@ def test_gvf_statics_prepared_with_the_scene_are_identical(cuda):
             assert torch.equal(ga[h], gb[h]), h
     for k in outs:
         torch.testing.assert_close(a[k], b[k], rtol=0, atol=0, equal_nan=True)
+
+
+@pytest.mark.parametrize("rows,cols,pixel,fields", [
+    (32, 32, 1.0, "classes"), (33, 65, 1.0, "classes"), (7, 40, 1.0, "classes"), (97, 70, 1.0, "classes"),
+    (64, 31, 2.0, "classes"), (70, 45, 4.0, "classes"), (40, 40, 1.25, "classes"),
+    (97, 70, 1.0, "random"), (33, 65, 2.0, "random"), (97, 70, 1.0, "both")])
+def test_walk_word_gvf_matches_per_hour_kernel(cuda, rows, cols, pixel, fields):
+    """The walk-word GVF kernel (walks of 6 to 22 steps, tiles cut by the raster
+    edge, rasters smaller than a walk; samples counted per value, added one by
+    one, or both in different tiles) against the per-hour kernel, with the walk
+    words prepared by the scene and by the day.  Per pixel both forms add at
+    most 22 float32 samples in each of 18 directions: 40 roundings of a sum
+    below the largest sample, relative to the largest sample."""
+    import torch
+    from solweig_cuda_b200 import _lib, batched, engine, synthetic
+    s = synthetic.make_scene(rows, cols, seed=rows + cols, pixel_size=pixel, building_cover=0.2)
+    scene = engine.Scene(s.dsm, s.trees, s.dem, pixel, landcover=s.landcover)
+    if fields != "classes":
+        part = slice(None) if fields == "random" else slice(0, cols // 4)
+        gen = torch.Generator(device="cuda").manual_seed(5)
+        scene.alb[:, part] = 0.1 + 0.3 * torch.rand(scene.alb[:, part].shape, generator=gen, device="cuda")
+        scene._gvf_statics(engine.stream_handle())
+    assert scene.struct.gvf_walks
+    met = synthetic.make_met(doy=100, latitude=48.0, longitude=0.0, seed=2)
+    n = scene.pixels
+    res = []
+    for hv, statics in ((0, True), (1, True), (1, False)):
+        if not statics:
+            scene.struct.gvf_walks = None
+        day = batched.ChosenDay(scene, 48.0, 0.0, 3.0, 0.0)
+        cfg = _lib.SolweigDayConfig.default()
+        cfg.gvf_hours = hv
+        day.set_config(cfg)
+        out = {k: v.clone() for k, v in day.run_day(met).items()}
+        torch.cuda.synchronize()
+        o = day.work_offsets()
+        gvf = day.work[o["gvf"]:o["gvf"] + 12 * 24 * n].view(torch.float32).view(24, 3, n).clone()
+        nosh = day.work[o["nosh"]:o["nosh"] + 4 * n].view(torch.float32).clone()
+        res.append((out, gvf, nosh, [h.daytime for h, _, _ in day.plan(met)]))
+    (_, g0, n0, dayflags), (o1, g1, n1, _), (o2, g2, n2, _) = res
+    torch.testing.assert_close(n1, n0, rtol=1e-5, atol=1e-6)
+    assert torch.equal(n2, n1)
+    eps = 40 * 2.0 ** -24
+    for h, d in enumerate(dayflags):
+        if d:
+            torch.testing.assert_close(g1[h, 0], g0[h, 0], rtol=eps, atol=eps * float(g0[h, 0].abs().max()))
+            torch.testing.assert_close(g1[h, 1], g0[h, 1], rtol=eps, atol=eps)
+            assert torch.equal(g1[h, 2], g0[h, 2])
+            assert torch.equal(g2[h], g1[h])
+    for k in o1:  # bit patterns: UTCI is NaN on building pixels
+        assert torch.equal(o2[k].view(torch.int32), o1[k].view(torch.int32)), k
