@@ -545,6 +545,45 @@ int solweig_utci(const float* ta, const float* rh, const float* tmrt, const floa
  * polynomial is collapsed on the host and evaluated per pixel in (Tmrt - Ta). */
 int solweig_utci_scalar(double ta, double rh, double va, const float* tmrt, float* out, int64_t n,
                         void* stream);
+/* Host plan of forcing hours (host memory only, no device work): the FP64
+ * scalars, per-patch weights and sun ray of hours [0, n) of one run, carrying
+ * the clearness index and the wave-delay clock from hour to hour. */
+typedef struct SolweigPlanScene {
+    double latitude;                /* degrees */
+    double scale, amaxvalue;        /* 1 / pixel size, highest object above the lowest ground */
+    double tgk_wall, tstart_wall, tmaxlst_wall;
+    int32_t rows, cols, patches, nbands;
+    /* per patch: azimuth (degrees), sin / cos of the altitude, cos of the zenith angle, solid angle */
+    double azimuth[SOLWEIG_MAX_PATCHES], sin_alt[SOLWEIG_MAX_PATCHES], cos_alt[SOLWEIG_MAX_PATCHES];
+    double cos_zen[SOLWEIG_MAX_PATCHES], steradian[SOLWEIG_MAX_PATCHES];
+    double band_inv_cos[SOLWEIG_MAX_BANDS]; /* 1 / cos of a band's zenith angle */
+} SolweigPlanScene;
+
+typedef struct SolweigPlanRow {
+    double altitude, azimuth;       /* sun, degrees */
+    double zen, jday, dectime, altmax;
+    double ta, rh, rad_g, rad_d, rad_i, p_kpa, ws, psi;
+    double new_day;                 /* not 0: the clearness index starts at 1 */
+    /* of the sun's azimuth and altitude; the ray's steps round on them */
+    double sin_az, cos_az, tan_az, tan_alt, sin_alt, cos_alt, tan_zen;
+} SolweigPlanRow;
+
+typedef struct SolweigPlanState {
+    double ci, firstdaytime, timeadd;
+} SolweigPlanState;
+
+typedef struct SolweigPlanScalars {
+    double ea, esky, i0, ci, rad_i, rad_d, ci_tg, ci_tgg, tgwall;
+    double steps;                   /* entries of the hour's ray */
+    double band_lsky[SOLWEIG_MAX_BANDS];
+} SolweigPlanScalars;
+
+/* hours [n] without their ray pointers; ray_dxdy [n][ray_capacity][2],
+ * ray_dz [n][ray_capacity]; luminance [n][SOLWEIG_MAX_PATCHES] (Perez, sum 1;
+ * 0 at night); state is read and left as the last hour leaves it. */
+int solweig_plan_hours(const SolweigPlanScene* scene, const SolweigPlanRow* rows, int n, double timestepdec,
+                       double twater, SolweigPlanState* state, SolweigHour* hours, SolweigPlanScalars* scalars,
+                       int32_t* ray_dxdy, double* ray_dz, int ray_capacity, double* luminance);
 /* Host function: UTCI as a polynomial in D = Tmrt - Ta for scalar weather,
  * coefficients[0..6] (all zero when an input is the -999 sentinel). */
 int solweig_utci_collapse(double ta, double rh, double va, double* coefficients);

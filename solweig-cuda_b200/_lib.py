@@ -117,6 +117,24 @@ class SolweigGradParams(ctypes.Structure):
     _fields_ = [("albedo", _vp), ("emissivity", _vp), ("transmissivity", _vp)]
 
 
+class SolweigPlanScene(ctypes.Structure):
+    """Scene and sky constants of the host plan."""
+    _fields_ = [("latitude", ctypes.c_double), ("scale", ctypes.c_double), ("amaxvalue", ctypes.c_double),
+                ("tgk_wall", ctypes.c_double), ("tstart_wall", ctypes.c_double), ("tmaxlst_wall", ctypes.c_double),
+                ("rows", ctypes.c_int32), ("cols", ctypes.c_int32), ("patches", ctypes.c_int32),
+                ("nbands", ctypes.c_int32)] + [
+        (name, ctypes.c_double * MAX_PATCHES) for name in ("azimuth", "sin_alt", "cos_alt", "cos_zen", "steradian")
+    ] + [("band_inv_cos", ctypes.c_double * MAX_BANDS)]
+
+
+# Columns of SolweigPlanRow and SolweigPlanScalars, and SolweigPlanState (all float64).
+PLAN_ROW = ("altitude", "azimuth", "zen", "jday", "dectime", "altmax", "ta", "rh", "rad_g", "rad_d", "rad_i",
+            "p_kpa", "ws", "psi", "new_day", "sin_az", "cos_az", "tan_az", "tan_alt", "sin_alt", "cos_alt", "tan_zen")
+PLAN_SCALARS = ("ea", "esky", "i0", "ci", "rad_i", "rad_d", "ci_tg", "ci_tgg", "tgwall", "steps") \
+    + tuple(f"band_lsky{b}" for b in range(MAX_BANDS))
+PLAN_STATE = ("ci", "firstdaytime", "timeadd")
+
+
 class SolweigDayConfig(ctypes.Structure):
     """Launch shapes of the batched day (``solweig_day_batched_ex``)."""
     _fields_ = [("shadow_bx", ctypes.c_int32), ("shadow_by", ctypes.c_int32),
@@ -143,7 +161,7 @@ EXPORTED_SYMBOLS = (
     "solweig_patch_sums", "solweig_day_batched_timed", "solweig_day_batched_ex", "solweig_day_batched_part",
     "solweig_day_batched_layout", "solweig_day_grad_work_bytes", "solweig_day_grad_forward",
     "solweig_day_grad_backward", "solweig_svf_ex", "solweig_svf_ex2", "solweig_svf_work_bytes",
-    "solweig_gvf_statics", "solweig_gvf_walk_words", "solweig_gvf_walks", "solweig_step64", "solweig_struct_sizes64", "solweig_wall_segments_burn",
+    "solweig_gvf_statics", "solweig_gvf_walk_words", "solweig_gvf_walks", "solweig_plan_hours", "solweig_step64", "solweig_struct_sizes64", "solweig_wall_segments_burn",
     "solweig_geometry_walls",
 )
 
@@ -185,6 +203,7 @@ def _declare(lib):
         "solweig_day_batched_part": (i32, [P, P, P, i32, P, P, i64, P, i32, i32, P, i64, P, i32, i32, i32, P]),
         "solweig_day_batched_layout": (i32, [i32, i32, i32, i32, P]),
         "solweig_gvf_statics": (i32, [P, P, i32, i32, P, P, P]),
+        "solweig_plan_hours": (i32, [P, P, i32, dbl, dbl, P, P, P, P, P, i32, P]),
         "solweig_gvf_walk_words": (i64, [i32, i32]),
         "solweig_gvf_walks": (i32, [P, P, i32, i32, P, P, i64, P, P]),
         "solweig_day_grad_work_bytes": (i64, [i32, i32, i32]),

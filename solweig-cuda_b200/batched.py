@@ -1,8 +1,8 @@
 """Batched form: a whole day (or many days) per CUDA-graph replay.
 
 All hours of a day are planned on the host first (FP64 solar geometry,
-Perez luminance, patch weights, sun rays), written into pinned memory and
-replayed as one captured graph: the hour-record and ray uploads, the state
+Perez luminance, patch weights, sun rays: ``engine.plan_day``), written into
+pinned memory and replayed as one captured graph: the hour-record and ray uploads, the state
 reset and the 2 kernels of every hour (``solweig_day``).  The graph is
 captured once per scene and replays for any forcing of the same length,
 because every kernel reads its hour record from device memory.
@@ -15,7 +15,8 @@ import numpy as np
 import torch
 
 from . import _lib
-from .engine import HourBuffers, device_ptr, outputs_struct, plan_day, plan_hours, stream_handle
+from . import sun as _sun
+from .engine import HourBuffers, device_ptr, outputs_struct, plan_day, stream_handle
 
 __all__ = ["BatchedDay", "ChosenDay", "MultiDay", "TileBatch", "DayError"]
 
@@ -74,6 +75,7 @@ class BatchedDay:
                     for k in self.out_names}
         self.use_graph = use_graph
         self.graph = None
+        self.warm = False  # an eager day has run
 
     @property
     def launches_per_day(self):
@@ -106,20 +108,25 @@ class BatchedDay:
             raise ValueError(f"expected {self.hours} forcing rows, got {len(met)}")
         plan = plan_day(self.scene, met, self.latitude, self.longitude, self.site_altitude, self.utc)
         self.buffers.wait_free()
-        for i, (h, ray, _) in enumerate(plan):
-            self.buffers.put(i, h, ray)
-        self.last_scalars = [p[2] for p in plan]
+        self.buffers.put_plan(plan)
+        self.last_plan = plan
         return plan
 
+    @property
+    def last_scalars(self):
+        """HourScalars of the rows of the last day."""
+        return [p[2] for p in self.last_plan]
+
     def run_day(self, met, outputs=None):
-        """Plan the day on the host and replay; returns {name: [H, rows, cols]} views
-        that stay valid until the next call."""
+        """Plan the day on the host and run it; returns {name: [H, rows, cols]} views
+        that stay valid until the next call.  The first day runs eagerly (a run of
+        one day pays for no capture), the second captures the graph."""
         self.plan(met)
-        if not self.use_graph:
+        if not self.use_graph or self.graph is None and not self.warm:
             self._sequence()
+            self.warm = True
         else:
             if self.graph is None:
-                self._sequence()          # eager pass: kernel attributes, allocator warm-up
                 torch.cuda.synchronize()
                 g = torch.cuda.CUDAGraph()
                 with torch.cuda.graph(g):
@@ -145,14 +152,14 @@ def day_launches(scene, config, sweep_parts=1):
     return sweep_parts * (2 + c) + c + win + walk + 7
 
 
+PIPELINE_HOURS = (2, 2, 2, 2, 4, 4, 8)
+
+
 class ChosenDay(BatchedDay):
     """The batched form: every hour of a day in a few launches
-    (``solweig_day_batched``: ray ceilings and shadow sweep over ranges of
-    hours, GVF over all hours, the BF16 tensor-core patch contraction,
-    hour-looping radiation).  Each sweep range is a CUDA graph (with the
-    upload of its hour records) replayed as soon as its hours are planned, so
-    the host plans the next range while the GPU sweeps; the rest of the day is
-    one more graph.
+    (``solweig_day_batched``: ray ceilings and shadow sweep, GVF over all hours,
+    the BF16 tensor-core patch contraction, hour-looping radiation), captured
+    as one CUDA graph with the upload of the hour records.
 
     Produces the all-direction planes (Tmrt, UTCI, Kdown, Kup, Ldown, Lup,
     Kside, Lside, shadow, Tg ...); the cardinal E/S/W/N planes are only made
@@ -161,19 +168,18 @@ class ChosenDay(BatchedDay):
     CARDINAL = ("keast", "ksouth", "kwest", "knorth", "least", "lsouth", "lwest", "lnorth")
 
     def __init__(self, scene, latitude, longitude, site_altitude=3.0, utc=0.0, hours=24,
-                 outputs=("tmrt", "utci"), use_graph=True, pipeline_hours=(2, 2, 2, 2, 4, 4, 8)):
+                 outputs=("tmrt", "utci"), use_graph=True, pipeline_hours=PIPELINE_HOURS):
         bad = [o for o in outputs if o in self.CARDINAL]
         if bad:
             raise ValueError(f"the batched form does not produce {bad}")
         super().__init__(scene, latitude, longitude, site_altitude, utc, hours, outputs, use_graph)
         self.scratch = None
-        # pipeline_hours: the sweep stage runs in ranges of hours, each launched
-        # as soon as its hours are planned (the host plans the next range while
-        # the GPU sweeps this one): an int gives ranges of that many hours, a
-        # sequence the successive range lengths (the last one repeats), 0 plans
-        # the whole day first.  The default starts with short ranges, so the
-        # GPU starts early, and grows them, so fewer launches are paid for.
-        self.ranges = self._ranges(hours, pipeline_hours)
+        # pipeline_hours: an int or a sequence of range lengths (the last one
+        # repeats) issues the sweep stage in ranges of hours with a graph each; 0
+        # and the default issue it as a whole.  Ranges let the GPU start before
+        # the last hours are planned, but planning a day takes 0.2 ms after the
+        # sun positions, less than seven sweep launches cost a small raster.
+        self.ranges = None if pipeline_hours is PIPELINE_HOURS else self._ranges(hours, pipeline_hours)
         self.part_graphs = None
         L = _lib.lib()
         self.work_bytes = int(L.solweig_day_batched_work_bytes(scene.rows, scene.cols, hours,
@@ -213,6 +219,7 @@ class ChosenDay(BatchedDay):
         self.config = config
         self.graph = None
         self.part_graphs = None
+        self.warm = False
 
     def _part(self, part, h0=0, h1=0):
         """One part of the day on the current stream (``solweig_day_batched_part``):
@@ -229,46 +236,29 @@ class ChosenDay(BatchedDay):
             ctypes.byref(self.config), part, h0, h1, stream_handle()), "solweig_day_batched_part")
 
     def run_day(self, met, outputs=None):
-        """Plan the day on the host and run it; with pipelined ranges each sweep
-        range starts as soon as its hours are planned.  Returns {name: [H, rows,
-        cols]} views that stay valid until the next call."""
+        """Plan the day on the host and run it, in one graph or in the ranges of
+        ``pipeline_hours``.  Returns {name: [H, rows, cols]} views that stay valid
+        until the next call."""
         if self.ranges is None:
             return super().run_day(met, outputs)
-        met = np.asarray(met, dtype=np.float64)
-        if len(met) != self.hours:
-            raise ValueError(f"expected {self.hours} forcing rows, got {len(met)}")
-        self.buffers.wait_free()
-        rows = plan_hours(self.scene, met, self.latitude, self.longitude, self.site_altitude, self.utc)
-        scalars = []
-        capture = self.use_graph and self.part_graphs is None
-        for c, (h0, h1) in enumerate(self.ranges):
-            for i in range(h0, h1):
-                h, ray, scal = next(rows)
-                self.buffers.put(i, h, ray)
-                scalars.append(scal)
-            if self.use_graph and not capture:
-                self.part_graphs[c].replay()
-            else:
-                self._part(0, h0, h1)
-        if self.use_graph and not capture:
-            self.part_graphs[-1].replay()
-        else:
-            self._part(1)
-        if capture:
-            # the eager pass above produced this day; capture the parts for the next ones
+        self.plan(met)
+        if self.use_graph and self.part_graphs is None and self.warm:
             torch.cuda.synchronize()
             graphs = []
-            for h0, h1 in self.ranges:
+            for part in [(0, h0, h1) for h0, h1 in self.ranges] + [(1,)]:
                 g = torch.cuda.CUDAGraph()
                 with torch.cuda.graph(g):
-                    self._part(0, h0, h1)
+                    self._part(*part)
                 graphs.append(g)
-            g = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(g):
-                self._part(1)
-            graphs.append(g)
             self.part_graphs = graphs
-        self.last_scalars = scalars
+        if self.use_graph and self.part_graphs is not None:
+            for g in self.part_graphs:
+                g.replay()
+        else:
+            for h0, h1 in self.ranges:
+                self._part(0, h0, h1)
+            self._part(1)
+            self.warm = True
         self.buffers.mark()
         names = self.out_names if outputs is None else outputs
         return {k: self.out[k] for k in names}
@@ -417,8 +407,7 @@ class MultiDay:
         for d in range(self.days):
             plan = plan_day(self.scene, met[d * H:(d + 1) * H], self.latitude, self.longitude,
                             self.site_altitude, self.utc)
-            for i, (h, ray, _) in enumerate(plan):
-                self.buffers.put(d * H + i, h, ray)
+            self.buffers.put_plan(plan, d * H)
 
     def _sequence(self):
         sc = self.scene
@@ -488,6 +477,7 @@ class TileBatch:
                     for s in self.scenes]
         self.configs = list(configs) if configs is not None else [_lib.SolweigDayConfig.default()] * n
         self.graph = None
+        self.warm = False  # an eager day has run
         self.launches = sum(day_launches(s_, c) for s_, c in zip(self.scenes, self.configs))
 
     @property
@@ -495,13 +485,20 @@ class TileBatch:
         return sum(s.pixels for s in self.scenes)
 
     def plan(self, mets):
+        suns = []  # tiles of one case share their sun positions: (forcing times, lat, lon, SolarHours)
         for s, b, met, lat, lon in zip(self.scenes, self.buffers, mets, self.latitudes, self.longitudes):
             met = np.asarray(met, dtype=np.float64)
             if len(met) != self.hours:
                 raise ValueError(f"expected {self.hours} forcing rows, got {len(met)}")
+            for when, at, sol in suns:
+                if at == (lat, lon) and np.array_equal(when, met[:, :4]):
+                    break
+            else:
+                sol = _sun.metdata(met, lat, lon, self.site_altitude, self.utc)
+                suns.append((met[:, :4], (lat, lon), sol))
+            plan = plan_day(s, met, lat, lon, self.site_altitude, self.utc, sol)
             b.wait_free()
-            for i, (h, ray, _) in enumerate(plan_day(s, met, lat, lon, self.site_altitude, self.utc)):
-                b.put(i, h, ray)
+            b.put_plan(plan)
 
     def _sequence(self):
         L = _lib.lib()
@@ -517,7 +514,9 @@ class TileBatch:
                 "solweig_day_batched_ex")
 
     def capture(self):
-        self._sequence()
+        if not self.warm:
+            self._sequence()
+            self.warm = True
         torch.cuda.synchronize()
         g = torch.cuda.CUDAGraph()
         with torch.cuda.graph(g):
@@ -531,7 +530,14 @@ class TileBatch:
         return self.out
 
     def run(self, mets):
+        """One day on every tile: eagerly the first time, then as one graph."""
         self.plan(mets)
+        if self.graph is None and not self.warm:
+            self._sequence()
+            self.warm = True
+            for b in self.buffers:
+                b.mark()
+            return self.out
         if self.graph is None:
             self.capture()
         return self.replay()

@@ -647,14 +647,96 @@ class HourScalars:
     band_lsky: object = None  # float64 band sky emittances (the record holds float32)
 
 
-def _ster_sin(L):
-    """(steradian, sin(altitude)) of every patch as Python floats, cached per layout."""
-    cached = getattr(L, "_ster_sin", None)
-    if cached is None:
-        cached = [(float(L.steradian[k]), float(np.sin(L.altitude[k] * (np.pi / 180))))
-                  for k in range(L.count)]
-        L._ster_sin = cached
-    return cached
+HOUR_DTYPE = np.dtype(_lib.SolweigHour)
+_ROW = {name: i for i, name in enumerate(_lib.PLAN_ROW)}
+_SCALAR = {name: i for i, name in enumerate(_lib.PLAN_SCALARS)}
+_BAND0 = _SCALAR["band_lsky0"]
+
+
+def _plan_scene(scene, latitude):
+    """The constants of the host plan (``SolweigPlanScene``)."""
+    L = scene.layout.host
+    s = _lib.SolweigPlanScene()
+    s.latitude, s.scale, s.amaxvalue = latitude, scene.scale, scene.amaxvalue
+    s.tgk_wall, s.tstart_wall, s.tmaxlst_wall = scene.tgk_wall, scene.tstart_wall, scene.tmaxlst_wall
+    s.rows, s.cols = scene.shape
+    s.patches, s.nbands = L.count, L.band_counts.size
+    for name, values in (("azimuth", L.azimuth), ("sin_alt", L.sin_alt), ("cos_alt", L.cos_alt),
+                         ("cos_zen", L.cos_zen), ("steradian", L.steradian)):
+        np.ctypeslib.as_array(getattr(s, name))[:L.count] = values
+    np.ctypeslib.as_array(s.band_inv_cos)[:s.nbands] = 1 / np.cos((90 - L.band_altitude) * (np.pi / 180))
+    return s
+
+
+class DayPlan:
+    """FP64 host plan of consecutive hours (``solweig_plan_hours``): a sequence of
+    (SolweigHour, ShadowRay or None, HourScalars), backed by
+
+    ``records``    [n] SolweigHour records (without their ray pointers),
+    ``rays``/``dz``  [n, capacity, 2] int32 / [n, capacity] float64 sun rays,
+    ``scalars``    [n, len(PLAN_SCALARS)] and ``luminance`` [n, MAX_PATCHES],
+    ``state``      (CI, firstdaytime, timeadd) after the last hour."""
+
+    def __init__(self, scene, latitude, rows, timestepdec, twater, state):
+        n = len(rows)
+        self.layout = scene.layout.host
+        self.capacity = max(scene.shape) + 2
+        self.records = np.zeros(n, dtype=HOUR_DTYPE)
+        self.rays = np.empty((n, self.capacity, 2), dtype=np.int32)
+        self.dz = np.empty((n, self.capacity), dtype=np.float64)
+        self.scalars = np.empty((n, len(_lib.PLAN_SCALARS)), dtype=np.float64)
+        self.luminance = np.zeros((n, _lib.MAX_PATCHES), dtype=np.float64)
+        self.state = np.array(state, dtype=np.float64)
+        rows = np.ascontiguousarray(rows, dtype=np.float64)
+        const = _plan_scene(scene, latitude)
+
+        def ptr(a):
+            return ctypes.c_void_p(a.ctypes.data)
+
+        _lib.check(_lib.lib().solweig_plan_hours(
+            ctypes.byref(const), ptr(rows), n, float(timestepdec), float(twater), ptr(self.state),
+            ptr(self.records), ptr(self.scalars), ptr(self.rays), ptr(self.dz), self.capacity,
+            ptr(self.luminance)), "solweig_plan_hours")
+
+    def __len__(self):
+        return len(self.records)
+
+    @property
+    def steps(self):
+        """Entries of the longest ray."""
+        return int(self.records["steps"].max()) if len(self) else 0
+
+    def band_lsky(self):
+        """Band sky emittances [n, MAX_BANDS] float64."""
+        return self.scalars[:, _BAND0:]
+
+    def __getitem__(self, i):
+        i = range(len(self))[i]
+        rec, sc = self.records[i], self.scalars[i]
+        hour = _lib.SolweigHour.from_buffer_copy(self.records, i * HOUR_DTYPE.itemsize)
+        ray = lv = None
+        if rec["daytime"]:
+            k = int(rec["steps"])
+            ray = rays.ShadowRay(self.rays[i, :k], self.dz[i, :k], float(rec["ray_low"]), float(rec["ray_high"]),
+                                 int(rec["ray_middle"]))
+            L = self.layout
+            lv = np.column_stack((L.altitude * (np.pi / 180) * (180 / np.pi),
+                                  L.azimuth * (np.pi / 180) * (180 / np.pi), self.luminance[i, :L.count]))
+        v = {name: float(sc[_SCALAR[name]]) for name in _lib.PLAN_SCALARS[:_BAND0]}
+        scal = HourScalars(ea=v["ea"], esky=v["esky"], I0=v["i0"], CI=v["ci"], radI=v["rad_i"], radD=v["rad_d"],
+                           CI_Tg=v["ci_tg"], CI_TgG=v["ci_tgg"], Tgwall=v["tgwall"], lv=lv,
+                           band_lsky=sc[_BAND0:_BAND0 + self.layout.band_counts.size].copy())
+        return hour, ray, scal
+
+
+def _sun_columns(rows, altitude, azimuth, zen):
+    """Fill the sun columns of plan rows [n, len(PLAN_ROW)] (numpy's own sines,
+    on which the digital rays round)."""
+    az, alt = np.asarray(azimuth) * (np.pi / 180.), np.asarray(altitude) * (np.pi / 180.)
+    for name, v in (("altitude", altitude), ("azimuth", azimuth), ("zen", zen), ("sin_az", np.sin(az)),
+                    ("cos_az", np.cos(az)), ("tan_az", np.tan(az)), ("tan_alt", np.tan(alt)),
+                    ("sin_alt", np.sin(alt)), ("cos_alt", np.cos(alt)), ("tan_zen", np.tan(zen))):
+        rows[:, _ROW[name]] = v
 
 
 def hour_plan(scene, latitude, altitude, azimuth, zen, jday, dectime, altmax, ta, rh, rad_g, rad_d,
@@ -664,111 +746,17 @@ def hour_plan(scene, latitude, altitude, azimuth, zen, jday, dectime, altmax, ta
     Returns ``(SolweigHour, ShadowRay or None, HourScalars, next_state)`` where
     next_state = (firstdaytime, timeadd, CI).
     """
-    L = scene.layout.host
-    h = _lib.SolweigHour()
-    _, _, _, snup = _sun.daylen(jday, latitude)
-    ea = 6.107 * 10 ** ((7.5 * ta) / (237.3 + ta)) * (rh / 100.)
-    msteg = 46.5 * (ea / (ta + 273.15))
-    esky = (1 - (1 + msteg) * np.exp(-((1.2 + 3.0 * msteg) ** 0.5))) + CONSTANTS["elvis"]
-    day = altitude > 0
-    CI = ci_prev
-    ray = None
-    lv = None
-    I0 = 0
-    CI_Tg = CI_TgG = None
-    tgwall = 0.0
-    if day:
-        I0, CI, Kt, _, _ = _sun.clearness_index(zen, jday, ta, rh / 100., rad_g, latitude, p_kpa)
-        if CI > 1 or CI == np.inf:
-            CI = 1
-        rad_i, rad_d = _sun.diffuse_fraction(rad_g, altitude, Kt, ta, rh)
-        lv = _sky.perez(zen * (180 / np.pi), azimuth, rad_d, rad_i, jday, L)
-        tgamp_wall = scene.tgk_wall * altmax + scene.tstart_wall
-        frac = dectime - np.floor(dectime)
-        tgwall = tgamp_wall * np.sin((((frac) - snup / 24) / (scene.tmaxlst_wall / 24 - snup / 24)) * np.pi / 2)
-        if tgwall < 0:
-            tgwall = 0
-        radI0, radD0 = _sun.diffuse_fraction(I0, altitude, 1., ta, rh)
-        corr = 0.1473 * np.log(90 - (zen / np.pi * 180)) + 0.3454
-        CI_Tg = (rad_g / radI0) + (1 - corr)
-        if CI_Tg > 1 or CI_Tg == np.inf:
-            CI_Tg = 1
-        radG0 = radI0 * (np.sin(altitude * (np.pi / 180))) + radD0
-        CI_TgG = (rad_g / radG0) + (1 - corr)
-        if CI_TgG > 1 or CI_TgG == np.inf:
-            CI_TgG = 1
-        tgwall = tgwall * CI_TgG
-        ray = rays.shadow_ray(azimuth, altitude, scene.scale, scene.amaxvalue, scene.shape, True)
-        # wave delay flags (all six TsWaveDelay calls share them)
-        if timeadd >= (59 / 1440):
-            weight = math.exp(-33.27 * timeadd)
-            update = 1
-            next_timeadd = timestepdec if timestepdec > (59 / 1440) else 0
-        else:
-            next_timeadd = timeadd + timestepdec
-            weight = math.exp(-33.27 * next_timeadd)
-            update = 0
-        h.firstdaytime = int(firstdaytime)
-        h.wave_update = update
-        h.wave_weight = weight
-        next_state = (0, next_timeadd, CI)
-    else:
-        CI_Tg = CI_TgG = CI
-        next_state = (1, 0, CI)
-    if CI < 0.95:
-        esky = CI * esky + (1 - CI) * 1.
-    h.daytime = int(day)
-    h.altitude, h.azimuth, h.zen = altitude, azimuth, zen
-    h.ta, h.rh, h.ws = ta, rh, ws
-    h.rad_g, h.rad_d, h.rad_i = rad_g, rad_d, rad_i
-    h.psi = psi
-    h.cos_alt = np.cos(altitude * (np.pi / 180))
-    h.sin_alt = np.sin(altitude * (np.pi / 180))
-    h.tan_zen = np.tan(zen)
-    h.esky = esky
-    h.ci_tgg = CI_TgG if day else 0.0
-    h.altmax = altmax
-    h.dectime_frac = dectime - math.floor(dectime)
-    h.snup = snup
-    h.tgwall = tgwall
-    h.twater = twater if twater is not None else 0.0
-    if ray is not None:
-        h.steps = ray.steps
-        h.ray_low, h.ray_high, h.ray_middle = ray.low, ray.high, ray.middle
-    # per-patch weights
-    band_e = _sky.band_emissivity(esky, L)
-    base = SBC * ((ta + 273.15) ** 4)
-    band_lsky = np.zeros(L.band_counts.size)
-    for b in range(L.band_counts.size):
-        k = int(L.band_offsets[b])
-        band_lsky[b] = (band_e[k] * base) / np.pi
-        h.band_lsky[b] = band_lsky[b]
-    if day:
-        lum = lv[:, 2]
-        # sequential float64 sum in patch order, as the reference loop
-        ster_sin = _ster_sin(L)
-        rad_tot = 0.0
-        for lk, w in zip(lum.tolist(), ster_sin):
-            rad_tot += lk * w[0] * w[1]
-        h.rad_tot = rad_tot
-        tan_alt = np.tan(altitude * (np.pi / 180))
-        diff = np.abs(azimuth - L.azimuth)
-        yi = 2 * np.cos(diff * (np.pi / 180)) * tan_alt
-        P = L.count
-        np.ctypeslib.as_array(h.lum)[:P] = lum.astype(np.float32)
-        np.ctypeslib.as_array(h.yi)[:P] = np.where(yi > 0, 0.0, yi)
-        np.ctypeslib.as_array(h.lw_sun_test)[:P] = ((diff > 90) & (diff < 270)).astype(np.uint8)
-    else:
-        h.rad_tot = 1.0
-    coef = (ctypes.c_double * 7)()
-    _lib.check(_lib.lib().solweig_utci_collapse(float(np.float32(ta)), float(np.float32(rh)),
-                                                float(np.float32(ws)), coef), "solweig_utci_collapse")
-    for i in range(7):
-        h.utci[i] = coef[i]
-    h.utci_valid = int(not (np.float32(ta) <= -999 or np.float32(rh) <= -999 or np.float32(ws) <= -999))
-    scal = HourScalars(ea=ea, esky=esky, I0=I0, CI=CI, radI=rad_i, radD=rad_d, CI_Tg=CI_Tg,
-                       CI_TgG=CI_TgG, Tgwall=tgwall, lv=lv, band_lsky=band_lsky)
-    return h, ray, scal, next_state
+    rows = np.zeros((1, len(_lib.PLAN_ROW)))
+    _sun_columns(rows, altitude, azimuth, zen)
+    for name, v in (("jday", jday), ("dectime", dectime), ("altmax", altmax), ("ta", ta), ("rh", rh),
+                    ("rad_g", rad_g), ("rad_d", rad_d), ("rad_i", rad_i), ("p_kpa", p_kpa), ("ws", ws),
+                    ("psi", psi)):
+        rows[0, _ROW[name]] = v
+    plan = DayPlan(scene, latitude, rows, timestepdec, twater if twater is not None else 0.0,
+                   (ci_prev, firstdaytime, timeadd))
+    h, ray, scal = plan[0]
+    ci, firstdaytime, timeadd = plan.state
+    return h, ray, scal, (int(firstdaytime), float(timeadd), float(ci))
 
 
 STEP_OUTPUTS = ("tmrt", "utci", "kdown", "kup", "ldown", "lup", "shadow", "tg", "keast", "ksouth",
@@ -810,6 +798,22 @@ class HourBuffers:
         raw = np.frombuffer(_lib.struct_bytes(hour), dtype=np.uint8)
         self.h_host.numpy()[slot * self.hsize:(slot + 1) * self.hsize] = raw
 
+    def put_plan(self, plan, first=0):
+        """``put`` of every hour of a DayPlan into the slots from ``first`` on;
+        returns the entries of the longest ray."""
+        n, k = len(plan), plan.steps
+        if k > self.kmax:
+            raise ValueError("sun ray longer than the ray buffer")
+        self.r_host.numpy()[first:first + n, :k] = plan.rays[:, :k]
+        self.z_host.numpy()[first:first + n, :k] = plan.dz[:, :k]
+        rec = self.h_host.numpy().view(HOUR_DTYPE)[first:first + n]
+        rec[:] = plan.records
+        slots = np.arange(first, first + n, dtype=np.uint64) * np.uint64(self.kmax)
+        steps = plan.records["steps"] > 0
+        rec["ray_dxdy"] = np.where(steps, np.uint64(self.r_dev.data_ptr()) + slots * np.uint64(8), np.uint64(0))
+        rec["ray_dz"] = np.where(steps, np.uint64(self.z_dev.data_ptr()) + slots * np.uint64(8), np.uint64(0))
+        return k
+
     def upload(self, first, count, steps):
         """Async copy of slots [first, first + count) to the device."""
         hs = self.hsize
@@ -827,31 +831,28 @@ class HourBuffers:
         return ctypes.c_void_p(self.h_dev.data_ptr())
 
 
-def plan_hours(scene, met, latitude, longitude, site_altitude, utc):
-    """FP64 host plan of the rows of one day, yielded row by row as
-    (SolweigHour, ShadowRay|None, HourScalars): the sun positions of all rows
-    first, then each row's scalars (the clearness index and the wave-delay
-    clock carry from row to row)."""
+def plan_day(scene, met, latitude, longitude, site_altitude, utc, sol=None):
+    """FP64 host plan of every row of one day (:class:`DayPlan`): the sun
+    positions of all rows (``sol``, when already known), then the scalars, the
+    clearness index and the wave-delay clock carrying from row to row."""
     met = np.asarray(met, dtype=np.float64)
-    sol = _sun.metdata(met, latitude, longitude, site_altitude, utc)
-    dectime = sol.dectime
-    timestepdec = (dectime[1] - dectime[0]) if len(met) > 1 else 1 / 24.
-    twater = float(np.mean(met[:, 11])) if scene.landcover else None
-    firstdaytime, timeadd, CI = 1, 0.0, 1.0
-    for i in range(len(met)):
-        if dectime[i] - np.floor(dectime[i]) == 0:
-            CI = 1.
-        psi = _leaf_psi(met[i, 1])
-        h, ray, scal, (firstdaytime, timeadd, CI) = hour_plan(
-            scene, latitude, sol.altitude[i], sol.azimuth[i], sol.zen[i], sol.jday[i], dectime[i],
-            sol.altmax[i], met[i, 11], met[i, 10], met[i, 14], met[i, 21], met[i, 22], met[i, 12],
-            met[i, 9], psi, CI, firstdaytime, timeadd, timestepdec, twater)
-        yield h, ray, scal
+    if sol is None:
+        sol = _sun.metdata(met, latitude, longitude, site_altitude, utc)
+    step = (sol.dectime[1] - sol.dectime[0]) if len(met) > 1 else 1 / 24.
+    return DayPlan(scene, latitude, plan_rows(met, sol), step, float(np.mean(met[:, 11])) if scene.landcover else 0.0,
+                   (1.0, 1.0, 0.0))
 
 
-def plan_day(scene, met, latitude, longitude, site_altitude, utc):
-    """FP64 host plan of every row of one day: [(SolweigHour, ShadowRay|None, HourScalars)]."""
-    return list(plan_hours(scene, met, latitude, longitude, site_altitude, utc))
+def plan_rows(met, sol):
+    """Rows of the host plan [n, len(PLAN_ROW)] from forcing rows and their sun positions."""
+    rows = np.zeros((len(met), len(_lib.PLAN_ROW)))
+    _sun_columns(rows, sol.altitude, sol.azimuth, sol.zen)
+    for name, v in (("jday", sol.jday), ("dectime", sol.dectime), ("altmax", sol.altmax), ("ta", met[:, 11]),
+                    ("rh", met[:, 10]), ("rad_g", met[:, 14]), ("rad_d", met[:, 21]), ("rad_i", met[:, 22]),
+                    ("p_kpa", met[:, 12]), ("ws", met[:, 9]), ("psi", [_leaf_psi(doy) for doy in met[:, 1]]),
+                    ("new_day", sol.dectime == np.floor(sol.dectime))):
+        rows[:, _ROW[name]] = v
+    return rows
 
 
 def outputs_struct(outputs, index=None):
@@ -862,9 +863,7 @@ def outputs_struct(outputs, index=None):
 
 
 class DayRunner:
-    """Plain form: one host plan, one hour-record upload and one kernel pair
-    per hour, launched as the hours are planned (the host plans hour h+1
-    while the GPU runs hour h)."""
+    """Plain form: the day's hour records uploaded, then three kernels per hour."""
 
     def __init__(self, scene, latitude, longitude, site_altitude=3.0, utc=0.0):
         self.scene = scene
@@ -900,10 +899,9 @@ class DayRunner:
         return {k: torch.empty((nrows,) + self.scene.shape, dtype=torch.float32, device=self.scene.device)
                 for k in outputs}
 
-    def _put(self, slot, hour, ray, scal):
-        """Stage hour record ``slot`` and copy it to the device."""
-        self.buffers.put(slot, hour, ray)
-        self.buffers.upload(slot, 1, ray.steps if ray is not None else 1)
+    def _stage(self, plan):
+        """Stage the hour records of a day and copy them to the device."""
+        self.buffers.upload(0, len(plan), self.buffers.put_plan(plan))
 
     def _outputs_struct(self, res, index):
         return outputs_struct(res, index)
@@ -913,39 +911,28 @@ class DayRunner:
         met = np.asarray(met, dtype=np.float64)
         if len(met) > self.buffers.hours:
             raise ValueError(f"at most {self.buffers.hours} rows per day")
-        sol = _sun.metdata(met, self.latitude, self.longitude, self.site_altitude, self.utc)
-        dectime = sol.dectime
-        timestepdec = (dectime[1] - dectime[0]) if len(met) > 1 else 1 / 24.
-        twater = float(np.mean(met[:, 11])) if self.scene.landcover else None
+        plan = plan_day(self.scene, met, self.latitude, self.longitude, self.site_altitude, self.utc)
         res = self._alloc_outputs(outputs, len(met))
         self.buffers.wait_free()
+        self._stage(plan)
         self.reset_state()
-        firstdaytime, timeadd, CI = 1, 0.0, 1.0
-        scalars = []
-        for i in range(len(met)):
-            if dectime[i] - np.floor(dectime[i]) == 0:
-                CI = 1.
-            psi = _leaf_psi(met[i, 1])
-            h, ray, scal, (firstdaytime, timeadd, CI) = hour_plan(
-                self.scene, self.latitude, sol.altitude[i], sol.azimuth[i], sol.zen[i], sol.jday[i],
-                dectime[i], sol.altmax[i], met[i, 11], met[i, 10], met[i, 14], met[i, 21],
-                met[i, 22], met[i, 12], met[i, 9], psi, CI, firstdaytime, timeadd, timestepdec,
-                twater)
-            self._put(i, h, ray, scal)
+        for i in range(len(plan)):
             self._launch(i, self._outputs_struct(res, i), stream)
-            scalars.append(scal)
         self.buffers.mark()
-        self.last_scalars = scalars
+        self.last_plan = plan
         return res
+
+    @property
+    def last_scalars(self):
+        """HourScalars of the rows of the last day."""
+        return [p[2] for p in self.last_plan]
 
     def profile_day(self, met):
         """Per-kernel device time of one day: {kernel: {ms, launches, bytes_per_launch}}."""
         sc = self.scene
         plan = plan_day(sc, met, self.latitude, self.longitude, self.site_altitude, self.utc)
         self.buffers.wait_free()
-        for i, (h, ray, _) in enumerate(plan):
-            self.buffers.put(i, h, ray)
-        self.buffers.upload(0, len(plan), self.buffers.kmax)
+        self._stage(plan)
         self.reset_state()
         out = {k: torch.empty(sc.shape, dtype=torch.float32, device=sc.device) for k in ("tmrt", "utci")}
         o = outputs_struct(out)
@@ -1050,12 +1037,13 @@ class DayRunner64(DayRunner):
             setattr(out, k, (t[index] if index is not None else t).data_ptr())
         return out
 
-    def _put(self, slot, hour, ray, scal):
-        super()._put(slot, hour, ray, scal)
-        n = self.h64size
-        raw = np.frombuffer(_lib.struct_bytes(hour64_record(self.scene, hour, scal)), dtype=np.uint8)
-        self.h64_host.numpy()[slot * n:(slot + 1) * n] = raw
-        self.h64_dev[slot * n:(slot + 1) * n].copy_(self.h64_host[slot * n:(slot + 1) * n], non_blocking=True)
+    def _stage(self, plan):
+        super()._stage(plan)
+        n = len(plan)
+        rec = self.h64_host.numpy().view(np.float64).reshape(-1, _lib.MAX_PATCHES + _lib.MAX_BANDS)
+        rec[:n, :_lib.MAX_PATCHES] = plan.luminance
+        rec[:n, _lib.MAX_PATCHES:] = plan.band_lsky()
+        self.h64_dev[:n * self.h64size].copy_(self.h64_host[:n * self.h64size], non_blocking=True)
 
     def _launch(self, slot, out_struct, stream=None):
         sc = self.scene

@@ -25,7 +25,8 @@ import numpy as np
 import torch
 
 from . import _lib
-from .engine import HourBuffers, device_ptr, plan_day, stream_handle
+from . import sun as _sun
+from .engine import DayPlan, HourBuffers, _ROW, device_ptr, plan_day, plan_rows, stream_handle
 
 __all__ = ["DayGradient", "DailyUTCI", "HOUR_FIELDS", "FORCING_COLUMNS"]
 
@@ -35,12 +36,13 @@ FORCING_COLUMNS = {"ta": 11, "rh": 10, "ws": 9}  # UMEP forcing table columns
 _OBJECTIVES = {"utci": 0, "tmrt": 1}
 
 
-def _hour_vector(h, scal, patches):
-    """FP64 values of the hour scalars the device consumes (HOUR_FIELDS + lum[P])."""
-    band = scal.band_lsky if scal.band_lsky is not None else np.zeros(8)
-    v = [h.ta, h.rad_i, h.rad_d, h.rad_tot, h.ci_tgg, h.tgwall] + list(np.resize(band, 8)) + list(h.utci)
-    lum = scal.lv[:, 2] if (h.daytime and scal.lv is not None) else np.zeros(patches)
-    return np.asarray(v, dtype=np.float64), np.asarray(lum, dtype=np.float64)
+def _hour_vectors(plan, patches):
+    """FP64 values of the hour scalars the device consumes (HOUR_FIELDS) and the
+    luminances of every hour of a plan: [n, 21], [n, P]."""
+    rec = plan.records
+    scalars = [rec[name] for name in ("ta", "rad_i", "rad_d", "rad_tot", "ci_tgg", "tgwall")]
+    return (np.concatenate([np.stack(scalars, axis=1), plan.band_lsky(), rec["utci"]], axis=1),
+            plan.luminance[:, :patches])
 
 
 def _utci_coefficients(ta, rh, ws):
@@ -74,9 +76,7 @@ class DayGradient:
             raise ValueError(f"expected {self.hours} forcing rows, got {len(met)}")
         plan = plan_day(self.scene, met, self.latitude, self.longitude, self.site_altitude, self.utc)
         self.buffers.wait_free()
-        for i, (h, ray, _) in enumerate(plan):
-            self.buffers.put(i, h, ray)
-        self.buffers.upload(0, self.hours, self.buffers.kmax)
+        self.buffers.upload(0, self.hours, self.buffers.put_plan(plan))
         return plan
 
     def _params(self, albedo, emissivity, transmissivity):
@@ -136,10 +136,21 @@ class DayGradient:
 
     def forcing_jacobian(self, met, delta=None):
         """{var: (d fields [H(src), H, 21], d lum [H(src), H, P])}: central
-        differences of the FP64 plan with respect to each hour's forcing."""
+        differences of the FP64 plan with respect to each hour's forcing.  The
+        sun positions do not depend on it, and an hour's forcing reaches later
+        hours only through the clearness index that the night carries on, so
+        each difference plans its hour and the night hours after it."""
         met = np.asarray(met, dtype=np.float64)
         delta = delta or {"ta": 1e-4, "rh": 1e-3, "ws": 1e-4}
         H, P = self.hours, self.patches
+        sol = _sun.metdata(met, self.latitude, self.longitude, self.site_altitude, self.utc)
+        step = (sol.dectime[1] - sol.dectime[0]) if H > 1 else 1 / 24.
+        rows = plan_rows(met, sol)
+        states = [(1.0, 1.0, 0.0)]  # before each hour
+        for i in range(H):
+            states.append(tuple(DayPlan(self.scene, self.latitude, rows[i:i + 1], step, 0.0, states[-1]).state))
+        day = sol.altitude > 0
+        reach = [src + 1 + int(np.argmax(np.r_[day[src + 1:], True])) for src in range(H)]
         out = {}
         for var, col in FORCING_COLUMNS.items():
             dF = np.zeros((H, H, len(HOUR_FIELDS)))
@@ -148,18 +159,15 @@ class DayGradient:
             for src in range(H):
                 vecs = []
                 for sgn in (1.0, -1.0):
-                    m = met.copy()
-                    m[src, col] += sgn * d
-                    plan = plan_day(self.scene, m, self.latitude, self.longitude, self.site_altitude, self.utc)
-                    vecs.append([_hour_vector(h, s, P) for h, _, s in plan])
-                for hh in range(H):
-                    dF[src, hh] = (vecs[0][hh][0] - vecs[1][hh][0]) / (2 * d)
-                    dL[src, hh] = (vecs[0][hh][1] - vecs[1][hh][1]) / (2 * d)
+                    part = rows[src:reach[src]].copy()
+                    part[0, _ROW[var]] = met[src, col] + sgn * d
+                    vecs.append(_hour_vectors(DayPlan(self.scene, self.latitude, part, step, 0.0, states[src]), P))
+                dF[src, src:reach[src]] = (vecs[0][0] - vecs[1][0]) / (2 * d)
+                dL[src, src:reach[src]] = (vecs[0][1] - vecs[1][1]) / (2 * d)
                 # UTCI coefficients: FP64 collapse (the plan rounds its inputs to float32)
                 ta, rh, ws = met[src, 11], met[src, 10], met[src, 9]
-                args = {"ta": [ta, rh, ws], "rh": [ta, rh, ws], "ws": [ta, rh, ws]}[var]
                 k = {"ta": 0, "rh": 1, "ws": 2}[var]
-                a_p, a_m = list(args), list(args)
+                a_p, a_m = [ta, rh, ws], [ta, rh, ws]
                 a_p[k] += d
                 a_m[k] -= d
                 dF[src, :, 14:21] = 0.0

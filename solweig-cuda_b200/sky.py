@@ -88,6 +88,7 @@ class PatchLayout:
         self.steradian = omega
         self.cos_alt = np.cos(alt * _D2R)
         self.sin_alt = np.sin(alt * _D2R)
+        self.cos_zen = np.cos((90 - alt) * _D2R)
         # Cardinal direction cosines used by the longwave per-direction sums
         # (define_patch_characteristics, src/umep_solweig.py:1262-1273).
         self.cardinal = np.column_stack([
