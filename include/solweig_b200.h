@@ -244,6 +244,15 @@ int solweig_svf_ex(const double* dsm, const double* vegdem, const double* vegdem
  * replace the offset and dz tables in the walks when capacity <= max(rows,
  * cols) + 2; the masks and planes are identical. */
 int64_t solweig_svf_work_bytes(int rows, int cols);
+/* The patches' visibility rays (src/svf.py:47-75) built on the device: host
+ * arrays [patches] of the azimuth's sine, cosine and tangent, of
+ * tan(altitude) / scale and of whether the columns are the major axis in;
+ * ray_dxdy [patches][capacity][2], ray_dz [patches][capacity] and lengths
+ * [patches] out (entries past a ray's length are not written).  amax: the
+ * height that ends a ray; a ray longer than capacity is cut there. */
+int solweig_svf_ray_tables(const double* sin_az, const double* cos_az, const double* tan_az, const double* rise,
+                           const uint8_t* ymajor, int patches, int rows, int cols, double amax, int capacity,
+                           int32_t* ray_dxdy, double* ray_dz, int32_t* lengths, void* stream);
 int solweig_svf_ex2(const double* dsm, const double* vegdem, const double* vegdem2,
                     const void* geo32, const uint8_t* flags, int rows, int cols, int patches,
                     int capacity, const int32_t* ray_dxdy, const double* ray_dz,

@@ -17,6 +17,7 @@ from __future__ import annotations
 import ctypes
 import math
 from dataclasses import dataclass
+from functools import lru_cache
 
 import numpy as np
 import torch
@@ -143,6 +144,44 @@ class SkyLayout:
         return self._device[key]
 
 
+@lru_cache(maxsize=4)
+def sky_layout(patch_option):
+    """The (constant) layout of ``patch_option``, built once."""
+    return SkyLayout(patch_option)
+
+
+def svf_ray_tables(patch_option, shape, amaxvalue, scale, device, stream=None):
+    """The patches' visibility rays on the device (``solweig_svf_ray_tables``):
+    (dxdy [P, capacity, 2], dz [P, capacity], lengths [P], capacity)."""
+    if not amaxvalue == amaxvalue:
+        raise ValueError("amaxvalue is not a number")
+    trig, ymajor = rays.svf_ray_constants(patch_option)
+    P = ymajor.size
+    cap = rays.svf_ray_capacity(patch_option, shape, amaxvalue, scale)
+    rise = np.ascontiguousarray(trig[3] / scale)
+    dxdy = torch.empty((P, cap, 2), dtype=torch.int32, device=device)
+    dz = torch.empty((P, cap), dtype=torch.float64, device=device)
+    lengths = torch.empty(P, dtype=torch.int32, device=device)
+    host = [ctypes.c_void_p(a.ctypes.data) for a in (trig[0], trig[1], trig[2], rise, ymajor)]
+    _lib.check(_lib.lib().solweig_svf_ray_tables(
+        *host, P, shape[0], shape[1], float(amaxvalue), cap, device_ptr(dxdy), device_ptr(dz), device_ptr(lengths),
+        stream_handle(stream)), "solweig_svf_ray_tables")
+    return dxdy, dz, lengths, cap
+
+
+def packed_geometry(dsm, vegdem, vegdem2):
+    """(dsm, vegdem, vegdem2, 0) as float4 per pixel when all three rasters
+    are exactly representable in float32 (the sweeps then load one sample
+    per step); None otherwise."""
+    stack = torch.stack((dsm, vegdem, vegdem2), dim=-1)
+    packed = stack.to(torch.float32)
+    if not bool(torch.equal(packed.to(torch.float64), stack)):
+        return None
+    geo = torch.zeros(dsm.shape + (4,), dtype=torch.float32, device=dsm.device)
+    geo[..., :3] = packed
+    return geo
+
+
 def _upload(arr, dtype, device):
     return torch.from_numpy(np.ascontiguousarray(arr, dtype=dtype)).to(device, non_blocking=False)
 
@@ -247,11 +286,10 @@ def wall_aspect(dsm_host, dsm_dev, walls_dev, pixel_size, stream=None):
     return aspect, walls
 
 
-def wall_aspect_device(dsm_host, dsm_dev, walls_dev, pixel_size, stream=None, host_work=None):
+def wall_aspect_device(dsm_host, dsm_dev, walls_dev, pixel_size, stream=None):
     """Wall aspect in degrees as a float64 device tensor (``src/walls.py:83-129``):
     the template kernel on the device, the gradient fall-back only at the few
-    wall pixels the templates leave unresolved (from ``dsm_host`` when given).
-    ``host_work`` (optional) runs on the host while the template kernel runs."""
+    wall pixels the templates leave unresolved (from ``dsm_host`` when given)."""
     rows, cols = dsm_dev.shape
     key = float(pixel_size)
     if key not in _TEMPLATE_CACHE:
@@ -260,8 +298,6 @@ def wall_aspect_device(dsm_host, dsm_dev, walls_dev, pixel_size, stream=None, ho
     mask = walls_dev > 0
     aspect = torch.zeros_like(dsm_dev)
     if not bool(mask.any()):
-        if host_work is not None:
-            host_work()
         return aspect
     if rows > 2 * radius + 2 and cols > 2 * radius + 2:
         dev = dsm_dev.device
@@ -270,8 +306,6 @@ def wall_aspect_device(dsm_host, dsm_dev, walls_dev, pixel_size, stream=None, ho
             device_ptr(dsm_dev), device_ptr(walls_dev), device_ptr(aspect), rows, cols, radius,
             device_ptr(t[0][0]), device_ptr(t[0][1]), device_ptr(t[1][0]), device_ptr(t[1][1]),
             device_ptr(t[2][0]), device_ptr(t[2][1]), stream_handle(stream)), "solweig_wall_aspect")
-    if host_work is not None:
-        host_work()
     unresolved = torch.nonzero((mask & (aspect == 0)).flatten()).flatten()
     if unresolved.numel():
         host = dsm_host if dsm_host is not None else dsm_dev.cpu().numpy()
@@ -329,30 +363,25 @@ class Scene:
         self.pixels = self.rows * self.cols
         self.pixel_size = float(pixel_size)
         self.scale = 1 / self.pixel_size
-        self.layout = SkyLayout(patch_option)
+        self.layout = sky_layout(int(patch_option))
         self.patch_option = int(patch_option)
         L = _lib.lib()
         st = stream_handle(stream)
         n = self.pixels
-        # Raise / clip semantics of src/series.py:252-291 (host syncs, so before
-        # the wall kernels: the SVF rays are built on the host while they run).
-        raise_dsm = max(0.0, -float(dsm_in.min()))
-        raise_dem = max(0.0, -float(dem_in.min()))
-        a_min, a_max = float(dsm_in.min()) + raise_dsm, float(dsm_in.max()) + raise_dsm
-        t1_max = float(trees_in.clamp_min(0.).max())
+        # Raise / clip semantics of src/series.py:252-291 (one host sync).
+        dsm_lo, dsm_hi, dem_lo, trees_hi = torch.stack(
+            (dsm_in.min(), dsm_in.max(), dem_in.min(), trees_in.clamp_min(0.).max())).tolist()
+        raise_dsm = max(0.0, -dsm_lo)
+        raise_dem = max(0.0, -dem_lo)
+        a_min, a_max, t1_max = dsm_lo + raise_dsm, dsm_hi + raise_dsm, trees_hi
         self.amaxvalue = float(max(a_max - a_min, t1_max))
         self.dsm_max = a_max
         self.hmax = float(a_max + max(t1_max, 0.0))
-        svf_ray_tables = []
-
-        def build_svf_rays():
-            svf_ray_tables.append(rays.svf_rays(patch_option, self.shape, self.amaxvalue, self.scale))
-
         # Walls from the unraised DSM, rounded through float32 (src/series.py:213-236).
         if walls is None:
             walls_dev = wall_heights_device(dsm_in, wall_threshold, stream)
             aspect_dev = wall_aspect_device(dsm if isinstance(dsm, np.ndarray) else None, dsm_in, walls_dev,
-                                            pixel_size, stream, host_work=build_svf_rays)
+                                            pixel_size, stream)
         else:
             walls_dev = _raster_to_device(walls, dev)
             aspect_dev = _raster_to_device(aspect, dev)
@@ -393,13 +422,8 @@ class Scene:
         del dsm_in, trees_in, dem_in, lc_in
         self.has_water = int(bool(((self.flags & 4) != 0).any().item())) if landcover is not None else 0
         # Sky view factor: bit-packed visibility + the 16 reduce planes.
-        if not svf_ray_tables:
-            build_svf_rays()
-        dxdy, dz, lengths, cap = svf_ray_tables[0]
-        self.svf_steps = int(lengths.sum())
-        t_dxdy = _upload(dxdy, np.int32, dev)
-        t_dz = _upload(dz, np.float64, dev)
-        t_len = _upload(lengths, np.int32, dev)
+        t_dxdy, t_dz, t_len, cap = svf_ray_tables(patch_option, self.shape, self.amaxvalue, self.scale, dev, stream)
+        self._svf_lengths = t_len
         nb = self.layout.struct.nbands
         self.masks = torch.empty((2 * _lib.MASK_WORDS, self.rows, self.cols), dtype=torch.int32,
                                  device=dev)
@@ -407,7 +431,7 @@ class Scene:
         self.veg_sums = torch.empty((4, self.rows, self.cols), **f32)
         self.sky_band_counts = torch.empty((nb, self.rows, self.cols), dtype=torch.uint8, device=dev)
         lay = self.layout
-        self.geo32 = self._packed_geometry()
+        self.geo32 = packed_geometry(self.dsm, self.vegdem, self.vegdem2)
         self._geo_checked = True
         # GVF step offsets, uploaded before the SVF launch: nothing after it
         # waits for the device, so the host returns (and can plan the day)
@@ -425,7 +449,7 @@ class Scene:
             lay.sectors.ctypes.data_as(ctypes.c_void_p), CONSTANTS["transVeg"],
             device_ptr(self.masks), device_ptr(planes), device_ptr(self.veg_sums),
             device_ptr(self.sky_band_counts), device_ptr(svf_work), svf_work.numel(), st), "solweig_svf")
-        del t_dxdy, t_dz, t_len, svf_work
+        del t_dxdy, t_dz, svf_work
         # Derived statics after the float32 round trip of the SVF planes.
         self.svf32 = torch.empty((15, self.rows, self.cols), **f32)
         self.svfbuveg = torch.empty(self.shape, **f32)
@@ -460,7 +484,7 @@ class Scene:
         self.scale = float(inputs["scale"])
         self.pixel_size = 1.0 / self.scale
         self.patch_option = int(inputs.get("patch_option", 2))
-        self.layout = SkyLayout(self.patch_option)
+        self.layout = sky_layout(self.patch_option)
         L = _lib.lib()
         st = stream_handle(stream)
 
@@ -576,22 +600,10 @@ class Scene:
         s.has_water = self.has_water
         s.hmax = self.hmax
         if getattr(self, "geo32", None) is None and not getattr(self, "_geo_checked", False):
-            self.geo32 = self._packed_geometry()
+            self.geo32 = packed_geometry(self.dsm, self.vegdem, self.vegdem2)
         self._geo_checked = True
         s.geo32 = self.geo32.data_ptr() if self.geo32 is not None else None
         return s
-
-    def _packed_geometry(self):
-        """(dsm, vegdem, vegdem2, 0) as float4 per pixel when all three rasters
-        are exactly representable in float32 (the sweep then loads one sample
-        per step); None otherwise."""
-        stack = torch.stack((self.dsm, self.vegdem, self.vegdem2), dim=-1)
-        packed = stack.to(torch.float32)
-        if not bool(torch.equal(packed.to(torch.float64), stack)):
-            return None
-        geo = torch.zeros(self.shape + (4,), dtype=torch.float32, device=self.dsm.device)
-        geo[..., :3] = packed
-        return geo
 
     def svfbuveg64(self):
         """svf - (1 - svfveg)(1 - transVeg) in float64 from the float32-rounded
@@ -603,6 +615,11 @@ class Scene:
             t = (svf - (1.0 - veg) * (1.0 - CONSTANTS["transVeg"])).contiguous()
             self._svfbuveg64 = t
         return t
+
+    @property
+    def svf_steps(self):
+        """Steps of the 153 visibility rays together."""
+        return int(self._svf_lengths.sum())
 
     @property
     def walls_host(self):

@@ -11,10 +11,11 @@ device compares the very same float64 values.
 from __future__ import annotations
 
 import math
+from functools import lru_cache
 
 import numpy as np
 
-__all__ = ["ShadowRay", "shadow_ray", "svf_rays", "gvf_offsets", "gvf_face_windows",
+__all__ = ["ShadowRay", "shadow_ray", "svf_rays", "svf_ray_constants", "svf_ray_capacity", "gvf_offsets", "gvf_face_windows",
            "sun_window", "svf_patch_directions"]
 
 _PI4 = np.pi / 4
@@ -103,6 +104,29 @@ def svf_patch_directions(patch_option):
     return azimuth, altitude, counts
 
 
+@lru_cache(maxsize=4)
+def svf_ray_constants(patch_option):
+    """Per patch (sin, cos, tan) of the azimuth, tan of the altitude and whether
+    the columns are the ray's major axis: what the device builds the rays of
+    :func:`svf_rays` from (``solweig_svf_ray_tables``)."""
+    azimuth, altitude, _ = svf_patch_directions(patch_option)
+    az = [a * (np.pi / 180.) for a in azimuth]
+    trig = np.array([[np.sin(a), np.cos(a), np.tan(a), np.tan(e * (np.pi / 180.))] for a, e in zip(az, altitude)])
+    return np.ascontiguousarray(trig.T), np.array([_ymajor(a) for a in az], dtype=np.uint8)
+
+
+def svf_ray_capacity(patch_option, shape, amaxvalue, scale):
+    """Steps that hold the longest ray of :func:`svf_rays`: heights grow linearly
+    with the step, so a ray ends within two steps past amaxvalue / rise."""
+    (s, c, _, rise), ymajor = svf_ray_constants(patch_option)
+    capacity = max(shape) + 1
+    if amaxvalue < 0:
+        return 1
+    slope = np.abs(1 / np.where(ymajor, s, c)) * (rise / scale)
+    bound = np.where(slope > 0, np.ceil(amaxvalue / np.where(slope > 0, slope, 1.0)) + 2, capacity)
+    return int(max(1, min(capacity, bound.max())))
+
+
 def svf_rays(patch_option, shape, amaxvalue, scale):
     """Per-patch visibility rays: ``(dxdy [P, cap, 2] int32, dz [P, cap], lengths [P], cap)``.
 
@@ -189,17 +213,17 @@ def gvf_offsets(scale, first=1.0, second=22.0):
     second_steps = int(np.round(second * scale))
     first_steps = int(first_steps)
     out = np.zeros((18, max(second_steps, 1), 2), dtype=np.int32)
+    n = np.arange(second_steps)
     for j, deg in enumerate(np.arange(5, 359, 20)):
         az = deg * (np.pi / 180)
         s, c, t = np.sin(az), np.cos(az), np.tan(az)
-        for n in range(second_steps):
-            if _ymajor(az):
-                dy = np.sign(s) * n
-                dx = -np.sign(c) * np.abs(np.round(n / t))
-            else:
-                dy = np.sign(s) * abs(round(n * t))
-                dx = -np.sign(c) * n
-            out[j, n] = int(dx), int(dy)
+        if _ymajor(az):
+            dy = np.sign(s) * n
+            dx = -np.sign(c) * np.abs(np.round(n / t))
+        else:
+            dy = np.sign(s) * np.abs(np.round(n * t))
+            dx = -np.sign(c) * n
+        out[j, :second_steps, 0], out[j, :second_steps, 1] = dx, dy
     return np.ascontiguousarray(out), first_steps, second_steps
 
 

@@ -13,8 +13,8 @@ import ctypes
 import numpy as np
 import torch
 
-from . import _lib, rays
-from .engine import CONSTANTS, SkyLayout, _as_device, _upload, device_ptr, stream_handle
+from . import _lib
+from .engine import CONSTANTS, _as_device, device_ptr, packed_geometry, sky_layout, stream_handle, svf_ray_tables
 
 __all__ = ["svf_calculator", "compute_diffsh", "DEFAULT_ANGLE_BATCH"]
 
@@ -36,11 +36,10 @@ def svf_calculator(patch_option, amaxvalue, a, vegdem, vegdem2, bush, scale,
     shape = (rows, cols)
     a, top, bot, bu = (_as_device(x, torch.float64, dev, shape) for x in (a, vegdem, vegdem2, bush))
     flags = ((bu > 1).to(torch.uint8) << 1).contiguous()
-    hmax = float(max(a.max().item(), top.max().item(), bot.max().item()))
-    layout = SkyLayout(patch_option)
-    dxdy, dz, lengths, cap = rays.svf_rays(patch_option, shape, float(amaxvalue), float(scale))
-    t_dxdy, t_dz, t_len = (_upload(dxdy, np.int32, dev), _upload(dz, np.float64, dev),
-                           _upload(lengths, np.int32, dev))
+    hmax = torch.stack((a.max(), top.max(), bot.max())).max().item()
+    layout = sky_layout(int(patch_option))
+    geo32 = packed_geometry(a, top, bot)
+    t_dxdy, t_dz, t_len, cap = svf_ray_tables(patch_option, shape, float(amaxvalue), float(scale), dev)
     P = layout.struct.patches
     masks = torch.empty((2 * _lib.MASK_WORDS, rows, cols), dtype=torch.int32, device=dev)
     planes = torch.empty((16, rows, cols), dtype=torch.float64, device=dev)
@@ -48,12 +47,15 @@ def svf_calculator(patch_option, amaxvalue, a, vegdem, vegdem2, bush, scale,
     counts = torch.empty((layout.struct.nbands, rows, cols), dtype=torch.uint8, device=dev)
     st = stream_handle()
     L = _lib.lib()
-    _lib.check(L.solweig_svf(
-        device_ptr(a), device_ptr(top), device_ptr(bot), device_ptr(flags), rows, cols, P, cap,
+    # ray ceilings, exits and step records of one patch word at a time
+    work = torch.empty(int(L.solweig_svf_work_bytes(rows, cols)), dtype=torch.uint8, device=dev)
+    _lib.check(L.solweig_svf_ex2(
+        device_ptr(a), device_ptr(top), device_ptr(bot), device_ptr(geo32), device_ptr(flags), rows, cols, P, cap,
         device_ptr(t_dxdy), device_ptr(t_dz), device_ptr(t_len), hmax, ctypes.byref(layout.struct),
         layout.band_weights.ctypes.data_as(ctypes.c_void_p),
         layout.sectors.ctypes.data_as(ctypes.c_void_p), float(transmissivity), device_ptr(masks),
-        device_ptr(planes), device_ptr(veg_sums), device_ptr(counts), st), "solweig_svf")
+        device_ptr(planes), device_ptr(veg_sums), device_ptr(counts), device_ptr(work), work.numel(), st), "solweig_svf")
+    del work, geo32  # before the cubes, which take seven times their memory
     cubes = [torch.empty((rows, cols, P), dtype=torch.float32, device=dev) for _ in range(3)]
     _lib.check(L.solweig_svf_unpack(device_ptr(masks), rows * cols, P, device_ptr(cubes[0]),
                                     device_ptr(cubes[1]), device_ptr(cubes[2]), st), "solweig_svf_unpack")
