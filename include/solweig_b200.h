@@ -358,6 +358,15 @@ int solweig_step64(const SolweigScene* scene, const double* svfbuveg, const Solw
                    const int32_t* gvf_dxdy /* host [18][second_steps][2] */, int first_steps,
                    int second_steps, double* scratch, void* stream);
 
+/* `count` consecutive hours from `hour` on: planes of hour i at out + i *
+ * hour_stride, scratch of count x SOLWEIG_SCRATCH64_PLANES planes, state carried
+ * through the hours.  solweig_step64 is one hour. */
+int solweig_step64_hours(const SolweigScene* scene, const double* svfbuveg, const SolweigSkyLayout* layout,
+                         const SolweigSky64* sky, const SolweigHour* hours, const SolweigHour64* hours64,
+                         int hour, int count, const SolweigState64* state, const SolweigOutputs64* out,
+                         int64_t hour_stride, const int32_t* gvf_dxdy, int first_steps, int second_steps,
+                         double* scratch, void* stream);
+
 /* Batched day ----------------------------------------------------------------
  * All nhours (<= 64) hours of one day (src/series.py:445-491) in seven
  * launches: shadow sweep and ground view factors for every hour (one launch

@@ -161,7 +161,7 @@ EXPORTED_SYMBOLS = (
     "solweig_patch_sums", "solweig_day_batched_timed", "solweig_day_batched_ex", "solweig_day_batched_part",
     "solweig_day_batched_layout", "solweig_day_grad_work_bytes", "solweig_day_grad_forward",
     "solweig_day_grad_backward", "solweig_svf_ex", "solweig_svf_ex2", "solweig_svf_work_bytes", "solweig_svf_ray_tables",
-    "solweig_gvf_statics", "solweig_gvf_walk_words", "solweig_gvf_walks", "solweig_plan_hours", "solweig_step64", "solweig_struct_sizes64", "solweig_wall_segments_burn",
+    "solweig_gvf_statics", "solweig_gvf_walk_words", "solweig_gvf_walks", "solweig_plan_hours", "solweig_step64_hours", "solweig_step64", "solweig_struct_sizes64", "solweig_wall_segments_burn",
     "solweig_geometry_walls",
 )
 
@@ -196,6 +196,7 @@ def _declare(lib):
         "solweig_gvf": (i32, [P, P, P, P, dbl, dbl, dbl, dbl, dbl, P, i32, i32, P, P, P]),
         "solweig_step": (i32, [P, P, P, i32, P, P, P, i32, i32, P, P]),
         "solweig_step_static_scratch": (i32, [P, P, P, i32, P, P, P, i32, i32, P]),
+        "solweig_step64_hours": (i32, [P, P, P, P, P, P, i32, i32, P, P, i64, P, i32, i32, P, P]),
         "solweig_step64": (i32, [P, P, P, P, P, P, i32, P, P, P, i32, i32, P, P]),
         "solweig_day_batched": (i32, [P, P, P, i32, P, P, i64, P, i32, i32, P, i64, P]),
         "solweig_day_batched_work_bytes": (i64, [i32, i32, i32, i32]),

@@ -912,6 +912,10 @@ class DayRunner:
             sc.first_steps, sc.second_steps, device_ptr(self.scratch), stream_handle(stream)),
             "solweig_step")
 
+    def _launch_day(self, count, res, stream=None):
+        for i in range(count):
+            self._launch(i, self._outputs_struct(res, i), stream)
+
     def _alloc_outputs(self, outputs, nrows):
         return {k: torch.empty((nrows,) + self.scene.shape, dtype=torch.float32, device=self.scene.device)
                 for k in outputs}
@@ -933,8 +937,7 @@ class DayRunner:
         self.buffers.wait_free()
         self._stage(plan)
         self.reset_state()
-        for i in range(len(plan)):
-            self._launch(i, self._outputs_struct(res, i), stream)
+        self._launch_day(len(plan), res, stream)
         self.buffers.mark()
         self.last_plan = plan
         return res
@@ -1016,9 +1019,15 @@ def hour64_record(scene, hour, scal):
 
 class DayRunner64(DayRunner):
     """Plain form with float64 radiation, the reference's ``dtype=float64``
-    (``run.py:27``, ``src/runtime.py:43-49``): one ``solweig_step64`` per hour
-    (shadow fields, ground view factors and radiation in float64), float64
-    thermal state and output planes; UTCI stays float32."""
+    (``run.py:27``, ``src/runtime.py:43-49``): shadow fields, ground view factors
+    and radiation in float64 (``solweig_step64_hours``), float64 thermal state
+    and output planes; UTCI stays float32.
+
+    Hours run in groups whose scratch takes up to GROUP_BYTES (one hour at
+    least), so that small rasters fill the device."""
+
+    GROUP_BYTES = 512 << 20
+
 
     def __init__(self, scene, latitude, longitude, site_altitude=3.0, utc=0.0, hours=24):
         self.scene = scene
@@ -1026,9 +1035,10 @@ class DayRunner64(DayRunner):
         dev = scene.device
         self.state = {k: torch.zeros(scene.shape, dtype=torch.float64, device=dev)
                       for k in _lib.STATE_FIELDS}
-        self.scratch = torch.empty((_lib.SCRATCH64_PLANES, scene.rows, scene.cols), dtype=torch.float64,
-                                   device=dev)
         slots = max(24, int(hours))
+        self.group = max(1, min(slots, self.GROUP_BYTES // (8 * _lib.SCRATCH64_PLANES * scene.pixels)))
+        self.scratch = torch.empty((self.group * _lib.SCRATCH64_PLANES, scene.rows, scene.cols),
+                                   dtype=torch.float64, device=dev)
         self.buffers = HourBuffers(scene, slots)
         self.h64size = ctypes.sizeof(_lib.SolweigHour64)
         self.h64_host = torch.empty(slots * self.h64size, dtype=torch.uint8, pin_memory=True)
@@ -1062,14 +1072,15 @@ class DayRunner64(DayRunner):
         rec[:n, _lib.MAX_PATCHES:] = plan.band_lsky()
         self.h64_dev[:n * self.h64size].copy_(self.h64_host[:n * self.h64size], non_blocking=True)
 
-    def _launch(self, slot, out_struct, stream=None):
+    def _launch_day(self, count, res, stream=None):
         sc = self.scene
-        _lib.check(_lib.lib().solweig_step64(
-            ctypes.byref(sc.struct), device_ptr(self.svfbuveg), device_ptr(self.layout_dev),
-            device_ptr(self.sky64_dev), self.buffers.ptr(), device_ptr(self.h64_dev), slot,
-            ctypes.byref(self.state_struct()), ctypes.byref(out_struct), sc.gvf_host_ptr,
-            sc.first_steps, sc.second_steps, device_ptr(self.scratch), stream_handle(stream)),
-            "solweig_step64")
+        for h0 in range(0, count, self.group):
+            _lib.check(_lib.lib().solweig_step64_hours(
+                ctypes.byref(sc.struct), device_ptr(self.svfbuveg), device_ptr(self.layout_dev),
+                device_ptr(self.sky64_dev), self.buffers.ptr(), device_ptr(self.h64_dev), h0,
+                min(self.group, count - h0), ctypes.byref(self.state_struct()),
+                ctypes.byref(self._outputs_struct(res, h0)), sc.pixels, sc.gvf_host_ptr, sc.first_steps,
+                sc.second_steps, device_ptr(self.scratch), stream_handle(stream)), "solweig_step64_hours")
 
     def profile_day(self, met):
         raise NotImplementedError("profile_day times the float32 kernels; time a DayRunner64 day with events")
