@@ -137,7 +137,7 @@ __device__ BuildingTerms building_terms(const DayTable& T, const PixelStatics<OP
         m_lshd[SOLWEIG_MASK_WORDS];
 #pragma unroll
     for (int w = 0; w < SOLWEIG_MASK_WORDS; ++w) {
-        const uint32_t test = T.test[w];
+        const uint32_t test = T.loop.test[w];
         m_sun[w] = ps.bld[w] & T.suf[isun][w];
         m_shd[w] = ps.bld[w] & T.pre[ishd][w];
         m_lsun[w] = m_sun[w] & test;

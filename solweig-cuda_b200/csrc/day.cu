@@ -48,6 +48,8 @@
 // compare of tan(asvf) with a float64 threshold found by bisection over the
 // doubles, so a pixel-hour needs two short scans from a 256-bucket start
 // table and band popcounts instead of a loop over its building patches.
+#include <algorithm>
+
 #include "day_kernels.cuh"
 
 using namespace solweig;
@@ -383,13 +385,24 @@ int day_batched_impl(const SolweigScene* scene, const SolweigSkyLayout* layout, 
     if (state) ra.state = *state;
     ra.out = *base;
     ra.hour_stride = hour_stride;
+    // A block takes all hours of its pixels; where that leaves the chip idle
+    // (fewer blocks than 2048 threads on each of the SMs), ranges of at least
+    // three hours: a range replays the wave delay up to it, so none is split
+    // off when the ground temperature is wanted or the state is kept.  64 x 48
+    // px: 131 -> 25 us with 8 ranges, 200 x 200 px: 164 -> 45 us.
     const unsigned blocks = blocks_for(px, cfg.rad_threads);
+    const unsigned full = 148u * (2048u / cfg.rad_threads);
+    int ranges = 1;
+    if (!(ra.out.tg || ra.out.tg_out || ra.state.tgmap1 || ra.state.tgout1))
+        ranges = std::max(1, std::min((int)((full + blocks - 1) / blocks), nhours / 3));
+    ra.chunk = (nhours + ranges - 1) / ranges;
+    const dim3 rgrid(blocks, (nhours + ra.chunk - 1) / ra.chunk);
     if (cfg.rad_threads == 128) {
-        if (S.patches == 153) day_radiation_kernel<2, 128><<<blocks, 128, 0, st>>>(S, ra);
-        else day_radiation_kernel<1, 128><<<blocks, 128, 0, st>>>(S, ra);
+        if (S.patches == 153) day_radiation_kernel<2, 128><<<rgrid, 128, 0, st>>>(S, ra);
+        else day_radiation_kernel<1, 128><<<rgrid, 128, 0, st>>>(S, ra);
     } else {
-        if (S.patches == 153) day_radiation_kernel<2, 256><<<blocks, 256, 0, st>>>(S, ra);
-        else day_radiation_kernel<1, 256><<<blocks, 256, 0, st>>>(S, ra);
+        if (S.patches == 153) day_radiation_kernel<2, 256><<<rgrid, 256, 0, st>>>(S, ra);
+        else day_radiation_kernel<1, 256><<<rgrid, 256, 0, st>>>(S, ra);
     }
     SOLWEIG_CHECK_LAUNCH("day_radiation_kernel");
     if (ev) cudaEventRecord(ev[5], st);

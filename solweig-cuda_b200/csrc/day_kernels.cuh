@@ -28,23 +28,30 @@ __host__ __device__ __forceinline__ int canon_off(int n, int k) {
     return (n >> 3) * (kSBO / 2) + (k >> 3) * 64 + (n & 7) * 8 + (k & 7);
 }
 
-// Sunlit / shaded tables of one hour (size a multiple of 16 bytes).
-struct DayTable {
+// What the radiation loop reads of one hour, rounded once from the float64 plan.
+struct alignas(16) HourLoop {
+    float band_down[SOLWEIG_MAX_BANDS], band_side[SOLWEIG_MAX_BANDS];
+    float lw_shade, lw_sun, sw_shade, sw_sun;
+    float rad_d, rad_g, rad_i_sin, rad_i_cos;
+    float rad_ratio, wave_w, tan_zen, night_lup;
+    float night_lup_water, ta;
+    uint32_t flags;     // kHour* bits
+    uint32_t pad;
+    double utci[8];     // 7 coefficients, air temperature
+    uint32_t test[8];   // longwave sun test of the hour
+};
+constexpr uint32_t kHourDay = 1u, kHourFirst = 2u, kHourUpdate = 4u, kHourUtci = 8u;
+
+// Sunlit / shaded tables of one hour.
+struct alignas(16) DayTable {
+    HourLoop loop;
     double tsun[kK];        // sorted: patch sunlit  <=> tan(asvf) <  T_k
     double vshade[kK];      // sorted: patch shaded  <=> tan(asvf) >= V_k
     uint32_t suf[kK + 1][SOLWEIG_MASK_WORDS];  // patches at sorted sunlit positions >= i
     uint32_t pre[kK + 1][SOLWEIG_MASK_WORDS];  // patches at sorted shaded positions <  j
-    uint32_t test[SOLWEIG_MASK_WORDS];         // longwave sun test of the hour
-    uint32_t pad[5];
-    // first sorted position whose threshold is >= bucket boundary i (see
-    // tan_bucket): the counts of thresholds <= t start there for t in bucket i
+    // first sorted position whose sunlit threshold is >= bucket boundary i (see
+    // tan_bucket): the count of thresholds <= t starts there for t in bucket i
     uint8_t sun_start[256];
-    uint8_t shd_start[256];
-    // hour scalars of the radiation loop, rounded once from the float64 plan
-    float band_down[SOLWEIG_MAX_BANDS], band_side[SOLWEIG_MAX_BANDS];
-    float lw_shade, lw_sun, sw_shade, sw_sun, rad_d, rad_g, direct_up, rad_i_sin, rad_i_cos, rad_ratio;
-    float wave_w, tan_zen, night_lup, night_lup_water;
-    float pad2[2];
 };
 
 // 256 buckets of tan(asvf): boundary i = tan(i * pi / 512) for i >= 1,
@@ -111,14 +118,15 @@ __device__ __forceinline__ float band_weighted(const uint32_t (&m)[SOLWEIG_MASK_
     return s;
 }
 
-// Patches of m in each band (popcounts of the band's bit ranges), and the
-// weighted sum of such counts.
+// Sums of wcos over the patches of m, and of wcos and wsin over those of mt.
 template <int OPT>
-__device__ __forceinline__ void band_counts(const uint32_t (&m)[SOLWEIG_MASK_WORDS], float (&c)[8]) {
+__device__ __forceinline__ void band_sums(const uint32_t (&m)[SOLWEIG_MASK_WORDS], const uint32_t (&mt)[SOLWEIG_MASK_WORDS],
+                                          const float* wcos, const float* wsin, float& mc, float& tc, float& ts) {
+    mc = tc = ts = 0.f;
 #pragma unroll
     for (int b = 0; b < 8; ++b) {
         const int lo = Bands<OPT>::off(b), hi = Bands<OPT>::off(b + 1);
-        int n = 0;
+        int n = 0, nt = 0;
 #pragma unroll
         for (int wd = 0; wd < SOLWEIG_MASK_WORDS; ++wd) {
             const int a = lo > wd * 32 ? lo : wd * 32;
@@ -126,16 +134,14 @@ __device__ __forceinline__ void band_counts(const uint32_t (&m)[SOLWEIG_MASK_WOR
             if (a < e) {
                 const uint32_t mask = (e - a == 32) ? 0xffffffffu : (((1u << (e - a)) - 1u) << (a - wd * 32));
                 n += __popc(m[wd] & mask);
+                nt += __popc(mt[wd] & mask);
             }
         }
-        c[b] = (float)n;
+        const float c = wcos[b];
+        mc = fmaf((float)n, c, mc);
+        tc = fmaf((float)nt, c, tc);
+        ts = fmaf((float)nt, wsin[b], ts);
     }
-}
-__device__ __forceinline__ float band_dot(const float (&c)[8], const float* w) {
-    float s = 0.f;
-#pragma unroll
-    for (int b = 0; b < 8; ++b) s = fmaf(c[b], w[b], s);
-    return s;
 }
 
 // Number of entries of the ascending array a[0..n) that are <= t.
@@ -378,7 +384,8 @@ __global__ void __launch_bounds__(kK) day_tables_kernel(const SolweigSkyLayout* 
                                                         const SolweigHour* __restrict__ hours,
                                                         DayTable* __restrict__ tables) {
     __shared__ double ts[kK], vs[kK];
-    __shared__ int perm_t[kK], perm_v[kK];
+    __shared__ double sorted[kK];
+    __shared__ int rank_t[kK], rank_v[kK];
     const SolweigHour& h = hours[blockIdx.x];
     DayTable& T = tables[blockIdx.x];
     const int P = L->patches;
@@ -398,63 +405,74 @@ __global__ void __launch_bounds__(kK) day_tables_kernel(const SolweigSkyLayout* 
             rt += (ts[j] < tk || (ts[j] == tk && j < k)) ? 1 : 0;
             rv += (vs[j] < vk || (vs[j] == vk && j < k)) ? 1 : 0;
         }
-        T.tsun[rt] = tk;
+        T.tsun[rt] = sorted[rt] = tk;
         T.vshade[rv] = vk;
-        perm_t[rt] = k;
-        perm_v[rv] = k;
+        rank_t[k] = rt;
+        rank_v[k] = rv;
     }
     __syncthreads();
+    // position i's masks from the patches' ranks: no patch is looked up by rank,
+    // so every thread reads the same ranks at once
     for (int i = k; i <= P; i += blockDim.x) {
-        uint32_t suf[SOLWEIG_MASK_WORDS] = {0, 0, 0, 0, 0}, pre[SOLWEIG_MASK_WORDS] = {0, 0, 0, 0, 0};
-        for (int r = 0; r < P; ++r) {
-            if (r >= i) suf[perm_t[r] >> 5] |= 1u << (perm_t[r] & 31);
-            if (r < i) pre[perm_v[r] >> 5] |= 1u << (perm_v[r] & 31);
-        }
         for (int w = 0; w < SOLWEIG_MASK_WORDS; ++w) {
-            T.suf[i][w] = suf[w];
-            T.pre[i][w] = pre[w];
+            uint32_t suf = 0u, pre = 0u;
+            for (int b = 0; b < 32 && 32 * w + b < P; ++b) {
+                suf |= (rank_t[32 * w + b] >= i ? 1u : 0u) << b;
+                pre |= (rank_v[32 * w + b] < i ? 1u : 0u) << b;
+            }
+            T.suf[i][w] = suf;
+            T.pre[i][w] = pre;
         }
     }
-    if (k < SOLWEIG_MASK_WORDS) {
+    if (k < 8) {
         uint32_t t = 0;
-        for (int b = 0; b < 32; ++b) {
+        for (int b = 0; b < 32 && k < SOLWEIG_MASK_WORDS; ++b) {
             const int kk = k * 32 + b;
             if (kk < P && h.daytime && h.lw_sun_test[kk]) t |= 1u << b;
         }
-        T.test[k] = t;
+        T.loop.test[k] = t;
     }
-    __syncthreads();  // sorted arrays complete
     for (int i = k; i < 256; i += blockDim.x) {
         const double bound = tan_bucket_bound(i);
-        int ns = 0, nv = 0;
-        for (int j = 0; j < P; ++j) {
-            ns += T.tsun[j] < bound ? 1 : 0;
-            nv += T.vshade[j] < bound ? 1 : 0;
+        int lo = 0, len = P;  // entries below the bound
+        while (len > 0) {
+            const int half = len >> 1;
+            if (sorted[lo + half] < bound) {
+                lo += half + 1;
+                len -= half + 1;
+            } else {
+                len = half;
+            }
         }
-        T.sun_start[i] = (uint8_t)ns;
-        T.shd_start[i] = (uint8_t)nv;
+        T.sun_start[i] = (uint8_t)lo;
     }
     if (k < SOLWEIG_MAX_BANDS) {
         const bool ok = k < L->nbands;
-        T.band_down[k] = ok ? h.band_lsky[k] * L->band_omega[k] * L->band_sin[k] : 0.f;
-        T.band_side[k] = ok ? h.band_lsky[k] * L->band_omega[k] * L->band_cos[k] : 0.f;
+        T.loop.band_down[k] = ok ? h.band_lsky[k] * L->band_omega[k] * L->band_sin[k] : 0.f;
+        T.loop.band_side[k] = ok ? h.band_lsky[k] * L->band_omega[k] * L->band_cos[k] : 0.f;
     }
     if (k == 32) {
         const double tk = h.ta + 273.15;
-        T.lw_shade = (float)((0.9 * kSBC * pow4(tk)) / kPi);
-        T.lw_sun = h.daytime ? (float)((0.9 * kSBC * pow4(h.ta + h.tgwall + 273.15)) / kPi) : 0.f;
-        T.sw_shade = (float)((0.2 * h.rad_d * 0.5) / kPi);
-        T.sw_sun = (float)((0.2 * (h.rad_i * h.cos_alt) + h.rad_d * 0.5) / kPi);
-        T.rad_d = (float)h.rad_d;
-        T.rad_g = (float)h.rad_g;
-        T.direct_up = (float)(h.rad_i * h.sin_alt);
-        T.rad_i_sin = (float)(h.rad_i * h.sin_alt);
-        T.rad_i_cos = (float)(h.rad_i * h.cos_alt);
-        T.rad_ratio = (float)(h.rad_d / h.rad_tot);
-        T.wave_w = (float)h.wave_weight;
-        T.tan_zen = (float)h.tan_zen;
-        T.night_lup = (float)(kSBC * pow4(tk));
-        T.night_lup_water = (float)(kSBC * 0.98 * pow4(h.twater + 273.15));
+        HourLoop& q = T.loop;
+        q.lw_shade = (float)((0.9 * kSBC * pow4(tk)) / kPi);
+        q.lw_sun = h.daytime ? (float)((0.9 * kSBC * pow4(h.ta + h.tgwall + 273.15)) / kPi) : 0.f;
+        q.sw_shade = (float)((0.2 * h.rad_d * 0.5) / kPi);
+        q.sw_sun = (float)((0.2 * (h.rad_i * h.cos_alt) + h.rad_d * 0.5) / kPi);
+        q.rad_d = (float)h.rad_d;
+        q.rad_g = (float)h.rad_g;
+        q.rad_i_sin = (float)(h.rad_i * h.sin_alt);
+        q.rad_i_cos = (float)(h.rad_i * h.cos_alt);
+        q.rad_ratio = (float)(h.rad_d / h.rad_tot);
+        q.wave_w = (float)h.wave_weight;
+        q.tan_zen = (float)h.tan_zen;
+        q.night_lup = (float)(kSBC * pow4(tk));
+        q.night_lup_water = (float)(kSBC * 0.98 * pow4(h.twater + 273.15));
+        q.ta = (float)h.ta;
+        q.flags = (h.daytime ? kHourDay : 0u) | (h.firstdaytime ? kHourFirst : 0u) |
+                  (h.wave_update ? kHourUpdate : 0u) | (h.utci_valid ? kHourUtci : 0u);
+        q.pad = 0u;
+        for (int i = 0; i < 7; ++i) q.utci[i] = h.utci[i];
+        q.utci[7] = h.ta;
     }
 }
 
@@ -805,6 +823,7 @@ struct DayRadArgs {
     SolweigState state;
     SolweigOutputs out;  // base pointers; hour h at + h * hour_stride
     long long hour_stride;
+    int chunk;           // hours per block (grid.y); all of them when a state or ground temperature is kept
 };
 
 
@@ -835,16 +854,20 @@ __device__ __forceinline__ float wedge_fsh_f(float ta, float tan_zen) {
     return isnan(fsh) ? 0.5f : fsh;
 }
 
-// Flux arithmetic of the hour loop in float32 (the hour's scalars are
-// staged once per block, rounded from the float64 host plan); the building
-// split keeps its exact float64 thresholds.  Against the per-hour form
-// (float64 fluxes) Tmrt differs by < 1e-3 K (tested).  Launched for full
-// occupancy, 2048 resident threads per SM (32 registers): the loop is
-// latency-bound, and the extra warps outweigh the spilled registers (per
-// 2000^2 day: 5.65 ms at 512 threads, 4.32 at 768, 3.70 at 1024, 3.46 at
-// 1280, 3.26 at 1536, 3.15 at 2048).  The hour tables and scalars are read
-// from the day's table array through L1 instead of being staged in shared
-// memory, so the hour loop has no barrier (3.15 -> 2.92 ms).
+// Flux arithmetic of the hour loop in float32 (the hour's scalars are rounded
+// once from the float64 host plan); the building split keeps its exact float64
+// thresholds.  Against the per-hour form (float64 fluxes) Tmrt differs by <
+// 1e-3 K (tested).
+//
+// What bounds it: instruction issue (77 % of the cycles) and the load/store
+// unit (73 %: the hour's scalars, read through L1 without a barrier, and
+// spills).  A building patch that is not sunlit is shaded, so one pass of
+// popcounts over the sunlit patches serves both sums and both tests (POPC runs
+// at an eighth of the issue rate), and patches exactly on a limit take a branch.
+// 2000^2 day: 2.86 -> 2.00 ms.  Full occupancy (2048 resident threads per SM,
+// 32 registers, spills) against 40 / 48 registers at 1536 / 1280 threads: 2.00
+// against 2.08 / 2.17 ms; the scalars and mask rows as 16-byte loads, which
+// live longer: 2.14 to 2.35 ms.
 template <int OPT, int THREADS>
 __global__ void __launch_bounds__(THREADS, 2048 / THREADS) day_radiation_kernel(SolweigScene S, DayRadArgs a) {
     __shared__ float wcos[SOLWEIG_MAX_BANDS], wsin[SOLWEIG_MAX_BANDS];
@@ -885,45 +908,70 @@ __global__ void __launch_bounds__(THREADS, 2048 / THREADS) day_radiation_kernel(
     const float tan_alfa = (float)tan(S.svfalfa[q]);
     const double tan_asvf = S.tan_asvf[q];
     const int tbucket = tan_bucket(tan_asvf);
-    const float vc = S.veg_sums[q], vs = S.veg_sums[n + q];
     const float oc = S.veg_sums[2 * n + q], os = S.veg_sums[3 * n + q];
     const float g_nosh = a.nosh[q];
     constexpr float ewall = 0.9f, albedo_b = 0.2f;
     constexpr float absK = 0.7f, absL = 0.95f, Fside = 0.22f, Fup = 0.06f, Fcyl = 0.28f;
-    constexpr float dsh_veg = 0.03f;
     constexpr float sbc = (float)kSBC, inv_pi = (float)(1.0 / kPi);
 
+    // sums over the vegetation and building patches: those not sunlit emit as shaded walls
+    float shd_c, shd_s;
+    {
+        float all_c;
+        band_sums<OPT>(bld, bld, wcos, wsin, all_c, shd_c, shd_s);
+        shd_c += S.veg_sums[q];
+        shd_s += S.veg_sums[n + q];
+    }
     float st_lup = a.state.tgmap1 ? a.state.tgmap1[q] : 0.f;
     float st_tg = a.state.tgout1 ? a.state.tgout1[q] : 0.f;
 
-    for (int hr = 0; hr < a.nhours; ++hr) {
+    // hours of this block (blockIdx.y); the wave-delay state of the hours before them
+    const int h0 = blockIdx.y * a.chunk, h1 = min(h0 + a.chunk, a.nhours);
+    for (int hr = 0; hr < h0; ++hr) {
+        const HourLoop& hs = a.tables[hr].loop;
+        if (!(hs.flags & kHourDay)) continue;
+        const float g_lup = a.gvf[(3LL * hr) * n + q];
+        const float prev = (hs.flags & kHourFirst) ? g_lup : st_lup;
+        st_lup = (hs.flags & kHourUpdate) ? g_lup * (1.f - hs.wave_w) + prev * hs.wave_w : prev;
+    }
+    for (int hr = h0; hr < h1; ++hr) {
         // the hour's table and scalars, read through L1 by every thread (no
         // shared staging, so the hour loop needs no barrier)
-        const DayTable& hs = a.tables[hr];
-        const SolweigHour& h = a.hours[hr];
-        const bool day = h.daytime != 0;
-        const float ta = (float)h.ta;
+        const DayTable& T = a.tables[hr];
+        const HourLoop& hs = T.loop;  // scalars are read where they are used: registers are short
+        const uint32_t flags = hs.flags;
+        const bool day = flags & kHourDay;
 
-        // building patches: sunlit / shaded split of the hour
-        const DayTable& T = hs;
-        const int P = S.patches;
-        const int isun = count_le_from(T.tsun, P, T.sun_start[tbucket], tan_asvf);
-        const int ishd = count_le_from(T.vshade, P, T.shd_start[tbucket], tan_asvf);
-        uint32_t m_sun[SOLWEIG_MASK_WORDS], m_shd[SOLWEIG_MASK_WORDS], m_lsun[SOLWEIG_MASK_WORDS],
-            m_lshd[SOLWEIG_MASK_WORDS];
+        // Building patches, sunlit (ref) and sunlit within the longwave's sun
+        // test (hs.lw_sun): the other ones are shaded.
+        float ref_c = 0.f, none_c = 0.f, lw_sun_c = 0.f, lw_sun_s = 0.f, lw_shd_c = shd_c, lw_shd_s = shd_s;
+        if (day) {
+            const int isun = count_le_from(T.tsun, S.patches, T.sun_start[tbucket], tan_asvf);
+            // every shaded threshold is at or above its patch's sunlit one, so
+            // at most isun of them are <= t, nearly always all of them
+            int ishd = isun;
+            while (ishd > 0 && T.vshade[ishd - 1] > tan_asvf) --ishd;
+            uint32_t m[SOLWEIG_MASK_WORDS], mt[SOLWEIG_MASK_WORDS];
 #pragma unroll
-        for (int w = 0; w < SOLWEIG_MASK_WORDS; ++w) {
-            const uint32_t test = T.test[w];
-            m_sun[w] = bld[w] & T.suf[isun][w];
-            m_shd[w] = bld[w] & T.pre[ishd][w];
-            m_lsun[w] = m_sun[w] & test;
-            m_lshd[w] = bld[w] & (~test | m_shd[w]);
+            for (int w = 0; w < SOLWEIG_MASK_WORDS; ++w) {
+                m[w] = bld[w] & T.suf[isun][w];
+                mt[w] = m[w] & hs.test[w];
+            }
+            band_sums<OPT>(m, mt, wcos, wsin, ref_c, lw_sun_c, lw_sun_s);
+            lw_shd_c -= lw_sun_c;
+            lw_shd_s -= lw_sun_s;
+            if (ishd < isun) {  // patches exactly on the limit are neither
+                float t_c, t_s;
+#pragma unroll
+                for (int w = 0; w < SOLWEIG_MASK_WORDS; ++w) {
+                    m[w] = bld[w] & ~m[w] & ~T.pre[ishd][w];
+                    mt[w] = m[w] & hs.test[w];
+                }
+                band_sums<OPT>(m, mt, wcos, wsin, none_c, t_c, t_s);
+                lw_shd_c -= t_c;
+                lw_shd_s -= t_s;
+            }
         }
-        float cnt_lsun[8], cnt_lshd[8];
-        band_counts<OPT>(m_lsun, cnt_lsun);
-        band_counts<OPT>(m_lshd, cnt_lshd);
-        const float lw_sun_c = band_dot(cnt_lsun, wcos), lw_sun_s = band_dot(cnt_lsun, wsin);
-        const float lw_shd_c = band_dot(cnt_lshd, wcos), lw_shd_s = band_dot(cnt_lshd, wsin);
         float ld_sky = 0.f, ls_sky = 0.f;
 #pragma unroll
         for (int b = 0; b < 8; ++b) {
@@ -931,9 +979,8 @@ __global__ void __launch_bounds__(THREADS, 2048 / THREADS) day_radiation_kernel(
             ld_sky = fmaf(hs.band_down[b], cnt, ld_sky);
             ls_sky = fmaf(hs.band_side[b], cnt, ls_sky);
         }
-        const float lw_shade = hs.lw_shade, lw_sun = hs.lw_sun;
 
-        float shadow = 0.f, tg = 0.f, tg_out = ta;
+        float shadow = 0.f, tg = 0.f, tg_out = hs.ta;
         float kup_all = 0.f, lup_all;
         float kdown = 0.f, kside = 0.f, kside_i = 0.f, kside_d = 0.f, d_rad = 0.f;
         if (day) {
@@ -944,12 +991,13 @@ __global__ void __launch_bounds__(THREADS, 2048 / THREADS) day_radiation_kernel(
             const float fsh = wedge_fsh_f(tan_alfa, hs.tan_zen);
             const float reflected = albedo_b * (1.f - svfbuveg) * (hs.rad_g * (1.f - fsh) + hs.rad_d * fsh);
             const float base_up = hs.rad_d * svfbuveg + reflected;
-            kup_all = g_alb * hs.direct_up + base_up * g_nosh;
-            const float prev = h.firstdaytime ? g_lup : st_lup;
+            kup_all = g_alb * hs.rad_i_sin + base_up * g_nosh;
+            const float prev = (flags & kHourFirst) ? g_lup : st_lup;
             lup_all = g_lup * (1.f - hs.wave_w) + prev * hs.wave_w;
-            st_lup = h.wave_update ? lup_all : prev;
+            st_lup = (flags & kHourUpdate) ? lup_all : prev;
             if (need_tg) {
                 // ground temperature (TsWaveDelay of Tg * shadow + Ta); not part of Tmrt
+                const SolweigHour& h = a.hours[hr];
                 const double amp = (double)S.tgk[q] * h.altmax + (double)S.tstart[q];
                 const double phase = ((h.dectime_frac - h.snup / 24.0) /
                                       ((double)S.tmaxlst[q] / 24.0 - h.snup / 24.0)) * kPi / 2.0;
@@ -957,51 +1005,54 @@ __global__ void __launch_bounds__(THREADS, 2048 / THREADS) day_radiation_kernel(
                 if (S.landcover == 1 && tgd < 0.0) tgd = 0.0;
                 if (water) tgd = h.twater - h.ta;
                 tg = (float)tgd;
-                const float cur = tg * shadow + ta;
-                const float prv = h.firstdaytime ? cur : st_tg;
+                const float cur = tg * shadow + hs.ta;
+                const float prv = (flags & kHourFirst) ? cur : st_tg;
                 tg_out = cur * (1.f - hs.wave_w) + prv * hs.wave_w;
-                st_tg = h.wave_update ? tg_out : prv;
+                st_tg = (flags & kHourUpdate) ? tg_out : prv;
             }
             // the contraction already added the vegetation patches at their
-            // diffuse transmissivity (dsh_veg): sky + dsh_veg x vegetation sums
-            const long long s0 = 2LL * hr;
-            const float lum = a.sums[s0 * n + q], cw = a.sums[(s0 + 1) * n + q];
+            // diffuse transmissivity: sky + 0.03 x vegetation sums
+            const long long s0 = 2LL * hr * n + q;
+            const float lum = a.sums[s0], cw = a.sums[s0 + n];
             d_rad = hs.rad_d * lum;
             kdown = hs.rad_i_sin * shadow + d_rad + reflected;
             kside_i = shadow * hs.rad_i_cos;
             kside_d = hs.rad_ratio * cw;
-            kside = kside_i + kside_d + hs.sw_sun * band_weighted<OPT>(m_sun, wcos) +
-                    hs.sw_shade * band_weighted<OPT>(m_shd, wcos) + hs.sw_shade * vc;
+            kside = kside_i + kside_d + hs.sw_sun * ref_c + hs.sw_shade * (shd_c - ref_c - none_c);
         } else {
             float lup = emis * hs.night_lup;
             if (S.landcover == 1 && (fl & 4)) lup = hs.night_lup_water;
             lup_all = lup;
         }
         const float refl = (ld_sky + lup_all) * ((1.f - ewall) * 0.5f * inv_pi);
-        const float ldown = ld_sky + lw_shade * vs + lw_shade * lw_shd_s + lw_sun * lw_sun_s + refl * os;
-        const float lside = ls_sky + lw_shade * vc + lw_shade * lw_shd_c + lw_sun * lw_sun_c + refl * oc;
+        const float ldown = ld_sky + hs.lw_shade * lw_shd_s + hs.lw_sun * lw_sun_s + refl * os;
+        const float lside = ls_sky + hs.lw_shade * lw_shd_c + hs.lw_sun * lw_sun_c + refl * oc;
         // E+S+W+N of Kup and Lup are 4x the all-direction values (see the file header).
         const float sstr = absK * (kside * Fcyl + (kdown + kup_all) * Fup + 2.f * kup_all * Fside) +
                            absL * ((ldown + lup_all) * Fup + lside * Fcyl + 2.f * lup_all * Fside);
         const float tmrt = sqrtf(sqrtf(sstr * (1.f / (absL * sbc)))) - 273.2f;
         if (in) {
-            const long long hs_ = a.hour_stride;
-            if (o.tmrt) o.tmrt[hr * hs_ + p] = tmrt;
-            if (o.utci)
-                o.utci[hr * hs_ + p] = ground ? utci_eval(h.utci, (double)tmrt, h.ta, h.utci_valid)
-                                              : __int_as_float(0x7fc00000);
-            if (o.kdown) o.kdown[hr * hs_ + p] = kdown;
-            if (o.kup) o.kup[hr * hs_ + p] = kup_all;
-            if (o.ldown) o.ldown[hr * hs_ + p] = ldown;
-            if (o.lup) o.lup[hr * hs_ + p] = lup_all;
-            if (o.lside) o.lside[hr * hs_ + p] = lside;
-            if (o.kside_i) o.kside_i[hr * hs_ + p] = kside_i;
-            if (o.kside_d) o.kside_d[hr * hs_ + p] = kside_d;
-            if (o.kside) o.kside[hr * hs_ + p] = kside;
-            if (o.d_rad) o.d_rad[hr * hs_ + p] = d_rad;
-            if (o.shadow) o.shadow[hr * hs_ + p] = shadow;
-            if (o.tg) o.tg[hr * hs_ + p] = tg;
-            if (o.tg_out) o.tg_out[hr * hs_ + p] = tg_out;
+            const long long at = hr * a.hour_stride + p;
+            if (o.tmrt) o.tmrt[at] = tmrt;
+            if (o.utci) {
+                float u = __int_as_float(0x7fc00000);
+                if (ground) {
+                    u = utci_eval(hs.utci, (double)tmrt, hs.utci[7], flags & kHourUtci);
+                }
+                o.utci[at] = u;
+            }
+            if (o.kdown) o.kdown[at] = kdown;
+            if (o.kup) o.kup[at] = kup_all;
+            if (o.ldown) o.ldown[at] = ldown;
+            if (o.lup) o.lup[at] = lup_all;
+            if (o.lside) o.lside[at] = lside;
+            if (o.kside_i) o.kside_i[at] = kside_i;
+            if (o.kside_d) o.kside_d[at] = kside_d;
+            if (o.kside) o.kside[at] = kside;
+            if (o.d_rad) o.d_rad[at] = d_rad;
+            if (o.shadow) o.shadow[at] = shadow;
+            if (o.tg) o.tg[at] = tg;
+            if (o.tg_out) o.tg_out[at] = tg_out;
         }
     }
     if (in) {
