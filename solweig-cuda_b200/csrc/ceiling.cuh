@@ -263,11 +263,13 @@ __device__ __forceinline__ void ceiling_scan(const float* __restrict__ plane, co
 // The four dilated planes of H (see the file comment), each rows x cols floats:
 //   dil[0], dil[1]: +-1, +-2 along the columns, row-major [r][c];
 //   dil[2], dil[3]: +-1, +-2 along the rows, transposed [c][r].
+// H itself goes to `height` (optional), row-major.
 // block (32, 8) over a 32 x 32 tile, H staged with a 2-pixel halo.
 constexpr int kDilTile = 32, kDilHalo = 2, kDilPitch = kDilTile + 2 * kDilHalo + 1;
 
 template <bool G32>
-__global__ void __launch_bounds__(256) ceiling_dilate_kernel(SolweigScene S, float* __restrict__ dil) {
+__global__ void __launch_bounds__(256) ceiling_dilate_kernel(SolweigScene S, float* __restrict__ dil,
+                                                             float* __restrict__ height) {
     __shared__ float tile[kDilTile + 2 * kDilHalo][kDilPitch];
     const int r0 = blockIdx.y * kDilTile, c0 = blockIdx.x * kDilTile;
     const int tid = threadIdx.y * 32 + threadIdx.x;
@@ -288,6 +290,7 @@ __global__ void __launch_bounds__(256) ceiling_dilate_kernel(SolweigScene S, flo
         const float* t = &tile[k + kDilHalo][threadIdx.x + kDilHalo];
         const float d1 = fmaxf(t[0], fmaxf(t[-1], t[1]));
         const float d2 = fmaxf(d1, fmaxf(t[-2], t[2]));
+        if (height) height[(long long)r * S.cols + c] = t[0];
         dil[(long long)r * S.cols + c] = d1;
         dil[n + (long long)r * S.cols + c] = d2;
     }

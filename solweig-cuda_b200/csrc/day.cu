@@ -235,8 +235,7 @@ int day_batched_impl(const SolweigScene* scene, const SolweigSkyLayout* layout, 
     if (part == kDaySweep) {
         const int nh = h1 - h0;
         // The ceiling planes (8 B per pixel-hour: ceiling and window maximum)
-        // live in the GVF region (12 B
-        // per pixel-hour) and the four dilated height planes (16 B per pixel)
+        // live in the GVF region (12 B per pixel-hour) and the four dilated height planes (16 B per pixel)
         // in the patch-sum region (at least 16 B per pixel): both are consumed
         // by the sweep before the GVF kernels and the contraction write those
         // regions.
@@ -250,10 +249,12 @@ int day_batched_impl(const SolweigScene* scene, const SolweigSkyLayout* layout, 
                 SOLWEIG_CHECK_LAUNCH("sweep_tile_max_kernel");
             }
         }
-        if (ceiling && h0 == 0) {
+        // the plane of H lives in the albedo-without-shadow plane, free until the GVF
+        float* height = S.geo32 ? nosh : nullptr;
+        if ((ceiling || height) && h0 == 0) {
             dim3 dgrid(blocks_for(S.cols, kDilTile), blocks_for(S.rows, kDilTile));
-            if (S.geo32) ceiling_dilate_kernel<true><<<dgrid, dim3(32, 8), 0, st>>>(S, dil);
-            else ceiling_dilate_kernel<false><<<dgrid, dim3(32, 8), 0, st>>>(S, dil);
+            if (S.geo32) ceiling_dilate_kernel<true><<<dgrid, dim3(32, 8), 0, st>>>(S, dil, height);
+            else ceiling_dilate_kernel<false><<<dgrid, dim3(32, 8), 0, st>>>(S, dil, height);
             SOLWEIG_CHECK_LAUNCH("ceiling_dilate_kernel");
         }
         if (ceiling) {
@@ -262,18 +263,9 @@ int day_batched_impl(const SolweigScene* scene, const SolweigSkyLayout* layout, 
                                                                                   ceiling + h0 * px);
             SOLWEIG_CHECK_LAUNCH("day_ray_ceiling_kernel");
         }
-        // first-outside steps of every row and column per hour (4 B each), in
-        // the GVF region after the ceiling planes (4 B per pixel-hour left; a
-        // raster one pixel wide spills a few bytes into the next region, free
-        // until the GVF stage)
-        int* exits = reinterpret_cast<int*>(wb + w.gvf + 8LL * px * nhours) + (long long)h0 * (S.rows + S.cols);
-        // then the hours' step records (16 B per step, at most max(rows, cols) + 2
-        // steps per hour), when they fit before the end of the GVF region
-        const long long rec_at = (w.gvf + 8LL * px * nhours + 4LL * (S.rows + S.cols) * nhours + 15) & ~15LL;
-        const int kmax = (S.rows > S.cols ? S.rows : S.cols) + 2;
-        longlong2* rec = nullptr;
-        if (rec_at + 16LL * kmax * nhours <= w.gvf + 12LL * px * nhours)
-            rec = reinterpret_cast<longlong2*>(wb + rec_at) + (long long)h0 * kmax;
+        const int kmax = (S.rows > S.cols ? S.rows : S.cols) + 2, kpitch = record_pitch(kmax);
+        int* exits = reinterpret_cast<int*>(wb + w.exits) + (long long)h0 * (S.rows + S.cols);
+        int2* rec = reinterpret_cast<int2*>(wb + w.rec) + (long long)h0 * kpitch;
         day_ray_exits_kernel<<<nh, 1024, 0, st>>>(S, hours + h0, exits, rec, kmax, err);
         SOLWEIG_CHECK_LAUNCH("day_ray_exits_kernel");
         if (window) {
@@ -296,14 +288,14 @@ int day_batched_impl(const SolweigScene* scene, const SolweigSkyLayout* layout, 
             return SOLWEIG_OK;
         }
         dim3 grid(blocks_for(S.cols, cfg.shadow_bx), blocks_for(S.rows, cfg.shadow_by), nh);
-        if (rec && S.geo32)
+        if (S.geo32 && px <= kPackedMaxPixels)
             day_shadow_kernel<true><<<grid, dim3(cfg.shadow_bx, cfg.shadow_by), 0, st>>>(
                 S, hours + h0, quads + h0 * px, lup_first ? lup_first + h0 * px : nullptr,
-                ceiling ? ceiling + h0 * px : nullptr, exits, rec, kmax);
+                ceiling ? ceiling + h0 * px : nullptr, exits, rec, kpitch, height);
         else
             day_shadow_kernel<false><<<grid, dim3(cfg.shadow_bx, cfg.shadow_by), 0, st>>>(
                 S, hours + h0, quads + h0 * px, lup_first ? lup_first + h0 * px : nullptr,
-                ceiling ? ceiling + h0 * px : nullptr, exits, nullptr, 0);
+                ceiling ? ceiling + h0 * px : nullptr, exits, rec, kpitch, height);
         SOLWEIG_CHECK_LAUNCH("day_shadow_kernel");
         return SOLWEIG_OK;
     }

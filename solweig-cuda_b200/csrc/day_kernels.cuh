@@ -4,6 +4,8 @@
 #pragma once
 #include <cuda_bf16.h>
 
+#include <algorithm>
+
 #include "ceiling.cuh"
 #include "gvf_walk.cuh"
 #include "hour.cuh"
@@ -206,18 +208,16 @@ __device__ __forceinline__ void warp_tile_pixel(int bx, int by, int& r, int& c) 
     }
 }
 
-// REC: the walks read the hour's step records (rec + z * kmax, written by
-// day_ray_exits_kernel) instead of the (dx, dy) and dz tables.  40 registers
-// (6 blocks of 256 per SM): the walk's float64 state no longer spills (per
-// 2000^2 day 5.77 ms against 5.97 ms at 32 registers and 8 blocks).
-template <bool REC>
-__global__ void __launch_bounds__(256, 6) day_shadow_kernel(SolweigScene S,
-                                                                   const SolweigHour* __restrict__ hours,
-                                                                   float4* __restrict__ quads,
-                                                                   float* __restrict__ lup_first,
-                                                                   const float2* __restrict__ ceiling,
-                                                                   const int* __restrict__ exits,
-                                                                   const longlong2* __restrict__ rec, int kmax) {
+// TABLES: the packed geometry with the hours' tables (exits, step records of
+// kpitch entries per hour, plane of H), else the rasters step by step.
+template <bool TABLES>
+__global__ void __launch_bounds__(256, 8) day_shadow_kernel(SolweigScene S, const SolweigHour* __restrict__ hours,
+                                                            float4* __restrict__ quads,
+                                                            float* __restrict__ lup_first,
+                                                            const float2* __restrict__ ceiling,
+                                                            const int* __restrict__ exits,
+                                                            const int2* __restrict__ rec, int kpitch,
+                                                            const float* __restrict__ height) {
     const int z = blockIdx.z;
     const SolweigHour& h = hours[z];
     if (!h.daytime) return;
@@ -226,29 +226,31 @@ __global__ void __launch_bounds__(256, 6) day_shadow_kernel(SolweigScene S,
     const bool in = r < S.rows && c < S.cols;
     const long long n = (long long)S.rows * S.cols;
     if (!in) return;
-    shadow_quad_pixel<REC>(S, h, r, c, quads + z * n, lup_first ? lup_first + z * n : nullptr,
-                           ceiling ? ceiling + z * n : nullptr,
-                           exits ? exits + (long long)z * (S.rows + S.cols) : nullptr,
-                           REC ? rec + (long long)z * kmax : nullptr);
+    const float2* ceil_z = ceiling ? ceiling + z * n : nullptr;
+    float* first_z = lup_first ? lup_first + z * n : nullptr;
+    if constexpr (TABLES) {
+        const SweepTables t{exits + (long long)z * (S.rows + S.cols), rec + (long long)z * kpitch, height, ceil_z};
+        shadow_quad_pixel(S, h, r, c, quads + z * n, first_z, nullptr, &t);
+    } else {
+        shadow_quad_pixel(S, h, r, c, quads + z * n, first_z, ceil_z, nullptr);
+    }
 }
 
 // Per daytime hour, the first-outside step of every row and column of the
-// raster (first_outside), for the bounds-check-free sweep, and with rec the
-// hour's step records for the steps [0, min(steps, kmax)).  A monotone ray
-// leaves the raster within max(rows, cols) steps, so kmax = max(rows, cols)
-// + 2 covers every walk; a ray table that stays inside longer has its exits
-// cut to kmax and sets the error flag to 3 (that hour's results invalid).
+// raster (first_outside), for the bounds-check-free sweep, and the hour's step
+// records for the steps [0, min(steps, kmax)).  A monotone ray leaves the
+// raster within max(rows, cols) steps, so kmax = max(rows, cols) + 2 covers
+// every walk; a ray table that stays inside longer has its exits cut to kmax
+// and sets the error flag to 3 (that hour's results invalid).
 __global__ void __launch_bounds__(1024) day_ray_exits_kernel(SolweigScene S, const SolweigHour* __restrict__ hours,
-                                                             int* __restrict__ exits, longlong2* __restrict__ rec,
+                                                             int* __restrict__ exits, int2* __restrict__ rec,
                                                              int kmax, int* __restrict__ error) {
     const SolweigHour& h = hours[blockIdx.x];
     if (!h.daytime) return;
     int* ex = exits + (long long)blockIdx.x * (S.rows + S.cols);
     ray_exits_block(reinterpret_cast<const int2*>(h.ray_dxdy), h.steps, S.rows, S.cols, ex);
-    if (rec == nullptr) return;
-    const int K = min(h.steps, kmax);
-    ray_records_block(reinterpret_cast<const int2*>(h.ray_dxdy), h.ray_dz, K, S.cols,
-                      rec + (long long)blockIdx.x * kmax);
+    ray_records_block(reinterpret_cast<const int2*>(h.ray_dxdy), h.ray_dz, min(h.steps, kmax), S.cols,
+                      rec + (long long)blockIdx.x * record_pitch(kmax));
     if (h.steps <= kmax) return;
     __syncthreads();  // ex[] written by the whole block
     int cut = 0;
@@ -1066,7 +1068,7 @@ __global__ void __launch_bounds__(THREADS, 2048 / THREADS) day_radiation_kernel(
 inline long long align256(long long x) { return (x + 255) & ~255LL; }
 
 struct DayWork {
-    long long quads, lup_first, gvf, nosh, sums, wf32, bw, tables, error, tilemax, walks, dict, total;
+    long long quads, lup_first, gvf, nosh, sums, wf32, bw, tables, error, tilemax, walks, dict, exits, rec, total;
 };
 
 DayWork day_work_layout(int rows, int cols, int nhours, bool water) {
@@ -1093,6 +1095,9 @@ DayWork day_work_layout(int rows, int cols, int nhours, bool water) {
     w.walks = o; o = align256(o + (water ? 0 : 4LL * walk_words(rows, cols)));
     w.dict = o;
     o = align256(o + (water ? 0 : walk_words(rows, cols) / kWkTileWords * 8 * kWkDictKeys * ((nhours + 3) / kWkHours)));
+    // per hour the first-outside steps of the rows and columns, and the ray's step records
+    w.exits = o; o = align256(o + 4LL * (rows + cols) * nhours);
+    w.rec = o; o = align256(o + 8LL * record_pitch(std::max(rows, cols) + 2) * nhours);
     w.total = o;
     return w;
 }

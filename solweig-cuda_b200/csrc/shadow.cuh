@@ -25,13 +25,7 @@
 //   * with a ray-ceiling plane (ceiling.cuh), every 4th step from step 4 on:
 //     ceiling(q_k) - dz_{k-1} (rounded up) < dsm_p bounds every later
 //     sample's h - dz_{j-1} below the pixel (dsm_p >= 0; for wall pixels
-//     also <= topmax >= 0), so nothing further can change;
-//   * (packed walk) at the same steps, window maximum(q_k) - dz_{k-1}
-//     (rounded up) <= dsm_p bounds the next kCeilSkip samples' h - dz_{j-1}
-//     by the pixel: none of their compares is above it and f cannot grow, so
-//     the walk skips them when, for a wall pixel, the bound is also <= topmax
-//     (the canopy top seen stays final); only the carried flags move: ever
-//     picks up veg when unshadowed, as each step would.
+//     also <= topmax >= 0), so nothing further can change.
 // Once a sample leaves the raster it never re-enters (the offsets grow
 // monotonically), so the first outside step is applied and the loop ends.
 #pragma once
@@ -153,116 +147,146 @@ __device__ __forceinline__ ShadowResult shadow_walk_geo(
 }
 
 // The same walk over the packed float4 geometry, for a ray known to stay in
-// the raster for `kend` steps (the first step outside, or `steps`): no
-// per-step bounds checks, linear sample offsets, and only the DSM height is
-// widened to float64 at a sample without canopy (tq, bq <= 0 compare the
-// same in float32).  Results are identical to shadow_walk_geo.
+// the raster for `kend` steps (the first step outside, or `steps`).
 //
-// The steps run in unrolled groups of four aligned at step 0, so the
-// ray-ceiling test (steps 4, 8, ...) is the first step of a group and costs
-// no per-step test.  With REC the hour's steps come as 16-byte records
-// {linear offset o.x * cols + o.y, dz bit pattern} (one uniform load per
-// step, ray_records_block); otherwise from the (dx, dy) and dz tables.
-template <bool REC, bool SKIP = true>
+// Most samples of a walk matter to nothing: with H = max(dsm, canopy, trunk) of
+// the sample, H - dz_{k-1} below `thr` (the pixel's height, or for a wall pixel
+// already in shadow the building top seen) means that no compare of the step
+// is above the pixel and f cannot grow.  A canopy top below the pixel enters no
+// output.  So a step is one 4-byte load of the plane of H and one float32
+// compare, with `lo` = dz_{k-1} rounded down (H - lo is rounded up, so a step is
+// never missed), four steps at a time from the hour's records {offset, lo};
+// only the steps that pass load the float4 sample and compare in
+// float64, exactly as shadow_walk_geo.  The same holds for the ray ceiling
+// (nothing ahead reaches thr: the walk ends) and the window maximum (skip
+// kCeilSkip steps), consulted at steps 4, 8, ....
+//
+// Step 0 is the pixel itself (dz_0 = 0).  Once the canopy flag is set at an
+// unshadowed step it is `ever`, and it only clears in shadow, so one flag is
+// carried.  What bounds it: instruction issue (76 % of the cycles) and the
+// latency of the loads, at 32 registers (8 blocks of 256 threads per SM; 40 and
+// 48 registers were slower).  Against float64 compares and a 16-byte sample per
+// step, at 71 instructions a step: sweep stage 5.37 -> 3.35 ms per 2000^2 day,
+// scene set-up 38.0 -> 27.7 ms at 2000^2 (visibility of the lowest 32 patches at
+// 1000^2 2.74 -> 1.68 ms), masks identical.
+template <typename T>
+__device__ __forceinline__ T load_at(const T* __restrict__ base, uint32_t byte) {
+    return __ldg(reinterpret_cast<const T*>(reinterpret_cast<const char*>(base) + byte));
+}
+
+// Addresses are 32-bit byte offsets from the planes (the callers keep rasters
+// above kPackedMaxPixels on the other walks).
+constexpr long long kPackedMaxPixels = 1ll << 28;
+
 __device__ __forceinline__ ShadowResult shadow_walk_packed(
-    const float4* __restrict__ geo, int cols, long long p, double a, double top_p, bool bush, double wall,
-    const int2* __restrict__ ray, const double* __restrict__ dz, const longlong2* __restrict__ rec, int steps,
-    int kend, double hmax, const float2* __restrict__ ceiling) {
+    const float4* __restrict__ geo, const float* __restrict__ height, const float2* __restrict__ ceiling, uint32_t p,
+    bool bush, double wall, const int2* __restrict__ rec, const double* __restrict__ dz, int steps, int kend,
+    float hmax) {
+    const uint32_t pb = 4u * p;  // byte of the pixel in the plane of H; x 2, x 4 in the others
+    const float4 own = load_at(geo, 4u * pb);
+    const double a = own.x;
+    const bool nonneg = own.x >= 0.f;  // samples outside the raster read 0: they matter to lower pixels
+    const bool is_wall = wall > 0.0;
     ShadowResult s;
     s.f = a;
-    s.topmax = top_p;
+    s.topmax = own.y;
     s.shadowed = false;
-    s.veg = bush;
-    s.ever = false;
-    const bool is_wall = wall > 0.0;
-    const bool nonneg = a >= 0.0;
-    const double clear = nonneg ? nextafter(hmax - a, __longlong_as_double(0x7ff0000000000000ll))
-                                : __longlong_as_double(0x7ff0000000000000ll);
-    const float4* __restrict__ gp = geo + p;
-    const float2* __restrict__ cp = ceiling != nullptr ? ceiling + p : nullptr;
-    double dz_prev = 0.0;
+    s.ever = steps > 0 && (bush || (own.y > own.x) != (own.z > own.x));
+    float thr = own.x;
     bool final = false;
-    int k = 0;
+    int k = 1;
     while (k < kend) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {  // u == k % 4
-            if (k >= kend) break;
-            long long off;
-            double dzk;
-            if (REC) {
-                const longlong2 r = __ldg(rec + k);
-                off = r.x;
-                dzk = __longlong_as_double(r.y);
-            } else {
-                const int2 o = __ldg(&ray[k]);
-                dzk = __ldg(&dz[k]);
-                off = (long long)o.x * cols + o.y;
-            }
-            if (dz_prev >= clear && (!is_wall || (s.topmax >= 0.0 && hmax - dzk <= s.topmax))) {
-                final = true;
-                break;
-            }
-            if (u == 0 && cp != nullptr && k >= 4) {
-                const float2 cm = __ldg(cp + off);
-                const double e = __dsub_ru((double)cm.x, dz_prev);
-                if (nonneg && e < a && (!is_wall || (s.topmax >= 0.0 && e <= s.topmax))) {
+        const int g = k & ~3, e = min(g + 4, kend);
+        const int4 ra = __ldg(reinterpret_cast<const int4*>(rec + g));
+        if (k == g && nonneg) {
+            const float lo = __int_as_float(ra.y);
+            if (ceiling != nullptr) {
+                const float2 cm = load_at(ceiling, 2u * (pb + (uint32_t)ra.x));
+                if (__fsub_ru(cm.x, lo) < thr) {
                     final = true;
                     break;
                 }
-                const double em = __dsub_ru((double)cm.y, dz_prev);
-                if (SKIP && nonneg && k + kCeilSkip <= kend && em <= a && (!is_wall || em <= s.topmax)) {
-                    // steps k .. k + kCeilSkip - 1 change nothing but the carried flags
-                    s.ever = s.ever || s.veg;
+                if (__fsub_ru(cm.y, lo) <= thr && k + kCeilSkip <= kend) {
                     k += kCeilSkip;
-                    dz_prev = REC ? __longlong_as_double(__ldg(rec + k - 1).y) : __ldg(&dz[k - 1]);
-                    break;  // the next group starts at k (still a multiple of 4)
+                    continue;
                 }
-            }
-            const float4 v = __ldg(gp + off);
-            s.f = fmax(s.f, (double)v.x - dzk);
-            s.shadowed = s.f > a;
-            if (v.y <= 0.f && v.z <= 0.f && nonneg && s.topmax >= 0.0) {
-                if (s.shadowed) s.veg = false;
-                else s.ever = s.ever || s.veg;
-            } else {
-                const double tq = v.y, bq = v.z;
-                s.topmax = fmax(s.topmax, tq - dzk);
-                if (s.shadowed) {
-                    s.veg = false;
-                } else {
-                    const int n = (int)(tq - dzk > a) + (int)(bq - dzk > a) + (int)(tq - dz_prev > a) +
-                                  (int)(bq - dz_prev > a);
-                    s.veg = s.veg || (n > 0 && n < 4);
-                    s.ever = s.ever || s.veg;
-                }
-            }
-            if (s.shadowed && (!is_wall || s.f - a >= wall)) {
+            } else if (__fsub_ru(hmax, lo) < thr) {
                 final = true;
                 break;
             }
-            dz_prev = dzk;
-            ++k;
+        }
+        uint32_t reach = 0u;
+        if (e - k == 4) {
+            const int4 rb = __ldg(reinterpret_cast<const int4*>(rec + g + 2));
+            const float h0 = __fsub_ru(load_at(height, pb + (uint32_t)ra.x), __int_as_float(ra.y));
+            const float h1 = __fsub_ru(load_at(height, pb + (uint32_t)ra.z), __int_as_float(ra.w));
+            const float h2 = __fsub_ru(load_at(height, pb + (uint32_t)rb.x), __int_as_float(rb.y));
+            const float h3 = __fsub_ru(load_at(height, pb + (uint32_t)rb.z), __int_as_float(rb.w));
+            if (fmaxf(fmaxf(h0, h1), fmaxf(h2, h3)) < thr) {
+                k = e;
+                continue;
+            }
+            reach = (h0 < thr ? 0u : 1u) | (h1 < thr ? 0u : 2u) | (h2 < thr ? 0u : 4u) | (h3 < thr ? 0u : 8u);
+        } else {
+#pragma unroll 1
+            for (int i = k; i < e; ++i) {
+                const int2 r = __ldg(rec + i);
+                if (!(__fsub_ru(load_at(height, pb + (uint32_t)r.x), __int_as_float(r.y)) < thr)) reach |= 1u << (i - g);
+            }
+        }
+        while (reach) {
+            const int i = g + __ffs((int)reach) - 1;
+            reach &= reach - 1u;
+            const int2 r = __ldg(rec + i);
+            const float lo = __int_as_float(r.y);
+            const float4 v = load_at(geo, 4u * (pb + (uint32_t)r.x));
+            if (!(__fsub_ru(v.x, lo) < thr)) {  // the building may reach the pixel
+                const double top = v.x - __ldg(&dz[i]);
+                if (top > s.f) {
+                    s.f = top;
+                    s.shadowed = true;
+                    if (!is_wall || top - a >= wall) {
+                        final = true;
+                        break;
+                    }
+                    thr = __double2float_rd(top);
+                }
+            }
+            // canopy above the pixel, while it is lit and the flag or a wall needs it
+            if (!s.shadowed && (is_wall || !s.ever) && !(__fsub_ru(fmaxf(v.y, v.z), lo) < own.x)) {
+                const double z = __ldg(&dz[i]), zp = __ldg(&dz[i - 1]), t = v.y, b = v.z;
+                s.topmax = fmax(s.topmax, t - z);
+                const int n = (int)(t - z > a) + (int)(b - z > a) + (int)(t - zp > a) + (int)(b - zp > a);
+                s.ever = s.ever || (n > 0 && n < 4);
+            }
         }
         if (final) break;
+        k = e;
     }
-    if (!final && k < steps) {
+    if (!final && kend < steps) {
         // First step whose sample is outside the raster: all shifted values are 0.
         s.f = fmax(s.f, 0.0);
         s.shadowed = s.f > a;
         s.topmax = fmax(s.topmax, 0.0);
-        if (s.shadowed) s.veg = false;
-        s.ever = s.ever || s.veg;
     }
+    s.veg = steps > 0 ? s.ever && !s.shadowed : bush;
     return s;
 }
 
-// Step records of one hour's ray for shadow_walk_packed<true>: rec[k] =
-// {o_k.x * cols + o_k.y, dz_k as a 64-bit pattern} for k < K, by one block.
+// Entries of a ray's record row: kmax steps padded to groups of four.
+__host__ __device__ __forceinline__ int record_pitch(int kmax) { return (kmax + 3) & ~3; }
+
+// Step records of one ray for shadow_walk_packed: rec[k] = {byte offset of the
+// sample in a float plane, dz_{k-1} rounded down} for k < K, by one block.
 __device__ __forceinline__ void ray_records_block(const int2* __restrict__ ray, const double* __restrict__ dz,
-                                                  int K, int cols, longlong2* __restrict__ rec) {
-    for (int k = threadIdx.x; k < K; k += blockDim.x) {
-        const int2 o = __ldg(&ray[k]);
-        rec[k] = make_longlong2((long long)o.x * cols + o.y, __double_as_longlong(__ldg(&dz[k])));
+                                                  int K, int cols, int2* __restrict__ rec) {
+    for (int k = threadIdx.x; k < record_pitch(K); k += blockDim.x) {
+        int2 v = make_int2(0, __float_as_int(0.f));
+        if (k < K) {
+            const int2 o = __ldg(&ray[k]);
+            v = make_int2(4 * (o.x * cols + o.y), __float_as_int(k > 0 ? __double2float_rd(__ldg(&dz[k - 1])) : 0.f));
+        }
+        rec[k] = v;
     }
 }
 

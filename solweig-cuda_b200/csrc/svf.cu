@@ -25,13 +25,9 @@ struct SvfRayParams {
 
 // grid.x: chunks of 32 consecutive pixels; grid.y: patch word (32 patches)
 // from word0 on.  geo32: the packed float4 geometry (exact float32 values) or
-// null.  With `ceiling` and `exits` (one launch per word, grid.y = 1): the
-// word's ray-ceiling planes [32][pixels] and first-outside steps [32][rows +
-// cols]; the walk then stops on the ceilings and, with geo32, needs no
-// bounds checks.
-// WALK: 0 float64 rasters, 1 packed geometry, 2 packed geometry without
-// bounds checks (`exits` given; used when the step records do not fit, else
-// svf_visibility_warp_kernel).
+// null.  With `ceiling` (one launch per word, grid.y = 1): the word's
+// ray-ceiling planes [32][pixels], on which the walk stops.
+// WALK: 0 float64 rasters, 1 packed geometry.
 // 32 registers (8 blocks per SM): the walks are latency-bound and full
 // occupancy outweighs the few spills (SVF 5.7 ms faster at 2000^2 than at
 // 40 registers).
@@ -40,7 +36,7 @@ __global__ void __launch_bounds__(32 * kSvfWarps, 8) svf_visibility_kernel(
     const double* __restrict__ dsm, const double* __restrict__ top, const double* __restrict__ bot,
     const float4* __restrict__ geo32, const uint8_t* __restrict__ flags, SvfRayParams prm,
     const int2* __restrict__ ray, const double* __restrict__ dz, const int32_t* __restrict__ lengths,
-    uint32_t* __restrict__ masks, int word0, const float2* __restrict__ ceiling, const int* __restrict__ exits) {
+    uint32_t* __restrict__ masks, int word0, const float2* __restrict__ ceiling) {
     __shared__ uint8_t state[kSvfPatchGroup][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long long pixels = (long long)prm.rows * prm.cols;
@@ -63,12 +59,7 @@ __global__ void __launch_bounds__(32 * kSvfWarps, 8) svf_visibility_kernel(
             const int K = lengths[patch];
             const float2* ceil_j = ceiling ? ceiling + (long long)j * pixels : nullptr;
             ShadowResult s;
-            if (WALK == 2) {
-                const int* e = exits + (long long)j * (prm.rows + prm.cols);
-                const int kend = min(K, min(__ldg(&e[r]), __ldg(&e[prm.rows + c])));
-                s = shadow_walk_packed<false>(geo32, prm.cols, p, a, top_p, bush, 0.0, ray + base, dz + base,
-                                              nullptr, K, kend, prm.hmax, ceil_j);
-            } else if (WALK == 1) {
+            if (WALK == 1) {
                 s = shadow_walk_geo(GeoF32x4{geo32}, prm.rows, prm.cols, r, c, a, top_p, bush, 0.0, ray + base,
                                     dz + base, K, prm.hmax, true, ceil_j);
             } else {
@@ -88,16 +79,17 @@ __global__ void __launch_bounds__(32 * kSvfWarps, 8) svf_visibility_kernel(
     }
 }
 
-// The step-record form (WALK 3) with one warp per 8 x 4 pixel tile walking
-// all patches of the word in turn (grid.x: tiles / 8, one word per launch):
-// the warps of a block carry similar work -- each walks all 32 patches of
-// its own pixels, so the uneven lengths of single walks (window skips,
-// ceiling exits) even out -- and each pixel's two bits are assembled in
-// registers, so no warp waits at a barrier.  Same walks, same bits.
+// The form on the packed geometry with ceilings, exits and step records, one
+// warp per 8 x 4 pixel tile walking all patches of the word in turn (grid.x:
+// tiles / 8, one word per launch): the warps of a block carry similar work --
+// each walks all 32 patches of its own pixels, so the uneven lengths of single
+// walks even out -- and each pixel's two bits are assembled in registers, so no
+// warp waits at a barrier.  Same bits as svf_visibility_kernel.
 __global__ void __launch_bounds__(32 * kSvfWarps, 8) svf_visibility_warp_kernel(
-    const float4* __restrict__ geo32, const uint8_t* __restrict__ flags, SvfRayParams prm,
-    const int32_t* __restrict__ lengths, uint32_t* __restrict__ masks, int word, const float2* __restrict__ ceiling,
-    const int* __restrict__ exits, const longlong2* __restrict__ rec, int kmax) {
+    const float4* __restrict__ geo32, const float* __restrict__ height, const uint8_t* __restrict__ flags,
+    SvfRayParams prm, const double* __restrict__ dz, const int32_t* __restrict__ lengths, uint32_t* __restrict__ masks,
+    int word, const float2* __restrict__ ceiling, const int* __restrict__ exits, const int2* __restrict__ rec,
+    int kpitch) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long long pixels = (long long)prm.rows * prm.cols;
     const int tiles_x = (prm.cols + 7) / 8;
@@ -107,9 +99,8 @@ __global__ void __launch_bounds__(32 * kSvfWarps, 8) svf_visibility_warp_kernel(
     const int rr = (int)(tile / tiles_x) * 4 + (lane >> 3), cc = (int)(tile % tiles_x) * 8 + (lane & 7);
     if (rr >= prm.rows || cc >= prm.cols) return;
     const long long p = (long long)rr * prm.cols + cc;
-    const float4 g = __ldg(&geo32[p]);  // the packed geometry holds the exact heights
-    const double a = g.x, top_p = g.y;
     const bool bush = flags[p] & 2;
+    const float hmax = __double2float_ru(prm.hmax);
     uint32_t sbits = 0u, vbits = 0u;
     for (int j = 0; j < kSvfPatchGroup; ++j) {
         const int patch = word * kSvfPatchGroup + j;
@@ -117,9 +108,9 @@ __global__ void __launch_bounds__(32 * kSvfWarps, 8) svf_visibility_warp_kernel(
         const int K = lengths[patch];
         const int* e = exits + (long long)j * (prm.rows + prm.cols);
         const int kend = min(K, min(__ldg(&e[rr]), __ldg(&e[prm.rows + cc])));
-        const ShadowResult s = shadow_walk_packed<true>(geo32, prm.cols, p, a, top_p, bush, 0.0, nullptr, nullptr,
-                                                        rec + (long long)j * kmax, K, kend, prm.hmax,
-                                                        ceiling + (long long)j * pixels);
+        const ShadowResult s = shadow_walk_packed(geo32, height, ceiling + (long long)j * pixels, (uint32_t)p, bush, 0.0,
+                                                  rec + (long long)j * kpitch,
+                                                  dz + (long long)patch * prm.capacity, K, kend, hmax);
         sbits |= (s.shadowed ? 0u : 1u) << j;
         vbits |= (s.ever ? 1u : 0u) << j;
     }
@@ -321,7 +312,7 @@ __global__ void __launch_bounds__(1024) patch_ray_exits_kernel(int rows, int col
                                                                const double* __restrict__ dz,
                                                                const int32_t* __restrict__ lengths, int capacity,
                                                                int patch0, int count, int* __restrict__ exits,
-                                                               longlong2* __restrict__ rec, int kmax) {
+                                                               int2* __restrict__ rec, int kmax) {
     const int j = blockIdx.x;
     if (j >= count) return;
     const int patch = patch0 + j;
@@ -329,7 +320,7 @@ __global__ void __launch_bounds__(1024) patch_ray_exits_kernel(int rows, int col
                     exits + (long long)j * (rows + cols));
     if (rec != nullptr)
         ray_records_block(rays + (long long)patch * capacity, dz + (long long)patch * capacity,
-                          min(lengths[patch], kmax), cols, rec + (long long)j * kmax);
+                          min(lengths[patch], kmax), cols, rec + (long long)j * record_pitch(kmax));
 }
 
 // Ray tables of the sky patches (src/svf.py:47-75): steps k = 0, 1, ... of the
@@ -371,11 +362,11 @@ __global__ void __launch_bounds__(256) svf_ray_tables_kernel(const __grid_consta
     if (threadIdx.x == 0) lengths[p] = amax < 0 ? 0 : first + 1;
 }
 
-// Work of solweig_svf_ex2: 4 dilated height planes, the 32 ray-ceiling
+// Work of solweig_svf_ex2: 4 dilated height planes and the plane of H, the 32 ray-ceiling
 // planes (ceiling and window maximum per pixel) of one patch word, its 32 first-outside tables and its step
 // records (kmax = max(rows, cols) + 2 per patch, >= every ray's length).
 struct SvfWork {
-    long long dil, ceil, exits, rec, total;
+    long long dil, height, ceil, exits, rec, total;
     int kmax;
 };
 
@@ -384,10 +375,11 @@ SvfWork svf_work_layout(int rows, int cols) {
     SvfWork w{};
     w.kmax = (rows > cols ? rows : cols) + 2;
     w.dil = 0;
-    w.ceil = (4LL * 4 * px + 255) & ~255LL;
+    w.height = 4LL * 4 * px;
+    w.ceil = (5LL * 4 * px + 255) & ~255LL;
     w.exits = (w.ceil + 8LL * kSvfPatchGroup * px + 255) & ~255LL;
     w.rec = (w.exits + 4LL * kSvfPatchGroup * (rows + cols) + 255) & ~255LL;
-    w.total = w.rec + 16LL * kSvfPatchGroup * w.kmax;
+    w.total = w.rec + 8LL * kSvfPatchGroup * record_pitch(w.kmax);
     return w;
 }
 
@@ -482,9 +474,9 @@ int svf_impl(const double* dsm, const double* vegdem, const double* vegdem2, con
     if (!work) {
         dim3 grid(svf_tiles(rows, cols), words);
         if (g4) svf_visibility_kernel<1><<<grid, 32 * kSvfWarps, 0, st>>>(dsm, vegdem, vegdem2, g4, flags, rp, rays,
-                                                                          ray_dz, lengths, masks, 0, nullptr, nullptr);
+                                                                          ray_dz, lengths, masks, 0, nullptr);
         else svf_visibility_kernel<0><<<grid, 32 * kSvfWarps, 0, st>>>(dsm, vegdem, vegdem2, g4, flags, rp, rays,
-                                                                       ray_dz, lengths, masks, 0, nullptr, nullptr);
+                                                                       ray_dz, lengths, masks, 0, nullptr);
         SOLWEIG_CHECK_LAUNCH("svf_visibility_kernel");
     } else {
         const SvfWork w = svf_work_layout(rows, cols);
@@ -496,7 +488,8 @@ int svf_impl(const double* dsm, const double* vegdem, const double* vegdem2, con
         float2* ceil = reinterpret_cast<float2*>(wb + w.ceil);
         int* exits = reinterpret_cast<int*>(wb + w.exits);
         // step records when every ray fits kmax (the host's ray tables do)
-        longlong2* rec = (g4 && capacity <= w.kmax) ? reinterpret_cast<longlong2*>(wb + w.rec) : nullptr;
+        int2* rec = (g4 && capacity <= w.kmax && pixels <= kPackedMaxPixels) ? reinterpret_cast<int2*>(wb + w.rec) : nullptr;
+        float* height = reinterpret_cast<float*>(wb + w.height);
         SolweigScene S{};
         S.rows = rows;
         S.cols = cols;
@@ -505,8 +498,8 @@ int svf_impl(const double* dsm, const double* vegdem, const double* vegdem2, con
         S.vegdem2 = vegdem2;
         S.geo32 = geo32;
         dim3 dgrid(blocks_for(cols, kDilTile), blocks_for(rows, kDilTile));
-        if (geo32) ceiling_dilate_kernel<true><<<dgrid, dim3(32, 8), 0, st>>>(S, dil);
-        else ceiling_dilate_kernel<false><<<dgrid, dim3(32, 8), 0, st>>>(S, dil);
+        if (geo32) ceiling_dilate_kernel<true><<<dgrid, dim3(32, 8), 0, st>>>(S, dil, height);
+        else ceiling_dilate_kernel<false><<<dgrid, dim3(32, 8), 0, st>>>(S, dil, nullptr);
         SOLWEIG_CHECK_LAUNCH("ceiling_dilate_kernel");
         for (int wd = 0; wd < words; ++wd) {
             const int p0 = wd * kSvfPatchGroup, cnt = std::min(kSvfPatchGroup, patches - p0);
@@ -518,14 +511,15 @@ int svf_impl(const double* dsm, const double* vegdem, const double* vegdem2, con
                                                           rec, w.kmax);
             SOLWEIG_CHECK_LAUNCH("patch_ray_exits_kernel");
             dim3 grid(svf_tiles(rows, cols), 1);
-            if (rec) svf_visibility_warp_kernel<<<blocks_for(svf_tiles(rows, cols), kSvfWarps), 32 * kSvfWarps, 0,
-                                                   st>>>(g4, flags, rp, lengths, masks, wd, ceil, exits, rec, w.kmax);
-            else if (g4) svf_visibility_kernel<2><<<grid, 32 * kSvfWarps, 0, st>>>(dsm, vegdem, vegdem2, g4, flags,
-                                                                                   rp, rays, ray_dz, lengths, masks,
-                                                                                   wd, ceil, exits);
-            else svf_visibility_kernel<0><<<grid, 32 * kSvfWarps, 0, st>>>(dsm, vegdem, vegdem2, g4, flags, rp,
-                                                                           rays, ray_dz, lengths, masks, wd, ceil,
-                                                                           nullptr);
+            if (rec)
+                svf_visibility_warp_kernel<<<blocks_for(svf_tiles(rows, cols), kSvfWarps), 32 * kSvfWarps, 0, st>>>(
+                    g4, height, flags, rp, ray_dz, lengths, masks, wd, ceil, exits, rec, record_pitch(w.kmax));
+            else if (g4)
+                svf_visibility_kernel<1><<<grid, 32 * kSvfWarps, 0, st>>>(dsm, vegdem, vegdem2, g4, flags, rp, rays,
+                                                                          ray_dz, lengths, masks, wd, ceil);
+            else
+                svf_visibility_kernel<0><<<grid, 32 * kSvfWarps, 0, st>>>(dsm, vegdem, vegdem2, g4, flags, rp, rays,
+                                                                          ray_dz, lengths, masks, wd, ceil);
             SOLWEIG_CHECK_LAUNCH("svf_visibility_kernel");
         }
     }
