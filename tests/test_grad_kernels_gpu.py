@@ -1,0 +1,52 @@
+"""Kernels of the day gradient at the edges of their tiles, passes and warps."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(rows, cols, hours, objective="utci", seed=3):
+    import torch
+    from solweig_cuda_b200 import engine, grad, synthetic
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    sc = synthetic.make_scene(rows, cols, seed=seed)
+    scene = engine.Scene(sc.dsm, sc.trees, sc.dem, 1.0, landcover=sc.landcover)
+    met = synthetic.make_met(doy=172, latitude=53.0, longitude=0.0, seed=4)[24 - hours:] if hours < 24 else \
+        synthetic.make_met(doy=172, latitude=53.0, longitude=0.0, seed=4)
+    rng = np.random.default_rng(5)
+    p = [rng.uniform(a, b, scene.shape).astype(np.float32) for a, b in ((0.1, 0.4), (0.9, 0.98), (0.02, 0.2))]
+    return scene, grad.DayGradient(scene, 53.0, 0.0, 3.0, 0.0, hours=hours, objective=objective), p, met
+
+
+# fewer pixels than a warp, one more than a warp's 32, several blocks; daytime
+# hours that fill their passes of four and that do not
+@pytest.mark.parametrize("rows,cols,hours", [(5, 6, 24), (3, 11, 7), (37, 41, 9), (70, 65, 24)])
+def test_luminance_gradient_is_the_masks_times_the_pixel_adjoints(rows, cols, hours):
+    """With the weight on one pixel every patch it sees has the same partial and
+    the others none; over all pixels the partials add up (float32 chains of at
+    most 512 additions)."""
+    scene, dg, p, met = _case(rows, cols, hours, "tmrt")
+    P = dg.patches
+    bits = np.unpackbits(scene.masks.cpu().numpy().view(np.uint8).reshape(2, -1, rows * cols, 4).transpose(0, 2, 1, 3)
+                         .reshape(2, rows * cols, -1), axis=2, bitorder="little")[:, :, :P].astype(bool)
+    sky, veg = bits[0] & ~bits[1], bits[0] & bits[1]
+    pixels = range(rows * cols) if rows * cols <= 33 else (0, 31, 32, rows * cols // 2, rows * cols - 1)
+    total = np.zeros((hours, 4, P))
+    for q in pixels:
+        w = np.zeros((rows, cols), np.float32)
+        w.flat[q] = 1.25
+        lum = dg.backward(*p, met, w)[4][:, :, :P]
+        total += lum
+        for hr in range(hours):
+            for i, mask in enumerate((sky[q], sky[q], veg[q], veg[q])):
+                assert not lum[hr, i, ~mask].any()
+                assert np.unique(lum[hr, i, mask]).size <= 1
+        if sky[q].any() and veg[q].any():
+            for i in (0, 1):
+                a, b = lum[:, i, sky[q]][:, 0], lum[:, i + 2, veg[q]][:, 0]
+                assert np.abs(b - 0.03 * a).max() <= 2e-7 * np.abs(a).max()
+        assert lum.any()
+    if rows * cols <= 33:
+        lum = dg.backward(*p, met, np.full((rows, cols), 1.25, np.float32))[4][:, :, :P]
+        assert np.abs(lum - total).max() <= 512 * 2.0 ** -24 * np.abs(total).max()
