@@ -70,18 +70,6 @@ extern "C" int solweig_day_batched_layout(int rows, int cols, int nhours, int ha
 
 namespace {
 
-int launch_gvf_walks(const SolweigScene& S, const int32_t* gvf_dxdy, int second, uint32_t* hits, uint32_t* walks,
-                     float* nosh, cudaStream_t st) {
-    GvfTable<kWkMaxSteps> tab;
-    fill_day_table(tab, gvf_dxdy, second, kWkMaxWidth);
-    const size_t smem = gvf_walks_smem_bytes();
-    set_smem_attr((const void*)gvf_walks_kernel, smem);
-    dim3 grid(blocks_for(S.cols, kWkTile), blocks_for(S.rows, kWkTile));
-    gvf_walks_kernel<<<grid, kWkPixels, smem, st>>>(S, second, tab, hits, walks, nosh);
-    SOLWEIG_CHECK_LAUNCH("gvf_walks_kernel");
-    return SOLWEIG_OK;
-}
-
 // Shared by the two entry points: `second` of solweig_gvf_statics is fixed.
 int gvf_scene_walks(const char* name, const SolweigScene* scene, const int32_t* gvf_dxdy, int second, uint32_t* hits,
                     uint32_t* walks, float* nosh, void* stream) {
@@ -301,38 +289,25 @@ int day_batched_impl(const SolweigScene* scene, const SolweigSkyLayout* layout, 
     }
     // kDayRest (the error flag was cleared by the sweep part of hour 0)
     DayWalkArgs wa;
-    wa.second = second_steps;
-    wa.halo = second_steps - 1;
-    wa.width = kWkTile + 2 * wa.halo;
     // The walk-word kernel: walks of 2 to 22 steps from the pixel itself (pixels
     // of 0.98 m and more), no water (whose first direction reads another Lup);
     // the per-hour kernel takes the rest (0.996 against 0.202 ms per 517 x 389
     // px day at 2 m).
     if (cfg.gvf_hours == 1 && !S.has_water && first_steps == 1 && second_steps >= 2 && second_steps <= kWkMaxSteps &&
-        walk_offsets(gvf_dxdy, second_steps, wa.width, &wa.at)) {
+        day_walk_args(gvf_dxdy, second_steps, &wa)) {
         uint32_t* walks = reinterpret_cast<uint32_t*>(wb + w.walks);
         const bool statics = S.gvf_walks && S.gvf_nosh && ((uintptr_t)S.gvf_walks & 15) == 0;
         if (!statics) {
             const int rc = launch_gvf_walks(S, gvf_dxdy, second_steps, nullptr, walks, nosh, st);
             if (rc) return rc;
         }
-        wa.magic = (uint32_t)((0x100000000ull + wa.width - 1) / wa.width);
         wa.walks = statics ? S.gvf_walks : walks;
-        // the samples' codes (4 B per pixel and pass) and the tiles' values live
-        // in the patch-sum region (16 B per pixel-hour), free until the contraction
-        const int passes = (nhours + kWkHours - 1) / kWkHours;
-        uint32_t* codes = reinterpret_cast<uint32_t*>(sums);
-        unsigned long long* dict = reinterpret_cast<unsigned long long*>(wb + w.dict);
-        wa.codes = codes;
-        wa.dict = dict;
-        const dim3 grid(blocks_for(S.cols, kWkTile), blocks_for(S.rows, kWkTile), passes);
-        gvf_codes_kernel<<<grid, kWkCodeThreads, 0, st>>>(
-            S.rows, S.cols, hours, nhours, quads, codes, dict, gvf, statics ? S.gvf_nosh : nullptr, nosh);
-        SOLWEIG_CHECK_LAUNCH("gvf_codes_kernel");
-        const size_t smem = day_walk_smem_bytes(wa.width);
-        set_smem_attr((const void*)day_gvf_walk_kernel, smem);
-        day_gvf_walk_kernel<<<grid, kWkThreads, smem, st>>>(S, hours, nhours, wa, quads, gvf);
-        SOLWEIG_CHECK_LAUNCH("day_gvf_walk_kernel");
+        // the samples' codes (4 B per pixel and pass) live in the patch-sum
+        // region (16 B per pixel-hour), free until the contraction
+        const int rc = launch_day_walk(S, hours, nhours, wa, quads, reinterpret_cast<uint32_t*>(sums),
+                                       reinterpret_cast<unsigned long long*>(wb + w.dict), gvf,
+                                       statics ? S.gvf_nosh : nullptr, nosh, st);
+        if (rc) return rc;
     } else if (first_steps == 1 && second_steps == 22) {
         cudaMemsetAsync(nosh, 0, 4 * px, st);
         GvfTable<22> tab;

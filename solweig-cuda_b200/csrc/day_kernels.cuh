@@ -1115,6 +1115,46 @@ void fill_day_table(GvfTable<TABLE>& tab, const int32_t* dxdy, int second, int p
     }
 }
 
+int launch_gvf_walks(const SolweigScene& S, const int32_t* gvf_dxdy, int second, uint32_t* hits, uint32_t* walks,
+                     float* nosh, cudaStream_t st) {
+    GvfTable<kWkMaxSteps> tab;
+    fill_day_table(tab, gvf_dxdy, second, kWkMaxWidth);
+    const size_t smem = gvf_walks_smem_bytes();
+    set_smem_attr((const void*)gvf_walks_kernel, smem);
+    dim3 grid(blocks_for(S.cols, kWkTile), blocks_for(S.rows, kWkTile));
+    gvf_walks_kernel<<<grid, kWkPixels, smem, st>>>(S, second, tab, hits, walks, nosh);
+    SOLWEIG_CHECK_LAUNCH("gvf_walks_kernel");
+    return SOLWEIG_OK;
+}
+
+// Arguments of the walk-word kernels for a table of walks; false unless every
+// walk starts at its pixel.
+bool day_walk_args(const int32_t* gvf_dxdy, int second, DayWalkArgs* wa) {
+    wa->second = second;
+    wa->halo = second - 1;
+    wa->width = kWkTile + 2 * wa->halo;
+    wa->magic = (uint32_t)((0x100000000ull + wa->width - 1) / wa->width);
+    return walk_offsets(gvf_dxdy, second, wa->width, &wa->at);
+}
+
+// The GVF planes of every daytime hour from the walk words in wa: codes takes
+// 4 bytes per pixel and pass of four hours.
+int launch_day_walk(const SolweigScene& S, const SolweigHour* hours, int nhours, DayWalkArgs& wa, const float4* quads,
+                    uint32_t* codes, unsigned long long* dict, float* gvf, const float* nosh_in, float* nosh,
+                    cudaStream_t st) {
+    wa.codes = codes;
+    wa.dict = dict;
+    const dim3 grid(blocks_for(S.cols, kWkTile), blocks_for(S.rows, kWkTile), (nhours + kWkHours - 1) / kWkHours);
+    gvf_codes_kernel<<<grid, kWkCodeThreads, 0, st>>>(S.rows, S.cols, hours, nhours, quads, codes, dict, gvf, nosh_in,
+                                                      nosh);
+    SOLWEIG_CHECK_LAUNCH("gvf_codes_kernel");
+    const size_t smem = day_walk_smem_bytes(wa.width);
+    set_smem_attr((const void*)day_gvf_walk_kernel, smem);
+    day_gvf_walk_kernel<<<grid, kWkThreads, smem, st>>>(S, hours, nhours, wa, quads, gvf);
+    SOLWEIG_CHECK_LAUNCH("day_gvf_walk_kernel");
+    return SOLWEIG_OK;
+}
+
 template <int TY, int FIRST, int SECOND, int TABLE>
 void launch_day_gvf_ty(const SolweigScene& S, const SolweigHour* hours, int nhours, const DayGvfArgs& ga,
                        const GvfTable<TABLE>& tab, const float4* quads, const float* lup_first, float* gvf,

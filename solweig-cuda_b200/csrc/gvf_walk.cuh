@@ -546,17 +546,16 @@ __global__ void __launch_bounds__(kWkPixels, 1) gvf_walks_kernel(SolweigScene S,
     constexpr int halo = kWkMaxSteps - 1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float* albs = reinterpret_cast<float*>(smem_raw);
-    uint8_t* bits = reinterpret_cast<uint8_t*>(albs + kWkStagedN);  // 1 ground, 2 wall
+    uint8_t* bits = reinterpret_cast<uint8_t*>(albs + kWkStagedN);  // 1 ground, 2 wall, 4 outside
     const int tr = blockIdx.y, tc = blockIdx.x;
     const int tid = threadIdx.x;
     const long long n = (long long)S.rows * S.cols;
     const int row0 = tr * kWkTile - halo, col0 = tc * kWkTile - halo;
-    const bool interior = row0 >= 0 && col0 >= 0 && row0 + kWkMaxWidth <= S.rows && col0 + kWkMaxWidth <= S.cols;
     for (int i = tid; i < kWkStagedN; i += kWkPixels) {
         const int rr = row0 + i / kWkMaxWidth, cc = col0 + i % kWkMaxWidth;
-        const bool in = interior || in_raster(rr, cc, S.rows, S.cols);
+        const bool in = in_raster(rr, cc, S.rows, S.cols);
         const long long q = in ? (long long)rr * S.cols + cc : 0;
-        bits[i] = in ? (uint8_t)((S.flags[q] & 1) | (S.walls[q] > 0.0 ? 2 : 0)) : (uint8_t)0;
+        bits[i] = in ? (uint8_t)((S.flags[q] & 1) | (S.walls[q] > 0.0 ? 2 : 0)) : (uint8_t)4;
         albs[i] = in ? S.alb[q] : 0.f;
     }
     __syncthreads();
@@ -573,33 +572,30 @@ __global__ void __launch_bounds__(kWkPixels, 1) gvf_walks_kernel(SolweigScene S,
     const float inv_second = 1.f / (float)second;
     float nsh = 0.f;
     uint32_t hits[4] = {0u, 0u, 0u, 0u};
+#pragma unroll 1
     for (int j = 0; j < kWkDirs; ++j) {
         int hit = 0, lim = 0;
         uint32_t walls = 0u;
         float s_alb = 0.f, n_alb = 0.f;
         if (own_ground) {
-            hit = lim = second;
-            for (int m = 0; m < second; ++m) {
-                if (!interior) {
-                    const int2 o = tab.offs[j * second + m];
-                    if (!in_raster(r + o.x, c + o.y, S.rows, S.cols)) {
-                        // frozen tail: step m (> 0: step 0 is the pixel) and the rest repeat step m - 1
-                        lim = m;
-                        const float al = albs[own + tab.delta[j * second + m - 1]];
-                        s_alb += al;
-                        s_alb += (second - 1 - m) * al;
-                        break;
-                    }
-                }
-                const int at = own + tab.delta[j * second + m];
-                const uint32_t b = bits[at];
-                if (!(b & 1u)) {
-                    hit = lim = m;
-                    break;
-                }
-                walls |= (b >> 1) << m;
+            const int* delta = tab.delta + j * second;
+            uint32_t b = 1u;
+            int m = 0;
+#pragma unroll 2
+            for (; m < second; ++m) {
+                const int at = own + delta[m];
+                b = bits[at];
+                if (!(b & 1u)) break;
+                if (b & 2u) walls |= 1u << m;
                 s_alb += albs[at];
-                if (m == 0) n_alb = s_alb;
+            }
+            n_alb = albs[own + delta[0]];
+            hit = lim = m;
+            if (b & 4u) {  // frozen tail: step m (> 0: step 0 is the pixel) and the rest repeat step m - 1
+                hit = second;
+                const float al = albs[own + delta[m - 1]];
+                s_alb += al;
+                s_alb += (second - 1 - m) * al;
             }
         }
         const bool frozen = hit > lim;

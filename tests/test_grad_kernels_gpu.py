@@ -50,3 +50,56 @@ def test_luminance_gradient_is_the_masks_times_the_pixel_adjoints(rows, cols, ho
     if rows * cols <= 33:
         lum = dg.backward(*p, met, np.full((rows, cols), 1.25, np.float32))[4][:, :, :P]
         assert np.abs(lum - total).max() <= 512 * 2.0 ** -24 * np.abs(total).max()
+
+
+# one tile, a column and a row more, less than a tile both ways, several tiles;
+# an odd number of daytime hours and one pass
+@pytest.mark.parametrize("rows,cols,hours", [(32, 32, 24), (33, 32, 9), (20, 45, 8), (70, 65, 24)])
+def test_transposed_walks_match_differences_at_tile_and_raster_edges(rows, cols, hours):
+    """Central differences of the forward in the albedo and emissivity of the
+    pixels at the raster's border and along the 32-pixel tiles' edges (relative
+    tolerance of the differences as for whole fields: 1e-3)."""
+    scene, dg, p, met = _case(rows, cols, hours)
+    rng = np.random.default_rng(8)
+    weights = rng.uniform(0.5, 1.5, (rows, cols)).astype(np.float32)
+    grads = dg.backward(*p, met, weights)[:2]
+    edges = np.zeros((rows, cols), bool)
+    for r in (0, 1, 31, 32, rows - 1):
+        edges[min(r, rows - 1)] = True
+    for c in (0, 1, 31, 32, cols - 1):
+        edges[:, min(c, cols - 1)] = True
+    for i in (0, 1):
+        v = np.where(edges, rng.uniform(0.5, 1.0, (rows, cols)), 0.0)
+        J = []
+        for h in (1e-2, -1e-2):
+            q = list(p)
+            q[i] = (p[i].astype(np.float64) + h * v).astype(np.float32)
+            J.append(float(np.nansum(dg.forward(*q, met).cpu().numpy() * weights)))
+        fd = (J[0] - J[1]) / 2e-2
+        ad = float((grads[i].cpu().numpy().astype(np.float64) * v).sum())
+        assert abs(ad - fd) <= 1e-3 * abs(fd), (i, ad, fd)
+
+
+@pytest.mark.parametrize("hours", [24, 9])
+def test_walks_that_do_not_start_at_their_pixel_take_the_general_path(hours):
+    """A table whose walks start one step out has no walk words: the general
+    kernels stay consistent with each other."""
+    scene, dg, p, met = _case(40, 37, hours)
+    table = scene.gvf_dxdy_host.reshape(-1)
+    assert np.shares_memory(table, scene.gvf_dxdy_host)
+    saved = table.copy()
+    try:
+        steps = table.reshape(18, 22, 2)
+        steps[:, 0] = steps[:, 1]
+        rng = np.random.default_rng(8)
+        w = rng.uniform(0.5, 1.5, scene.shape).astype(np.float32)
+        grad = dg.backward(*p, met, w)[0].cpu().numpy().astype(np.float64)
+        v = rng.uniform(0.5, 1.0, scene.shape)
+        J = []
+        for h in (1e-2, -1e-2):
+            a = (p[0].astype(np.float64) + h * v).astype(np.float32)
+            J.append(float(np.nansum(dg.forward(a, p[1], p[2], met).cpu().numpy() * w)))
+        fd = (J[0] - J[1]) / 2e-2
+        assert abs(float((grad * v).sum()) - fd) <= 1e-3 * abs(fd)
+    finally:
+        table[:] = saved
