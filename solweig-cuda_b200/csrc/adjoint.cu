@@ -13,7 +13,7 @@
 //
 //  forward (also re-run by the backward: per-hour recomputation, nothing is
 //  kept from the forward call)
-//    day_shadow_kernel        masks of every hour (shadow sweep, psi of the hour)
+//    the day's sweep stage    masks of every hour (shadow sweep, psi of the hour)
 //    param_quads_kernel       GVF field quads from the parameters: shadow with t,
 //                             Lup with e, albedo a
 //    gvf_walks_kernel         walk words and the albedo-without-shadow plane
@@ -80,7 +80,8 @@ struct GradPtrs {
 __global__ void param_quads_kernel(SolweigScene S, const SolweigHour* __restrict__ hours, int nhours,
                                    const float4* __restrict__ q0, float4* __restrict__ q1,
                                    uint8_t* __restrict__ sv, const float* __restrict__ alb,
-                                   const float* __restrict__ emis, const float* __restrict__ tau) {
+                                   const float* __restrict__ emis, const float* __restrict__ tau,
+                                   const int* __restrict__ error) {
     const long long n = (long long)S.rows * S.cols;
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= n * nhours) return;
@@ -91,6 +92,12 @@ __global__ void param_quads_kernel(SolweigScene S, const SolweigHour* __restrict
     const float4 q = q0[idx];
     const float s0 = q.x;
     const float psi = (float)h.psi;
+    if (*error) {  // a ray longer than the sweep's records: no result rather than a wrong one
+        const float nan = __int_as_float(0x7fffffff);
+        sv[idx] = 0;
+        q1[idx] = make_float4(nan, nan, nan, q.w);
+        return;
+    }
     // shadow = (float)(sh - (1 - vegsh)(1 - psi)): 1, psi, 0 or psi - 1
     int sh, vegsh;
     if (s0 == 1.0f) { sh = 1; vegsh = 1; }
@@ -1131,16 +1138,16 @@ static int grad_prepare(const SolweigScene* scene, const SolweigSkyLayout* layou
     __nv_bfloat16* bw = reinterpret_cast<__nv_bfloat16*>(wb + dw.bw);
     DayTable* tables = reinterpret_cast<DayTable*>(wb + dw.tables);
     int* err = reinterpret_cast<int*>(wb + dw.error);
-    cudaMemsetAsync(err, 0, sizeof(int), st);
-    {
-        dim3 grid(blocks_for(S.cols, 16), blocks_for(S.rows, 16), nhours);
-        day_shadow_kernel<false><<<grid, dim3(16, 16), 0, st>>>(S, hours, quads0, nullptr, nullptr, nullptr,
-                                                                nullptr, 0, nullptr);
-        SOLWEIG_CHECK_LAUNCH("day_shadow_kernel");
-    }
+    // The batched day's sweep stage (ray ceilings, step records and the sweep,
+    // which also clears the error flag) in the same work regions: 0.58 -> 0.25 ms
+    // for 17 hours of 500 x 500 pixels against the sweep alone.
+    const SolweigOutputs none{};
+    int rc = solweig_day_batched_part(scene, layout, hours, nhours, nullptr, &none, 0, gvf_dxdy, first_steps,
+                                      second_steps, work, work_bytes, nullptr, 0, 0, nhours, st);
+    if (rc) return rc;
     param_quads_kernel<<<blocks_for(px * nhours, 256), 256, 0, st>>>(S, hours, nhours, quads0, quads1, sv,
                                                                       prm->albedo, prm->emissivity,
-                                                                      prm->transmissivity);
+                                                                      prm->transmissivity, err);
     SOLWEIG_CHECK_LAUNCH("param_quads_kernel");
     Sp = S;
     Sp.emis = prm->emissivity;
@@ -1152,7 +1159,7 @@ static int grad_prepare(const SolweigScene* scene, const SolweigSkyLayout* layou
     walk_words = day_walk_args(gvf_dxdy, second_steps, &wa);
     if (walk_words) {
         uint32_t* walks = reinterpret_cast<uint32_t*>(wb + dw.walks);
-        int rc = launch_gvf_walks(Sp, gvf_dxdy, second_steps, nullptr, walks, nosh, st);
+        rc = launch_gvf_walks(Sp, gvf_dxdy, second_steps, nullptr, walks, nosh, st);
         if (rc) return rc;
         wa.walks = walks;
         rc = launch_day_walk(Sp, hours, nhours, wa, quads1, reinterpret_cast<uint32_t*>(wb + gw.codes),
