@@ -833,29 +833,6 @@ __device__ __forceinline__ float* hour_plane(float* base, int hr, long long stri
     return base ? base + hr * stride : nullptr;
 }
 
-// Fraction of shaded wall (cylindric_wedge, NaN -> 0.5) in float32.
-__device__ __forceinline__ float wedge_fsh_f(float ta, float tan_zen) {
-    const float xa = 1.f - 2.f / (ta * tan_zen);
-    const float ha = 2.f / (ta * tan_zen);
-    const float ba = 1.f / ta;
-    const float hkil = 2.f * ba * ha;
-    float ukil = 0.f;
-    if (xa < 0.f) {
-        // phi = atan(za / qa) in [0, pi/2): cos and sin from the same triangle,
-        // 1 / hypot(qa, za) with qa^2 + za^2 = ba^2 + 3 qa^2 / 4
-        const float qa = tan_zen / 2.f;
-        const float za = sqrtf(ba * ba - qa * qa / 4.f);
-        const float phi = atanf(za / qa);
-        const float ih = rsqrtf(fmaf(qa, qa, za * za));
-        const float cphi = qa * ih, sphi = za * ih;
-        const float area = (sphi - phi * cphi) / (1.f - cphi);
-        ukil = 2.f * ba * xa * area;
-    }
-    const float pi2 = 2.f * (float)kPi;
-    const float fsh = (pi2 * ba - (hkil + ukil)) / (pi2 * ba);
-    return isnan(fsh) ? 0.5f : fsh;
-}
-
 // Flux arithmetic of the hour loop in float32 (the hour's scalars are rounded
 // once from the float64 host plan); the building split keeps its exact float64
 // thresholds.  Against the per-hour form (float64 fluxes) Tmrt differs by <
@@ -866,7 +843,7 @@ __device__ __forceinline__ float wedge_fsh_f(float ta, float tan_zen) {
 // spills).  A building patch that is not sunlit is shaded, so one pass of
 // popcounts over the sunlit patches serves both sums and both tests (POPC runs
 // at an eighth of the issue rate), and patches exactly on a limit take a branch.
-// 2000^2 day: 2.86 -> 2.00 ms.  Full occupancy (2048 resident threads per SM,
+// 2000^2 day: 2.86 -> 1.90 ms.  Full occupancy (2048 resident threads per SM,
 // 32 registers, spills) against 40 / 48 registers at 1536 / 1280 threads: 2.00
 // against 2.08 / 2.17 ms; the scalars and mask rows as 16-byte loads, which
 // live longer: 2.14 to 2.35 ms.
@@ -990,7 +967,7 @@ __global__ void __launch_bounds__(THREADS, 2048 / THREADS) day_radiation_kernel(
             const float g_lup = a.gvf[g0];
             const float g_alb = a.gvf[g0 + n];
             shadow = a.gvf[g0 + 2 * n];
-            const float fsh = wedge_fsh_f(tan_alfa, hs.tan_zen);
+            const float fsh = wedge_fsh_tan(tan_alfa, hs.tan_zen);
             const float reflected = albedo_b * (1.f - svfbuveg) * (hs.rad_g * (1.f - fsh) + hs.rad_d * fsh);
             const float base_up = hs.rad_d * svfbuveg + reflected;
             kup_all = g_alb * hs.rad_i_sin + base_up * g_nosh;

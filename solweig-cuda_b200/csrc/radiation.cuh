@@ -159,21 +159,24 @@ __device__ __forceinline__ float utci_eval(const double* c, double tmrt, double 
 }
 
 // Fraction of shaded wall, cylindric_wedge (NaN -> 0.5), from ta = tan(svfalfa).
-__device__ __forceinline__ double wedge_fsh_tan(double ta, double tan_zen) {
-    const double xa = 1.0 - 2.0 / (ta * tan_zen);
-    const double ha = 2.0 / (ta * tan_zen);
-    const double ba = 1.0 / ta;
-    const double hkil = 2.0 * ba * ha;
-    double ukil = 0.0;
-    if (xa < 0.0) {
-        const double qa = tan_zen / 2.0;
-        const double za = sqrt(ba * ba - qa * qa / 4.0);
-        const double phi = atan(za / qa);
-        const double area = (sin(phi) - phi * cos(phi)) / (1.0 - cos(phi));
-        ukil = 2.0 * ba * xa * area;
+// With h = 2 / (tan(svfalfa) tan(zenith)) the wedge's b and q satisfy b / q = h,
+// so the angle of its arc, above h = 1, is atan(t) with t^2 = h^2 - 1/4, the
+// arc's (sin - phi cos) / (1 - cos) is (t - phi) (1 + sqrt(1 + t^2)) / t^2, and
+// b drops out of the ratio: one arc tangent, two divisions and two roots
+// instead of six divisions, three roots and trigonometric functions of phi.
+// Radiation of a 2000^2 day (float32): 2.00 -> 1.90 ms; reverse pass of 500 x 500
+// pixels (float64): 2.26 -> 2.10 ms.  Its error against longer precision is no
+// larger in either type.
+template <typename T>
+__device__ __forceinline__ T wedge_fsh_tan(T ta, T tan_zen) {
+    const T h = T(2) / (ta * tan_zen);
+    T arc = T(0);
+    if (h > T(1)) {
+        const T tt = h * h - T(0.25), t = sqrt(tt);
+        arc = (T(1) - h) * ((t - atan(t)) * (T(1) + sqrt(tt + T(1))) / tt);
     }
-    const double fsh = (2.0 * kPi * ba - (hkil + ukil)) / (2.0 * kPi * ba);
-    return isnan(fsh) ? 0.5 : fsh;
+    const T fsh = T(1) - (h + arc) * T(1.0 / kPi);
+    return isnan(fsh) ? T(0.5) : fsh;
 }
 
 __device__ __forceinline__ double wedge_fsh(double svfalfa, double tan_zen) {
