@@ -98,28 +98,6 @@ struct Bands<1> {  // 145 patches: 30, 30, 24, 24, 18, 12, 6, 1
     }
 };
 
-// sum over bands of w[b] * popcount(m restricted to band b).
-template <int OPT>
-__device__ __forceinline__ float band_weighted(const uint32_t (&m)[SOLWEIG_MASK_WORDS], const float* w) {
-    float s = 0.f;
-#pragma unroll
-    for (int b = 0; b < 8; ++b) {
-        const int lo = Bands<OPT>::off(b), hi = Bands<OPT>::off(b + 1);
-        int c = 0;
-#pragma unroll
-        for (int wd = 0; wd < SOLWEIG_MASK_WORDS; ++wd) {
-            const int a = lo > wd * 32 ? lo : wd * 32;
-            const int e = hi < wd * 32 + 32 ? hi : wd * 32 + 32;
-            if (a < e) {
-                const uint32_t mask = (e - a == 32) ? 0xffffffffu : (((1u << (e - a)) - 1u) << (a - wd * 32));
-                c += __popc(m[wd] & mask);
-            }
-        }
-        s = fmaf((float)c, w[b], s);
-    }
-    return s;
-}
-
 // Sums of wcos over the patches of m, and of wcos and wsin over those of mt.
 template <int OPT>
 __device__ __forceinline__ void band_sums(const uint32_t (&m)[SOLWEIG_MASK_WORDS], const uint32_t (&mt)[SOLWEIG_MASK_WORDS],
@@ -144,21 +122,6 @@ __device__ __forceinline__ void band_sums(const uint32_t (&m)[SOLWEIG_MASK_WORDS
         tc = fmaf((float)nt, c, tc);
         ts = fmaf((float)nt, wsin[b], ts);
     }
-}
-
-// Number of entries of the ascending array a[0..n) that are <= t.
-__device__ __forceinline__ int count_le(const double* a, int n, double t) {
-    int lo = 0;
-    while (n > 0) {
-        const int half = n >> 1;
-        if (a[lo + half] <= t) {
-            lo += half + 1;
-            n -= half + 1;
-        } else {
-            n = half;
-        }
-    }
-    return lo;
 }
 
 // Monotone integer keys of the doubles (NaN excluded).
