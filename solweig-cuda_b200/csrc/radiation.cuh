@@ -18,51 +18,49 @@
 
 namespace solweig {
 
-// Per-patch values of one hour staged in shared memory (divergent indexing).
+// One patch of an hour, read by a whole warp at once (four 16-byte loads).
+struct alignas(16) PatchRow {
+    float lum, lum_cw;    // Perez luminance; times cos(alt) * omega
+    float wcos, wsin;     // omega * cos(alt), omega * sin(alt)
+    float card[4];        // longwave E,S,W,N cosines (0 = not in that half)
+    float lsky_side;      // sky longwave of the patch on a vertical surface
+    uint32_t lw_test;     // longwave sun test
+    double x_off;         // yi (added to tan(asvf))
+    double lo, hi;        // sunlit below, shaded above
+};
+
+// Values of one hour staged in shared memory.
 struct PatchSmem {
-    float lum[SOLWEIG_MAX_PATCHES];      // Perez luminance
-    float lum_cw[SOLWEIG_MAX_PATCHES];   // luminance * cos(alt) * omega
-    float wcos[SOLWEIG_MAX_PATCHES];     // omega * cos(alt)
-    float wsin[SOLWEIG_MAX_PATCHES];     // omega * sin(alt)
-    double x_off[SOLWEIG_MAX_PATCHES];   // yi (added to tan(asvf))
-    double lo[SOLWEIG_MAX_PATCHES];      // sunlit below
-    double hi[SOLWEIG_MAX_PATCHES];      // shaded above
-    uint8_t lw_test[SOLWEIG_MAX_PATCHES];
-    float card[4][SOLWEIG_MAX_PATCHES];  // longwave E,S,W,N cosines (0 = not in that half)
-    float lsky_side[SOLWEIG_MAX_PATCHES];  // sky longwave of the patch on a vertical surface
+    PatchRow row[SOLWEIG_MAX_PATCHES];
     float band_down[SOLWEIG_MAX_BANDS];  // sky longwave per visible patch, horizontal
     float band_side[SOLWEIG_MAX_BANDS];  // sky longwave per visible patch, vertical
-    uint32_t valid[SOLWEIG_MASK_WORDS];  // bits of existing patches
+    int patches;
 };
 
 __device__ __forceinline__ void stage_patches(PatchSmem& sm, const SolweigSkyLayout& L,
                                               const SolweigHour& h) {
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
     const int nt = blockDim.x * blockDim.y;
-    for (int k = tid; k < SOLWEIG_MAX_PATCHES; k += nt) {
-        const bool ok = k < L.patches;
-        sm.lum[k] = ok ? h.lum[k] : 0.f;
-        sm.lum_cw[k] = ok ? h.lum[k] * L.cos_alt[k] * L.omega[k] : 0.f;
-        sm.wcos[k] = ok ? L.omega[k] * L.cos_alt[k] : 0.f;
-        sm.wsin[k] = ok ? L.omega[k] * L.sin_alt[k] : 0.f;
-        sm.x_off[k] = ok ? h.yi[k] : 0.0;
-        sm.lo[k] = ok ? L.sunlit_below[k] : 0.0;
-        sm.hi[k] = ok ? L.shaded_above[k] : 0.0;
-        sm.lw_test[k] = ok ? h.lw_sun_test[k] : 0;
-        for (int d = 0; d < 4; ++d) sm.card[d][k] = ok ? L.cardinal[d][k] : 0.f;
-        const int b = ok ? L.band_of_patch[k] : 0;
-        sm.lsky_side[k] = ok ? h.band_lsky[b] * L.band_omega[b] * L.band_cos[b] : 0.f;
+    for (int k = tid; k < L.patches; k += nt) {
+        PatchRow& row = sm.row[k];
+        row.lum = h.lum[k];
+        row.lum_cw = h.lum[k] * L.cos_alt[k] * L.omega[k];
+        row.wcos = L.omega[k] * L.cos_alt[k];
+        row.wsin = L.omega[k] * L.sin_alt[k];
+        for (int d = 0; d < 4; ++d) row.card[d] = L.cardinal[d][k];
+        const int b = L.band_of_patch[k];
+        row.lsky_side = h.band_lsky[b] * L.band_omega[b] * L.band_cos[b];
+        row.lw_test = h.lw_sun_test[k];
+        row.x_off = h.yi[k];
+        row.lo = L.sunlit_below[k];
+        row.hi = L.shaded_above[k];
     }
     if (tid < SOLWEIG_MAX_BANDS) {
         const bool ok = tid < L.nbands;
         sm.band_down[tid] = ok ? h.band_lsky[tid] * L.band_omega[tid] * L.band_sin[tid] : 0.f;
         sm.band_side[tid] = ok ? h.band_lsky[tid] * L.band_omega[tid] * L.band_cos[tid] : 0.f;
     }
-    if (tid < SOLWEIG_MASK_WORDS) {
-        const int lo = tid * 32;
-        const int nbits = L.patches - lo;
-        sm.valid[tid] = nbits >= 32 ? 0xffffffffu : (nbits <= 0 ? 0u : ((1u << nbits) - 1u));
-    }
+    if (tid == 0) sm.patches = L.patches;
 }
 
 // Results of the per-pixel patch loop (weights, before hour scaling).
@@ -75,80 +73,73 @@ struct PatchSums {
     float card_sky[4], card_veg[4], card_sun[4], card_shade[4], card_obst[4];
 };
 
+// Every lane takes the patches in the same order, so a patch's values are four
+// broadcast loads and the sums conditional additions.  A loop per class over
+// each pixel's own bits (sky, vegetation, building, obstruction), with a load
+// per value and lanes at different patches, took 155 us of an hour of 400 x 360
+// pixels with the cardinal terms; this takes 70 us (four blocks per SM; three:
+// 74, five: 86).  What bounds it is instruction issue.
 template <bool Cardinal>
 __device__ __forceinline__ PatchSums patch_loop(const PatchSmem& sm, const uint32_t* S,
                                                 const uint32_t* V, double tan_asvf, bool daytime) {
     PatchSums ps{};
 #pragma unroll
     for (int w = 0; w < SOLWEIG_MASK_WORDS; ++w) {
-        const uint32_t valid = sm.valid[w];
-        const uint32_t sky = S[w] & ~V[w] & valid;
-        const uint32_t veg = S[w] & V[w] & valid;
-        const uint32_t bld = ~S[w] & ~V[w] & valid;
-        if (daytime) {
-            for (uint32_t m = sky; m; m &= m - 1) {
-                const int k = w * 32 + __ffs(m) - 1;
-                ps.lum_sky += sm.lum[k];
-                ps.cw_sky += sm.lum_cw[k];
+        const int kn = min(32, sm.patches - 32 * w);
+#pragma unroll 1
+        for (int i = 0; i < kn; ++i) {
+            const PatchRow& row = sm.row[32 * w + i];
+            const float4 l = *reinterpret_cast<const float4*>(&row.lum);
+            const bool s = (S[w] >> i) & 1u, v = (V[w] >> i) & 1u;
+            const bool sky = s && !v, veg = s && v, bld = !s && !v;
+            if (sky) {
+                ps.lum_sky += l.x;
+                ps.cw_sky += l.y;
             }
-            for (uint32_t m = veg; m; m &= m - 1) {
-                const int k = w * 32 + __ffs(m) - 1;
-                ps.lum_veg += sm.lum[k];
-                ps.cw_veg += sm.lum_cw[k];
+            if (veg) {
+                ps.lum_veg += l.x;
+                ps.cw_veg += l.y;
             }
-        }
-        for (uint32_t m = bld; m; m &= m - 1) {
-            const int k = w * 32 + __ffs(m) - 1;
-            const double x = tan_asvf + sm.x_off[k];
-            const bool sunlit = x < sm.lo[k];
-            const bool shaded = x > sm.hi[k];
-            if (daytime) {
-                if (sunlit) ps.sw_sun += sm.wcos[k];
-                if (shaded) ps.sw_shade += sm.wcos[k];
-            }
-            const bool test = sm.lw_test[k] != 0;
-            const bool lsun = test && sunlit;
-            const bool lshade = !test || shaded;
-            if (lsun) {
-                ps.lw_sun_c += sm.wcos[k];
-                ps.lw_sun_s += sm.wsin[k];
-            }
-            if (lshade) {
-                ps.lw_shade_c += sm.wcos[k];
-                ps.lw_shade_s += sm.wsin[k];
+            const float4 c = *reinterpret_cast<const float4*>(row.card);
+            const float card[4] = {c.x, c.y, c.z, c.w};
+            if (bld) {
+                const double x = tan_asvf + row.x_off;
+                const bool sunlit = x < row.lo, shaded = x > row.hi;
+                const bool test = row.lw_test != 0;
+                const bool lsun = test && sunlit, lshade = !test || shaded;
+                if (sunlit) ps.sw_sun += l.z;
+                if (shaded) ps.sw_shade += l.z;
+                if (lsun) {
+                    ps.lw_sun_c += l.z;
+                    ps.lw_sun_s += l.w;
+                }
+                if (lshade) {
+                    ps.lw_shade_c += l.z;
+                    ps.lw_shade_s += l.w;
+                }
+                if (Cardinal) {
+#pragma unroll
+                    for (int d = 0; d < 4; ++d) {
+                        if (lsun) ps.card_sun[d] += l.z * card[d];
+                        if (lshade) ps.card_shade[d] += l.z * card[d];
+                    }
+                }
             }
             if (Cardinal) {
+                const float side = row.lsky_side;
 #pragma unroll
                 for (int d = 0; d < 4; ++d) {
-                    if (lsun) ps.card_sun[d] += sm.wcos[k] * sm.card[d][k];
-                    if (lshade) ps.card_shade[d] += sm.wcos[k] * sm.card[d][k];
+                    if (sky) ps.card_sky[d] += side * card[d];
+                    if (v) ps.card_veg[d] += l.z * card[d];
+                    if (!sky) ps.card_obst[d] += l.z * card[d];
                 }
             }
         }
-        if (Cardinal) {
-            for (uint32_t m = sky; m; m &= m - 1) {
-                const int k = w * 32 + __ffs(m) - 1;
-#pragma unroll
-                for (int d = 0; d < 4; ++d) ps.card_sky[d] += sm.lsky_side[k] * sm.card[d][k];
-            }
-            const uint32_t vmask = V[w] & valid;
-            for (uint32_t m = vmask; m; m &= m - 1) {
-                const int k = w * 32 + __ffs(m) - 1;
-#pragma unroll
-                for (int d = 0; d < 4; ++d) ps.card_veg[d] += sm.wcos[k] * sm.card[d][k];
-            }
-            const uint32_t obst = ~(S[w] & ~V[w]) & valid;
-            for (uint32_t m = obst; m; m &= m - 1) {
-                const int k = w * 32 + __ffs(m) - 1;
-#pragma unroll
-                for (int d = 0; d < 4; ++d) ps.card_obst[d] += sm.wcos[k] * sm.card[d][k];
-            }
-        }
     }
+    if (!daytime) ps.lum_sky = ps.cw_sky = ps.lum_veg = ps.cw_veg = ps.sw_sun = ps.sw_shade = 0.f;
     return ps;
 }
 
-// UTCI from the hour's collapsed polynomial in D = Tmrt - Ta.
 __device__ __forceinline__ float utci_eval(const double* c, double tmrt, double ta, int valid) {
     if (!valid || tmrt <= -999.0) return -999.0f;
     const double d = tmrt - ta;

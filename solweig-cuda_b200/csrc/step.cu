@@ -292,7 +292,7 @@ __device__ __forceinline__ void radiation_body(
 // One kernel for both branches: the day/night choice is read from the hour
 // record in device memory, so a captured day replays for any forcing.
 template <bool Cardinal>
-__global__ void __launch_bounds__(kStepBX* kStepBY, 3) step_radiation_kernel(
+__global__ void __launch_bounds__(kStepBX* kStepBY, 4) step_radiation_kernel(
     SolweigScene S, const SolweigSkyLayout* __restrict__ L, const SolweigHour* __restrict__ hours,
     int hour, SolweigState st, SolweigOutputs out, const float4* __restrict__ quad,
     const float* __restrict__ gvfp) {
