@@ -148,108 +148,176 @@ __device__ inline CeilingFrame ceiling_frame(const SolweigScene& S, const int2* 
     return f;
 }
 
-__device__ __forceinline__ long long ceiling_pixel(const CeilingFrame& f, int cols, int x, int y) {
-    const int a = f.s_major > 0 ? x : f.nx - 1 - x;
-    const int b = f.s_minor > 0 ? y : f.nb - 1 - y;
-    return f.rows_major ? (long long)a * cols + b : (long long)b * cols + a;
-}
-
-// R(X) = floor(X m / d) while X steps down by one: quotient and remainder
-// carried in 32-bit integers (X m <= rows * cols), no division per step.
+// Position on a sheared line that steps X down by one: y = line + R(X) with
+// R(X) = floor(X m / d), quotient and remainder carried in 32-bit integers
+// (X m <= rows * cols), and the offset of (X, y) in the dilated plane carried
+// along -- no division and no product per step.  I: int, or for huge rasters
+// long long.
+template <typename I>
 struct ShearCursor {
-    int rx, rem;
-    __device__ __forceinline__ ShearCursor(int x, int m, int d) {
-        const int num = x * m;
-        rx = num / d;
-        rem = num - rx * d;
+    int y, rem;
+    I at;            // offset as if y were in the raster
+    I at_x;          // its change as X goes down by one; as y does: -s_minor
+    __device__ __forceinline__ ShearCursor(const CeilingFrame& f, int line, int x) {
+        const int num = x * f.m, r = num / f.d;
+        rem = num - r * f.d;
+        y = line + r;
+        at = (I)(f.s_major > 0 ? x : f.nx - 1 - x) * f.nb + (f.s_minor > 0 ? y : f.nb - 1 - y);
+        at_x = -f.s_major * (I)f.nb;
     }
-    __device__ __forceinline__ void step_down(int m, int d) {  // m <= d
-        rem -= m;
-        if (rem < 0) {
-            rem += d;
-            --rx;
+    __device__ __forceinline__ bool step_down(const CeilingFrame& f) {  // m <= d; true when y went down
+        at += at_x;
+        rem -= f.m;
+        const bool down = rem < 0;
+        if (down) {
+            rem += f.d;
+            --y;
+            at -= f.s_minor;
         }
+        return down;
     }
 };
 
 constexpr int kCeilBatch = 8;  // samples fetched ahead of the dependent max chain
 
-// H dilated by +-W along the minor axis around Y = y at major index a:
-// plane[a * nb + b].  A line whose centre lies up to W outside the raster
-// still sees its in-raster neighbours: the edge pixel's window covers them.
-__device__ __forceinline__ float ceiling_sample(const float* __restrict__ plane, const CeilingFrame& f, int a, int y) {
+// H dilated by +-W along the minor axis around Y = y: plane[at] for y in the
+// raster.  A line whose centre lies up to W outside it still sees its in-raster
+// neighbours: the edge pixel's window covers them.
+template <typename I>
+__device__ __forceinline__ float ceiling_sample(const float* __restrict__ plane, const CeilingFrame& f, I at, int y) {
     if (y < -f.band || y >= f.nb + f.band) return __int_as_float(0xff800000);
     const int yc = min(max(y, 0), f.nb - 1);
-    const int b = f.s_minor > 0 ? yc : f.nb - 1 - yc;
-    return __ldg(&plane[(long long)a * f.nb + b]);
+    return __ldg(&plane[at + (I)(f.s_minor * (yc - y))]);
 }
 
 // One backward scan of [x0, x1) from g over the lane's sheared line; with OUT,
 // writes every pixel of the line: (ceiling, window maximum).  A batch of loads
-// is issued before the dependent chain consumes it.  win[i] holds Hd at
-// x + 1 + i (the samples of the window after x), preloaded at the segment end.
-template <bool OUT>
+// is issued before the dependent chain consumes it, without range tests when the
+// batch surely lies inside the raster.  ahead[j] is the maximum of Hd at
+// x + 1 .. x + 1 + j, so the windows of a batch are running maxima of the batch and
+// of `ahead`.  y goes down with x: the part of the segment before the line enters
+// the raster is all -inf and skipped, and the scan ends when the line has left
+// (both for the whole warp, by its first and last line).
+//
+// The lanes' lines are neighbours along Y.  Where the rows of the raster run along
+// X, a lane's 8-byte stores would each touch a sector of their own, four times
+// over: a batch goes through shared memory (`stage`, per warp) and is written row
+// by row, 64 bytes at a time.  That was the bound: planes of a 2000^2 day 0.58 ->
+// 0.31 ms, of 153 patches at 512 x 448 0.37 -> 0.26 ms; the cheaper steps alone
+// gave 0.57 and 0.35.  Now it is the latency of the segments' two passes.
+constexpr int kCeilStagePitch = 36;  // float2; 8 banks from one step to the next
+template <bool OUT, typename I>
 __device__ __forceinline__ float ceiling_run(const float* __restrict__ plane, const CeilingFrame& f, int cols,
-                                             int line, int x0, int x1, float g, float2* __restrict__ out) {
+                                             int line, int x0, int x1, float g, float2* __restrict__ out,
+                                             float2 (*stage)[kCeilStagePitch]) {
+    static_assert(kCeilBatch == kCeilSkip, "a batch is a window");
     const float ninf = __int_as_float(0xff800000);
-    float win[kCeilSkip - 1];
+    if (x0 >= x1) return g;
+    const int lane = threadIdx.x;  // the block's rows are warps
+    const int top = f.nb + f.band - (line - lane);  // the warp is in reach of the raster for R(x) < top
+    if (top <= 0) return g;
+    if (f.m > 0) x1 = (int)min((long long)x1, ((long long)top * f.d + f.m - 1) / f.m);
+    if (x0 >= x1) return g;
+    float ahead[kCeilSkip - 1];
 #pragma unroll
     for (int i = 0; i < kCeilSkip - 1; ++i) {
-        win[i] = ninf;
+        ahead[i] = i > 0 ? ahead[i - 1] : ninf;
         if (OUT && x1 + i < f.nx) {
-            const int xx = x1 + i;
-            const int a = f.s_major > 0 ? xx : f.nx - 1 - xx;
-            win[i] = ceiling_sample(plane, f, a, line + (int)(((long long)xx * f.m) / f.d));
+            const int xx = x1 + i, y = line + (int)(((long long)xx * f.m) / f.d);
+            const int a = f.s_major > 0 ? xx : f.nx - 1 - xx, b = f.s_minor > 0 ? y : f.nb - 1 - y;
+            ahead[i] = fmaxf(ahead[i], ceiling_sample<I>(plane, f, (I)a * f.nb + b, y));
         }
     }
-    auto emit = [&](int x, int y, float v) {
-        float m = v;
-#pragma unroll
-        for (int i = 0; i < kCeilSkip - 1; ++i) m = fmaxf(m, win[i]);
-#pragma unroll
-        for (int i = kCeilSkip - 2; i > 0; --i) win[i] = win[i - 1];
-        win[0] = v;
-        if (OUT && y >= 0 && y < f.nb) out[ceiling_pixel(f, cols, x, y)] = make_float2(g, m);
-    };
-    ShearCursor cur(max(x1 - 1, 0), f.m, f.d);
     int x = x1 - 1;
+    ShearCursor<I> cur(f, line, x);
+    // the raster offset of the pixel: of a column-major ray another one than the plane's
+    const int a1 = f.s_major > 0 ? x : f.nx - 1 - x, b1 = f.s_minor > 0 ? cur.y : f.nb - 1 - cur.y;
+    I px = f.rows_major ? (I)a1 * cols + b1 : (I)b1 * cols + a1;
+    const I px_x = f.rows_major ? -f.s_major * (I)cols : (I)-f.s_major;
+    const I px_y = f.rows_major ? (I)-f.s_minor : -f.s_minor * (I)cols;
     for (; x - (kCeilBatch - 1) >= x0; x -= kCeilBatch) {
+        if (cur.y + (kCeilLanes - 1 - lane) < -f.band) return g;
         float v[kCeilBatch];
-        int y[kCeilBatch];
+        int y = cur.y;
+        uint32_t down = 0u;  // steps after which y is one lower
+        const bool inside = y < f.nb && y >= kCeilBatch;
+        if (inside) {
 #pragma unroll
-        for (int u = 0; u < kCeilBatch; ++u) {
-            y[u] = line + cur.rx;
-            const int a = f.s_major > 0 ? x - u : f.nx - 1 - (x - u);
-            v[u] = ceiling_sample(plane, f, a, y[u]);
-            cur.step_down(f.m, f.d);
+            for (int u = 0; u < kCeilBatch; ++u) {
+                v[u] = __ldg(&plane[cur.at]);
+                if (cur.step_down(f)) down |= 1u << u;
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < kCeilBatch; ++u) {
+                v[u] = ceiling_sample<I>(plane, f, cur.at, cur.y);
+                if (cur.step_down(f)) down |= 1u << u;
+            }
         }
+        float window = ninf;
 #pragma unroll
         for (int u = 0; u < kCeilBatch; ++u) {
             g = fmaxf(v[u], __fsub_ru(g, f.delta));
-            if (OUT) emit(x - u, y[u], v[u]);
+            if (OUT) {
+                window = fmaxf(window, v[u]);
+                const float2 cell = make_float2(g, u + 1 < kCeilBatch ? fmaxf(window, ahead[kCeilSkip - 2 - u]) : window);
+                if (!f.rows_major) stage[u][lane] = cell;
+                else if (inside || (y >= 0 && y < f.nb)) out[px] = cell;
+                px += px_x;
+                if ((down >> u) & 1u) {
+                    px += px_y;
+                    --y;
+                }
+            }
+        }
+        if (OUT && !f.rows_major) {
+            // step u of row i (from the lowest) comes from the lane `back` rows below it
+            __syncwarp();
+            const int u = lane & (kCeilBatch - 1), fell = __popc(down & ((1u << (kCeilBatch - 1)) - 1u));
+            const int back = fell - __popc(down & ((1u << u) - 1u));
+            const int ylow = cur.y + (int)((down >> (kCeilBatch - 1)) & 1u) - lane;  // of lane 0 at the last step
+            const int xu = x - u, a = f.s_major > 0 ? xu : f.nx - 1 - xu;
+            for (int i = lane / kCeilBatch; i < kCeilLanes + fell; i += kCeilLanes / kCeilBatch) {
+                const int from = i - back, yi = ylow + i;
+                if (from < 0 || from >= kCeilLanes || yi < 0 || yi >= f.nb) continue;
+                out[(I)(f.s_minor > 0 ? yi : f.nb - 1 - yi) * cols + a] = stage[u][from];
+            }
+            __syncwarp();
+        }
+        if (OUT) {
+            ahead[0] = v[kCeilBatch - 1];
+#pragma unroll
+            for (int j = 1; j < kCeilSkip - 1; ++j) ahead[j] = fmaxf(ahead[j - 1], v[kCeilBatch - 1 - j]);
         }
     }
+#pragma unroll 1
     for (; x >= x0; --x) {
-        const int yy = line + cur.rx;
-        const int a = f.s_major > 0 ? x : f.nx - 1 - x;
-        const float v = ceiling_sample(plane, f, a, yy);
+        const float v = ceiling_sample<I>(plane, f, cur.at, cur.y);
         g = fmaxf(v, __fsub_ru(g, f.delta));
-        if (OUT) emit(x, yy, v);
-        cur.step_down(f.m, f.d);
+        if (OUT) {
+            if (cur.y >= 0 && cur.y < f.nb) out[px] = make_float2(g, fmaxf(v, ahead[kCeilSkip - 2]));
+#pragma unroll
+            for (int j = kCeilSkip - 2; j > 0; --j) ahead[j] = fmaxf(v, ahead[j - 1]);
+            ahead[0] = v;
+            px += px_x;
+        }
+        if (cur.step_down(f)) px += px_y;
     }
     return g;
 }
 
 // Both phases for one block of 32 sheared lines (see the file comment).
+template <typename I>
 __device__ __forceinline__ void ceiling_scan(const float* __restrict__ plane, const CeilingFrame& f, int cols,
-                                             int line0, float (*s_seg)[kCeilLanes], float2* __restrict__ out) {
+                                             int line0, float (*s_seg)[kCeilLanes], float2* __restrict__ out,
+                                             float2 (*stage)[kCeilStagePitch]) {
     const int seg = (f.nx + kCeilWarps - 1) / kCeilWarps;
     const int w = threadIdx.y;
     const int x0 = min(f.nx, w * seg), x1 = min(f.nx, x0 + seg);
     const int line = line0 + threadIdx.x;
     const float ninf = __int_as_float(0xff800000);
     // phase 1: segment maxima from -inf
-    s_seg[w][threadIdx.x] = ceiling_run<false>(plane, f, cols, line, x0, x1, ninf, nullptr);
+    s_seg[w][threadIdx.x] = ceiling_run<false, I>(plane, f, cols, line, x0, x1, ninf, nullptr, nullptr);
     __syncthreads();
     // phase 2: carry of the later segments, then the rescan that writes
     float carry = ninf;
@@ -257,7 +325,7 @@ __device__ __forceinline__ void ceiling_scan(const float* __restrict__ plane, co
         const int s0 = min(f.nx, s * seg), s1 = min(f.nx, s0 + seg);
         carry = fmaxf(s_seg[s][threadIdx.x], __fsub_ru(carry, __fmul_rd((float)(s1 - s0), f.delta)));
     }
-    ceiling_run<true>(plane, f, cols, line, x0, x1, carry, out);
+    ceiling_run<true, I>(plane, f, cols, line, x0, x1, carry, out, stage);
 }
 
 // The four dilated planes of H (see the file comment), each rows x cols floats:
@@ -313,6 +381,7 @@ __device__ __forceinline__ void ray_ceiling_block(const SolweigScene& S, const i
                                                   const double* __restrict__ dz, int K,
                                                   const float* __restrict__ dil, float2* __restrict__ out,
                                                   float (*s_seg)[kCeilLanes]) {
+    __shared__ float2 s_stage[kCeilWarps][kCeilBatch][kCeilStagePitch];
     if (K < kCeilMinSteps) return;
     const long long n = (long long)S.rows * S.cols;
     const CeilingFrame f = ceiling_frame(S, ray, dz, K);
@@ -328,13 +397,17 @@ __device__ __forceinline__ void ray_ceiling_block(const SolweigScene& S, const i
     // lane l owns sheared line N = line_first + l - R(nx - 1)
     const int line0 = line_first - (f.lines - f.nb);
     const float* plane = dil + (long long)((f.rows_major ? 0 : 2) + (f.band - 1)) * n;
-    ceiling_scan(plane, f, S.cols, line0, s_seg, out);
+    // offsets stay within twice (lines + nx) times a side: 32 bits unless the raster is huge
+    if ((long long)(f.nb + f.nx) * (f.lines + f.nx) < (1ll << 29))
+        ceiling_scan<int>(plane, f, S.cols, line0, s_seg, out, s_stage[threadIdx.y]);
+    else
+        ceiling_scan<long long>(plane, f, S.cols, line0, s_seg, out, s_stage[threadIdx.y]);
 }
 
 // grid (ceil((rows + cols) / 32), 1, hours), block (32, kCeilWarps): the ceiling plane
 // of every daytime hour whose ray has at least kCeilMinSteps steps, from the
 // dilated planes of ceiling_dilate_kernel.
-static __global__ void __launch_bounds__(kCeilLanes * kCeilWarps) day_ray_ceiling_kernel(
+static __global__ void __launch_bounds__(kCeilLanes * kCeilWarps, 2) day_ray_ceiling_kernel(
     SolweigScene S, const SolweigHour* __restrict__ hours, const float* __restrict__ dil,
     float2* __restrict__ ceiling) {
     __shared__ float s_seg[kCeilWarps][kCeilLanes];
@@ -346,7 +419,7 @@ static __global__ void __launch_bounds__(kCeilLanes * kCeilWarps) day_ray_ceilin
 
 // The same for sky-patch rays: grid.z = patch - patch0 of a group of count
 // patches; tables [patch][capacity] with lengths[patch] steps.
-static __global__ void __launch_bounds__(kCeilLanes * kCeilWarps) patch_ray_ceiling_kernel(
+static __global__ void __launch_bounds__(kCeilLanes * kCeilWarps, 2) patch_ray_ceiling_kernel(
     SolweigScene S, const int2* __restrict__ rays, const double* __restrict__ dz,
     const int32_t* __restrict__ lengths, int capacity, int patch0, int count, const float* __restrict__ dil,
     float2* __restrict__ ceiling) {
