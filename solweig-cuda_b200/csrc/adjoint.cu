@@ -727,10 +727,7 @@ __global__ void __launch_bounds__(256) gvf_transpose_words_kernel(SolweigScene S
     double v[kWkHours] = {0.0, 0.0, 0.0, 0.0};
     if (p < n) {
         const int r = (int)(p / S.cols), c = (int)(p - (long long)r * S.cols);
-        const int tiles_x = (S.cols + kWkTile - 1) / kWkTile;
-        const int ty = r % kWkTile, tx = c % kWkTile;  // the inverse of walk_pixel
-        const int t = ((ty >> 2) * 4 + (tx >> 3)) * 32 + (ty & 3) * 8 + (tx & 7);
-        const uint32_t* walk = walks + (long long)((r / kWkTile) * tiles_x + c / kWkTile) * kWkTileWords + t;
+        const uint32_t* walk = walks + walk_word_at(r, c, S.cols);
         const uint32_t* code = codes + blockIdx.y * n + p;
         uint32_t* out = words + (long long)blockIdx.y * 2 * kTrGroups * n + p;
         int wall_steps[kWkHours] = {0, 0, 0, 0};

@@ -26,17 +26,13 @@
 // staged tile in the kernel's parameters, read through the uniform datapath.
 #pragma once
 #include "gvf_fields.cuh"
+#include "gvf_words.cuh"
 
 namespace solweig {
 
 namespace {
 
-constexpr int kWkTile = 32;                 // pixels of a tile side
-constexpr int kWkMaxSteps = 22;             // longest walk (halo 21)
-constexpr int kWkPixels = kWkTile * kWkTile;
 constexpr int kWkThreads = 512;             // two pixels each, one after the other
-constexpr int kWkDirs = SOLWEIG_GVF_DIRECTIONS;
-constexpr int kWkTileWords = kWkDirs * kWkTile * kWkTile;
 constexpr int kWkHours = 4;                 // hours per pass
 constexpr int kWkValues = 6;                // distinct samples of an hour that can be counted
 constexpr int kWkTileValues = 15;           // ... that one tile can number (4-bit codes, 15: not ground)
@@ -45,26 +41,6 @@ constexpr int kWkMaxWidth = kWkTile + 2 * (kWkMaxSteps - 1);  // staged tile sid
 
 // Every second 5-bit field of a count word, in 10 bits each (18 walks fit).
 constexpr uint32_t kWkFields = 0x01f07c1fu;
-
-// Walk word: wall pixels met (bit m: step m, before the walk ends), samples
-// read (0 off the ground), frozen tail (the walk left the raster and repeats
-// its last sample), own wall faces away from the direction.
-constexpr uint32_t kWkWallBits = (1u << kWkMaxSteps) - 1u;
-constexpr int kWkLimShift = 22;
-constexpr uint32_t kWkFrozen = 1u << 27, kWkFace = 1u << 28;
-
-__host__ __device__ __forceinline__ long long walk_words(int rows, int cols) {
-    return (long long)((rows + kWkTile - 1) / kWkTile) * ((cols + kWkTile - 1) / kWkTile) * kWkTileWords;
-}
-
-// Tile pixel t: each warp takes an 8 x 4 (columns x rows) piece, as
-// walk lengths of nearby pixels are alike in both directions.  The walk words
-// of a direction are stored in this order.
-__device__ __forceinline__ void walk_pixel(int t, int& ty, int& tx) {
-    const int w = t >> 5, l = t & 31;
-    tx = (w & 3) * 8 + (l & 7);
-    ty = (w >> 2) * 4 + (l >> 3);
-}
 
 // ---------------------------------------------------------- packed float32
 

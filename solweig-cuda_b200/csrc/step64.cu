@@ -27,6 +27,7 @@
 // compiles its kernels, src/runtime.py:11), so no multiply-add is contracted.
 // UTCI is evaluated from the float32-rounded Tmrt and air temperature, as
 // utci_calculator casts its inputs (src/utci.py:8-12).
+#include "gvf_words.cuh"
 #include "hour.cuh"
 #include "radiation.cuh"
 
@@ -40,15 +41,25 @@ enum Scratch64 : int {
     kS64Shadow = 2,    // sh - (1 - vegsh)(1 - psi)
     kS64LupFirst = 3,  // Lup excess before the override (first search direction)
     kS64Bits = 4,      // one byte per pixel: 1 = sunlit wall
-    kS64Gvf = 5,       // 15 planes: Lup, albedo, albedo without shadow x (all, E, S, W, N)
+    kS64Gvf = 5,       // 15 planes: Lup, albedo, albedo without shadow x (all, E, S, W, N); the last
+                       // five of a launch's first daytime hour serve all its hours
 };
 
 struct GvfOffsets64 {
     int2 offs[SOLWEIG_GVF_DIRECTIONS * SOLWEIG_GVF_MAX_STEPS];
+    long long ahead[SOLWEIG_GVF_DIRECTIONS * SOLWEIG_GVF_MAX_STEPS];  // pixels from the walking one
 };
 
 __device__ __forceinline__ double* hour_scratch(double* sc, long long n) {
     return sc + (long long)blockIdx.z * SOLWEIG_SCRATCH64_PLANES * n;
+}
+
+// First daytime hour of a launch, whose scratch holds the albedo-without-shadow
+// planes of all of them.
+__device__ __forceinline__ int first_day_hour(const SolweigHour* __restrict__ hours) {
+    int z = 0;
+    while (!hours[z].daytime) ++z;
+    return z;
 }
 
 __global__ void __launch_bounds__(kStep64BX* kStep64BY) step64_fields_kernel(
@@ -100,25 +111,26 @@ __global__ void __launch_bounds__(kStep64BX* kStep64BY) step64_fields_kernel(
     reinterpret_cast<uint8_t*>(sc + kS64Bits * n)[p] = sunwall;
 }
 
-// Ground view factors of the daytime hours into the 15 scratch GVF planes (the
+// Ground view factors of the daytime hours into the scratch GVF planes (the
 // step reads no gvfSum / gvfNorm, so the shadow sums are not kept).  A walk
 // adds its samples in order up to the first building; past it (or past the
 // raster's edge, where the last sample repeats) every step adds the same
-// terms, which come as one product.  With the scene's walk lengths (`hits`)
-// the ground bits are not read at all.  What bounds it: the latency of the
-// samples' loads through L1 and the FP64 pipe; 64 registers (8 blocks per SM)
-// against 128: 25.3 against 26.3 ms per 1000^2 day.
-__global__ void __launch_bounds__(kStep64BX* kStep64BY, 8) step64_gvf_kernel(
-    SolweigScene S, const SolweigHour* __restrict__ hours, const __grid_constant__ GvfOffsets64 tab, int first,
-    int second, bool hits, double* __restrict__ scratch) {
-    const SolweigHour& h = hours[blockIdx.z];
-    if (!h.daytime) return;
-    const int c = blockIdx.x * kStep64BX + threadIdx.x;
-    const int r = blockIdx.y * kStep64BY + threadIdx.y;
-    if (r >= S.rows || c >= S.cols) return;
+// terms, which come as one product.  WALK: the scene's walk words (kWalkWords)
+// give the walk's length and the wall pixels it meets, so a step only reads its
+// sample; its walk lengths (kWalkHits) leave a sunlit-wall byte per step; else
+// the ground bits are read first.  The albedo without shadow is the same in
+// every hour of a launch: NOSH (the first daytime hour) sums its five planes.
+// What bounds it: the latency of the samples' loads through L1 and the FP64
+// pipe; 64 registers (8 blocks per SM).  17 hours of 300 x 280 pixels: 1.13 ->
+// 0.68 ms against lengths, a byte and an albedo per step and hour (5 or 6 blocks
+// per SM: 0.78, 0.76 against 0.75 before the offsets came ready).
+enum Walk64 { kWalkGround, kWalkHits, kWalkWords };
+
+template <int WALK, bool NOSH>
+__device__ __forceinline__ void gvf64_pixel(const SolweigScene& S, const SolweigHour& h, const GvfOffsets64& tab,
+                                            int first, int second, int r, int c, double* __restrict__ sc) {
     const long long n = (long long)S.rows * S.cols;
     const long long p = (long long)r * S.cols + c;
-    double* sc = hour_scratch(scratch, n);
     const double2* sample = reinterpret_cast<const double2*>(sc + kS64Sample * n) + p;
     const double* lup1p = sc + kS64LupFirst * n + p;
     const uint8_t* sunp = reinterpret_cast<const uint8_t*>(sc + kS64Bits * n) + p;
@@ -137,13 +149,21 @@ __global__ void __launch_bounds__(kStep64BX* kStep64BY, 8) step64_gvf_kernel(
     const double by_second = 1.0 / dsecond, by_second1 = 1.0 / (dsecond + 1.0);
     double lup[5] = {0, 0, 0, 0, 0}, alb[5] = {0, 0, 0, 0, 0}, nosh[5] = {0, 0, 0, 0, 0};
     uint32_t code = 0u;
+    const uint32_t* words = WALK == kWalkWords ? S.gvf_walks + walk_word_at(r, c, S.cols) : nullptr;
     for (int j = 0; j < SOLWEIG_GVF_DIRECTIONS; ++j) {
         const int2* o = tab.offs + j * second;
+        const long long* ahead = tab.ahead + j * second;
         // lim samples are read; hit = first step with a building (second: none)
         int lim, hit;
-        if (!own_ground) {
+        uint32_t walls = 0u;
+        if (WALK == kWalkWords) {
+            const uint32_t word = __ldg(words + j * kWkPixels);
+            lim = min((int)((word >> kWkLimShift) & 31u), second);
+            hit = word & kWkFrozen ? second : lim;
+            walls = word & kWkWallBits;
+        } else if (!own_ground) {
             lim = hit = 0;
-        } else if (hits) {
+        } else if (WALK == kWalkHits) {
             if (j % 5 == 0) code = S.gvf_hits[(long long)(j / 5) * n + p];
             lim = min((int)(code & 31u), second);
             hit = code & 32u ? second : lim;
@@ -156,7 +176,7 @@ __global__ void __launch_bounds__(kStep64BX* kStep64BY, 8) step64_gvf_kernel(
                     if (k == 0) hit = 0;  // nothing seen: no ground
                     break;
                 }
-                if (!(__ldg(flagp + (long long)o[k].x * S.cols + o[k].y) & 1)) {
+                if (!(__ldg(flagp + ahead[k]) & 1)) {
                     lim = hit = k;
                     break;
                 }
@@ -166,15 +186,28 @@ __global__ void __launch_bounds__(kStep64BX* kStep64BY, 8) step64_gvf_kernel(
         double2 t = make_double2(0.0, 0.0);
         double t_alb = 0.0;
         int sun = second;  // first step showing a sunlit wall
+        if (WALK == kWalkWords) {
+            for (; walls; walls &= walls - 1u) {
+                const int k = __ffs((int)walls) - 1;
+                if (sunp[ahead[k]]) {
+                    sun = k;
+                    break;
+                }
+            }
+        }
         for (int k = 0; k < lim; ++k) {
-            const long long q = (long long)o[k].x * S.cols + o[k].y;
+            const long long q = ahead[k];
             t = sample[q];
-            if (j == 0 && S.has_water) t.x = lup1p[q];
-            t_alb = (double)__ldg(albp + q);
-            if (sunp[q] && sun == second) sun = k;
+            if (WALK != kWalkWords) {
+                if (j == 0 && S.has_water) t.x = lup1p[q];
+                if (sunp[q] && sun == second) sun = k;
+            }
             s_lup += t.x;
             s_albsh += t.y;
-            s_alb += t_alb;
+            if (NOSH) {
+                t_alb = (double)__ldg(albp + q);
+                s_alb += t_alb;
+            }
             if (k + 1 <= first) {
                 n_lup = s_lup; n_albsh = s_albsh; n_alb = s_alb;
             }
@@ -200,18 +233,21 @@ __global__ void __launch_bounds__(kStep64BX* kStep64BY, 8) step64_gvf_kernel(
         const double lup2 = sun_far ? (w_sun * lwall + s_lup) * by_second1 : s_lup * by_second;
         const double alb1 = sun_near ? (n_sun_near * albedo_b + n_albsh) * by_first1 : n_albsh * by_first;
         const double alb2 = sun_far ? (w_sun * albedo_b + s_albsh) * by_second1 : s_albsh * by_second;
-        const double nosh1 = wall_near ? (n_wall_near * albedo_b + n_alb) * by_first1 : n_alb * by_first;
-        const double nosh2 = wall_far ? (n_wall * albedo_b + s_alb) * by_second : s_alb * by_second;
         const double d_lup = (lup1 * 0.5 + lup2 * 0.4) / 0.9 + own_lup * ground;
         const double d_alb = (alb1 * 0.5 + alb2 * 0.4) / 0.9 + own_alb * ground * own_sh;
-        const double d_nosh = ((nosh1 * 0.5 + nosh2 * 0.4) / 0.9) * own_b + own_alb * ground;
+        double d_nosh = 0.0;
+        if (NOSH) {
+            const double nosh1 = wall_near ? (n_wall_near * albedo_b + n_alb) * by_first1 : n_alb * by_first;
+            const double nosh2 = wall_far ? (n_wall * albedo_b + s_alb) * by_second : s_alb * by_second;
+            d_nosh = ((nosh1 * 0.5 + nosh2 * 0.4) / 0.9) * own_b + own_alb * ground;
+        }
         const unsigned groups = gvf_direction_groups(j);
 #pragma unroll
         for (int g = 0; g < 5; ++g)
             if (groups & (1u << g)) {
                 lup[g] += d_lup;
                 alb[g] += d_alb;
-                nosh[g] += d_nosh;
+                if (NOSH) nosh[g] += d_nosh;
             }
     }
     const double ambient = kSBC * (double)S.emis[p] * pow4(ta + 273.15);
@@ -221,8 +257,22 @@ __global__ void __launch_bounds__(kStep64BX* kStep64BY, 8) step64_gvf_kernel(
         const double div = g == 0 ? 18.0 : 9.0;
         gvf[(long long)g * n + p] = lup[g] / div + ambient;
         gvf[(long long)(5 + g) * n + p] = alb[g] / div;
-        gvf[(long long)(10 + g) * n + p] = nosh[g] / div;
+        if (NOSH) gvf[(long long)(10 + g) * n + p] = nosh[g] / div;
     }
+}
+
+template <int WALK>
+__global__ void __launch_bounds__(kStep64BX* kStep64BY, 8) step64_gvf_kernel(
+    SolweigScene S, const SolweigHour* __restrict__ hours, const __grid_constant__ GvfOffsets64 tab, int first,
+    int second, double* __restrict__ scratch) {
+    const SolweigHour& h = hours[blockIdx.z];
+    if (!h.daytime) return;
+    const int c = blockIdx.x * kStep64BX + threadIdx.x;
+    const int r = blockIdx.y * kStep64BY + threadIdx.y;
+    if (r >= S.rows || c >= S.cols) return;
+    double* sc = hour_scratch(scratch, (long long)S.rows * S.cols);
+    if (first_day_hour(hours) == (int)blockIdx.z) gvf64_pixel<WALK, true>(S, h, tab, first, second, r, c, sc);
+    else gvf64_pixel<WALK, false>(S, h, tab, first, second, r, c, sc);
 }
 
 // Per-patch and per-band values of one hour (float64), staged in shared memory.
@@ -424,9 +474,11 @@ __global__ void __launch_bounds__(kStep64BX* kStep64BY, 6) step64_radiation_kern
         const double reflected = albedo_b * (1.0 - svb) * (h.rad_g * (1.0 - fsh) + h.rad_d * fsh);
         const double base = h.rad_d * svb + reflected;
         const double* gvf = sc + kS64Gvf * n;
+        const double* nosh =
+            scratch + ((long long)first_day_hour(hours) * SOLWEIG_SCRATCH64_PLANES + kS64Gvf + 10) * n;
 #pragma unroll
         for (int d = 0; d < 5; ++d) {
-            kup[d] = gvf[(long long)(5 + d) * n + p] * h.rad_i * h.sin_alt + base * gvf[(long long)(10 + d) * n + p];
+            kup[d] = gvf[(long long)(5 + d) * n + p] * h.rad_i * h.sin_alt + base * nosh[(long long)d * n + p];
             lup[d] = gvf[(long long)d * n + p];
         }
         d_rad = lum * h.rad_d;
@@ -547,17 +599,22 @@ extern "C" int solweig_step64_hours(const SolweigScene* scene, const double* svf
                       "solweig_step64: GVF steps first=%d second=%d", first_steps, second_steps);
     SOLWEIG_CHECK_ARG(((uintptr_t)scratch & 15) == 0, "solweig_step64: scratch not 16-byte aligned");
     GvfOffsets64 tab;
-    for (int i = 0; i < SOLWEIG_GVF_DIRECTIONS * second_steps; ++i)
+    for (int i = 0; i < SOLWEIG_GVF_DIRECTIONS * second_steps; ++i) {
         tab.offs[i] = make_int2(gvf_dxdy[2 * i], gvf_dxdy[2 * i + 1]);
+        tab.ahead[i] = (long long)gvf_dxdy[2 * i] * S.cols + gvf_dxdy[2 * i + 1];
+    }
     // the scene's walk lengths are those of these steps (they come with its walk words)
     const bool hits = S.gvf_hits && first_steps == 1 && second_steps <= 22 && !S.has_water;
+    const bool words = hits && S.gvf_walks && ((uintptr_t)S.gvf_walks & 3) == 0;
     cudaStream_t st = as_stream(stream);
     const SolweigHour* hr = hours + hour;
     dim3 block(kStep64BX, kStep64BY);
     dim3 grid(blocks_for(S.cols, kStep64BX), blocks_for(S.rows, kStep64BY), count);
     step64_fields_kernel<<<grid, block, 0, st>>>(S, hr, scratch);
     SOLWEIG_CHECK_LAUNCH("step64_fields_kernel");
-    step64_gvf_kernel<<<grid, block, 0, st>>>(S, hr, tab, first_steps, second_steps, hits, scratch);
+    if (words) step64_gvf_kernel<kWalkWords><<<grid, block, 0, st>>>(S, hr, tab, first_steps, second_steps, scratch);
+    else if (hits) step64_gvf_kernel<kWalkHits><<<grid, block, 0, st>>>(S, hr, tab, first_steps, second_steps, scratch);
+    else step64_gvf_kernel<kWalkGround><<<grid, block, 0, st>>>(S, hr, tab, first_steps, second_steps, scratch);
     SOLWEIG_CHECK_LAUNCH("step64_gvf_kernel");
     step64_wave_kernel<<<blocks_for((long long)S.rows * S.cols, 128), 128, 0, st>>>(S, hr, count, *state, *out,
                                                                                    hour_stride, scratch);
