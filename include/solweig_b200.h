@@ -240,9 +240,10 @@ int solweig_svf_ex(const double* dsm, const double* vegdem, const double* vegdem
  * solweig_svf_work_bytes(rows, cols) bytes (no counterpart in the reference):
  * per word of 32 patches, upper bounds of the heights ahead along each patch
  * ray let the visibility walks stop early, per-row / per-column exit steps
- * drop their bounds checks, and 16-byte step records (linear offset, dz)
- * replace the offset and dz tables in the walks when capacity <= max(rows,
- * cols) + 2; the masks and planes are identical. */
+ * drop their bounds checks, and with geo32 8-byte step records (linear offset,
+ * height rounded down) and a plane of max(dsm, vegdem, vegdem2) replace most
+ * samples when capacity <= max(rows, cols) + 2; the masks and planes are
+ * identical. */
 int64_t solweig_svf_work_bytes(int rows, int cols);
 /* The patches' visibility rays (src/svf.py:47-75) built on the device: host
  * arrays [patches] of the azimuth's sine, cosine and tangent, of

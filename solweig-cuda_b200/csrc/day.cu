@@ -74,13 +74,15 @@ namespace {
 int gvf_scene_walks(const char* name, const SolweigScene* scene, const int32_t* gvf_dxdy, int second, uint32_t* hits,
                     uint32_t* walks, float* nosh, void* stream) {
     SOLWEIG_CHECK_ARG(!scene->has_water, "%s: scenes with water walk per hour", name);
-    SOLWEIG_CHECK_ARG(scene->rows > 0 && scene->cols > 0 && scene->flags && scene->alb && scene->walls &&
-                          scene->gvf_face,
+    // the words need the walls and the faces, the lengths alone don't
+    SOLWEIG_CHECK_ARG(scene->rows > 0 && scene->cols > 0 && scene->flags && scene->alb &&
+                          (!walks || (scene->walls && scene->gvf_face)),
                       "%s: bad scene", name);
     for (int j = 0; j < SOLWEIG_GVF_DIRECTIONS; ++j)
         for (int m = 0; m < second; ++m) {
             const int32_t* o = gvf_dxdy + 2 * (j * second + m);
-            SOLWEIG_CHECK_ARG(o[0] >= -m && o[0] <= m && o[1] >= -m && o[1] <= m,
+            const int reach = walks ? m : second - 1;  // words: a walk starts at its pixel; lengths: the staged halo
+            SOLWEIG_CHECK_ARG(o[0] >= -reach && o[0] <= reach && o[1] >= -reach && o[1] <= reach,
                               "%s: GVF offset (%d, %d) at step %d", name, o[0], o[1], m);
         }
     return launch_gvf_walks(*scene, gvf_dxdy, second, hits, walks, nosh, as_stream(stream));

@@ -531,7 +531,7 @@ __global__ void __launch_bounds__(kWkPixels, 1) gvf_walks_kernel(SolweigScene S,
         const int rr = row0 + i / kWkMaxWidth, cc = col0 + i % kWkMaxWidth;
         const bool in = in_raster(rr, cc, S.rows, S.cols);
         const long long q = in ? (long long)rr * S.cols + cc : 0;
-        bits[i] = in ? (uint8_t)((S.flags[q] & 1) | (S.walls[q] > 0.0 ? 2 : 0)) : (uint8_t)4;
+        bits[i] = in ? (uint8_t)((S.flags[q] & 1) | (S.walls && S.walls[q] > 0.0 ? 2 : 0)) : (uint8_t)4;
         albs[i] = in ? S.alb[q] : 0.f;
     }
     __syncthreads();
@@ -542,7 +542,7 @@ __global__ void __launch_bounds__(kWkPixels, 1) gvf_walks_kernel(SolweigScene S,
     const long long p = valid ? (long long)r * S.cols + c : 0;
     const int own = (ty + halo) * kWkMaxWidth + tx + halo;
     const bool own_ground = valid && (bits[own] & 1u);
-    const uint32_t face = valid ? S.gvf_face[p] : 0u;
+    const uint32_t face = valid && S.gvf_face ? S.gvf_face[p] : 0u;
     const long long tile = (long long)(tr * gridDim.x + tc) * kWkTileWords;
     constexpr float albedo_b = 0.2f;
     const float inv_second = 1.f / (float)second;
@@ -565,9 +565,9 @@ __global__ void __launch_bounds__(kWkPixels, 1) gvf_walks_kernel(SolweigScene S,
                 if (b & 2u) walls |= 1u << m;
                 s_alb += albs[at];
             }
-            n_alb = albs[own + delta[0]];
+            n_alb = m > 0 ? albs[own + delta[0]] : 0.f;
             hit = lim = m;
-            if (b & 4u) {  // frozen tail: step m (> 0: step 0 is the pixel) and the rest repeat step m - 1
+            if ((b & 4u) && m > 0) {  // frozen tail: step m and the rest repeat step m - 1
                 hit = second;
                 const float al = albs[own + delta[m - 1]];
                 s_alb += al;

@@ -103,3 +103,39 @@ def test_walks_that_do_not_start_at_their_pixel_take_the_general_path(hours):
         assert abs(float((grad * v).sum()) - fd) <= 1e-3 * abs(fd)
     finally:
         table[:] = saved
+
+
+def test_walk_lengths_alone_need_no_walls_and_any_offset_of_the_halo():
+    """solweig_gvf_statics without walls and faces, and with a table whose walks
+    start one step out: lengths as a loop over the steps finds them."""
+    import ctypes
+    import torch
+    from solweig_cuda_b200 import _lib
+    from solweig_cuda_b200.engine import device_ptr, stream_handle
+    scene, _, _, _ = _case(37, 41, 24)
+    rows, cols = scene.shape
+    table = scene.gvf_dxdy_host.reshape(18, 22, 2).copy()
+    table[:, 0] = table[:, 1]
+    struct = _lib.SolweigScene.from_buffer_copy(scene.struct)
+    struct.walls = struct.gvf_face = None
+    hits = torch.empty((4, rows, cols), dtype=torch.int32, device="cuda")
+    nosh = torch.empty((rows, cols), dtype=torch.float32, device="cuda")
+    _lib.check(_lib.lib().solweig_gvf_statics(ctypes.byref(struct), table.ctypes.data_as(ctypes.c_void_p), 1, 22,
+                                              device_ptr(hits), device_ptr(nosh), stream_handle()),
+               "solweig_gvf_statics")
+    got = hits.cpu().numpy()
+    ground = scene.flags.cpu().numpy().reshape(rows, cols) & 1
+    rr, cc = np.mgrid[:rows, :cols]
+    for j in range(18):
+        lim, frozen = np.zeros((rows, cols), int), np.zeros((rows, cols), bool)
+        going = ground.astype(bool).copy()
+        for m in range(22):
+            r, c = rr + table[j, m, 0], cc + table[j, m, 1]
+            inside = (r >= 0) & (r < rows) & (c >= 0) & (c < cols)
+            free = inside & (ground[np.clip(r, 0, rows - 1), np.clip(c, 0, cols - 1)] == 1)
+            frozen |= going & ~inside & (m > 0)
+            going &= free
+            lim += going
+        code = (got[j // 5] >> (6 * (j % 5))) & 63
+        assert np.array_equal(code & 31, lim), j
+        assert np.array_equal((code & 32) != 0, frozen), j
