@@ -509,12 +509,14 @@ __global__ void __launch_bounds__(kWkThreads, 2) day_gvf_walk_kernel(SolweigScen
 // The scene's walk words and albedo-without-shadow plane (one launch per
 // scene), and on request the walk-length codes alone ([4][px], 5 directions
 // of 6 bits per word: samples read, frozen tail).  32 x 32 tiles staged with
-// a halo of 21 as ground / wall bits and albedo, 1024 threads.
+// a halo of 21 as ground / wall / outside bits and albedo, 1024 threads, two blocks
+// per SM (32 registers; one block at 34: 0.28 against 0.34 ms at 1000^2, bound by
+// instruction issue).
 constexpr int kWkStagedN = kWkMaxWidth * kWkMaxWidth;
 
 size_t gvf_walks_smem_bytes() { return sizeof(float) * kWkStagedN + ((kWkStagedN + 15) & ~15); }
 
-__global__ void __launch_bounds__(kWkPixels, 1) gvf_walks_kernel(SolweigScene S, int second,
+__global__ void __launch_bounds__(kWkPixels, 2) gvf_walks_kernel(SolweigScene S, int second,
                                                                      const __grid_constant__ GvfTable<kWkMaxSteps> tab,
                                                                      uint32_t* __restrict__ hits_out,
                                                                      uint32_t* __restrict__ walks_out,
