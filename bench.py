@@ -225,12 +225,12 @@ def _peaks():
 # What bounds each stage of the batched day (from the ncu summaries in
 # profiles/): the HBM fraction of the gather-bound stages is small by nature.
 STAGE_LIMITER = {
-    "day_shadow_kernel": "latency of the ray-step gathers through L1/L2 and lane divergence of the walk lengths",
-    "day_gvf_kernel": "instruction issue of the 18 x 22 walks and the block barriers of the 4-hour passes "
-                      "(shared-memory wavefronts about half of their peak)",
+    "day_shadow_kernel": "instruction issue of the ray steps and lane divergence of the walk lengths",
+    "day_gvf_kernel": "instruction issue of the 18 walks per pixel and their shared-memory loads "
+                      "(wavefronts at 56 % of their peak)",
     "day_tables_kernel": "negligible (one block per hour)",
     "patch_gemm_kernel": "expansion of the mask bits into the BF16 operand stages (the MMAs overlap it)",
-    "day_radiation_kernel": "latency of the per-pixel hour loop",
+    "day_radiation_kernel": "instruction issue of the per-pixel hour loop",
 }
 
 
