@@ -431,6 +431,7 @@ __global__ void __launch_bounds__(kWkThreads, 2) day_gvf_walk_kernel(SolweigScen
                         const int s = tb.shift[k][i], sh = 10 * (s >> 1);
                         const uint32_t nf = ((s & 1 ? free_o : free_e) >> sh) & 1023u;
                         const uint32_t ns = ((s & 1 ? sun_o[k] : sun_e[k]) >> sh) & 1023u;
+                        if ((nf | ns) == 0u) continue;  // not read by this pixel: nothing, though it may be NaN or inf
                         const float g = fmaf(inv_far, (float)nf, inv_far1 * (float)ns);
                         const float2 v = tb.value[k][i];
                         lup = fmaf(g, v.x, lup);
