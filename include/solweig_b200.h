@@ -97,10 +97,12 @@ typedef struct SolweigScene {
        water), from solweig_gvf_walks: walk-length codes [4][pixels], the
        albedo-without-shadow GVF [pixels] and (16-byte aligned) the walk words
        of the batched day; a day without gvf_nosh or gvf_walks prepares them in
-       its work buffer */
+       its work buffer.  gvf_table: solweig_gvf_table_key of the step table they
+       were made for; a call with another table does without them. */
     const uint32_t* gvf_hits;
     const float* gvf_nosh;
     const uint32_t* gvf_walks;
+    uint64_t gvf_table;
 } SolweigScene;
 
 /* Per-patch constants of the sky-vault layout (host arrays, copied per call). */
@@ -445,10 +447,13 @@ int solweig_day_batched_timed(const SolweigScene* scene, const SolweigSkyLayout*
  *   hits   device uint32 [4][pixels] or NULL: samples read (5 bits) and the
  *          repeat flag, 5 directions of 6 bits per word
  *   nosh   device float32 [pixels]: albedo-without-shadow GVF
- * Set scene->gvf_walks / gvf_nosh to them and every later day skips that walk;
- * the results are identical.  solweig_gvf_statics gives hits and nosh alone,
+ * Set scene->gvf_walks / gvf_nosh to them and gvf_table to the table's key, and
+ * every later day with that table skips that walk; the results are identical.  solweig_gvf_statics gives hits and nosh alone,
  * for the 1 m walk (second_steps 22). */
 int64_t solweig_gvf_walk_words(int rows, int cols);
+/* Key of a step table (host [18][second_steps][2]), never 0; 0 for a null table
+ * or a step count outside 1..SOLWEIG_GVF_MAX_STEPS. */
+uint64_t solweig_gvf_table_key(const int32_t* gvf_dxdy, int first_steps, int second_steps);
 int solweig_gvf_walks(const SolweigScene* scene, const int32_t* gvf_dxdy, int first_steps, int second_steps,
                       uint32_t* hits, uint32_t* walks, int64_t words, float* nosh, void* stream);
 int solweig_gvf_statics(const SolweigScene* scene, const int32_t* gvf_dxdy, int first_steps, int second_steps,

@@ -37,6 +37,7 @@ class SolweigScene(ctypes.Structure):
         ("patches", ctypes.c_int32), ("nbands", ctypes.c_int32), ("landcover", ctypes.c_int32),
         ("has_water", ctypes.c_int32), ("hmax", ctypes.c_double), ("geo32", _vp),
         ("gvf_hits", _vp), ("gvf_nosh", _vp), ("gvf_walks", _vp),
+        ("gvf_table", ctypes.c_uint64),
     ]
 
 
@@ -161,7 +162,7 @@ EXPORTED_SYMBOLS = (
     "solweig_patch_sums", "solweig_day_batched_timed", "solweig_day_batched_ex", "solweig_day_batched_part",
     "solweig_day_batched_layout", "solweig_day_grad_work_bytes", "solweig_day_grad_forward",
     "solweig_day_grad_backward", "solweig_svf_ex", "solweig_svf_ex2", "solweig_svf_work_bytes", "solweig_svf_ray_tables",
-    "solweig_gvf_statics", "solweig_gvf_walk_words", "solweig_gvf_walks", "solweig_plan_hours", "solweig_step64_hours", "solweig_step64", "solweig_struct_sizes64", "solweig_wall_segments_burn",
+    "solweig_gvf_statics", "solweig_gvf_walk_words", "solweig_gvf_table_key", "solweig_gvf_walks", "solweig_plan_hours", "solweig_step64_hours", "solweig_step64", "solweig_struct_sizes64", "solweig_wall_segments_burn",
     "solweig_geometry_walls",
 )
 
@@ -207,6 +208,7 @@ def _declare(lib):
         "solweig_gvf_statics": (i32, [P, P, i32, i32, P, P, P]),
         "solweig_plan_hours": (i32, [P, P, i32, dbl, dbl, P, P, P, P, P, i32, P]),
         "solweig_gvf_walk_words": (i64, [i32, i32]),
+        "solweig_gvf_table_key": (ctypes.c_uint64, [P, i32, i32]),
         "solweig_gvf_walks": (i32, [P, P, i32, i32, P, P, i64, P, P]),
         "solweig_day_grad_work_bytes": (i64, [i32, i32, i32]),
         "solweig_day_grad_forward": (i32, [P, P, P, i32, P, i32, i32, P, i32, P, P, i64, P]),

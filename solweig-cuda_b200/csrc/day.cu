@@ -99,6 +99,11 @@ extern "C" int solweig_gvf_statics(const SolweigScene* scene, const int32_t* gvf
     return gvf_scene_walks("solweig_gvf_statics", scene, gvf_dxdy, second_steps, hits, nullptr, nosh, stream);
 }
 
+extern "C" uint64_t solweig_gvf_table_key(const int32_t* gvf_dxdy, int first_steps, int second_steps) {
+    if (!gvf_dxdy || second_steps < 1 || second_steps > SOLWEIG_GVF_MAX_STEPS) return 0;
+    return gvf_table_key(gvf_dxdy, first_steps, second_steps);
+}
+
 extern "C" int64_t solweig_gvf_walk_words(int rows, int cols) {
     return rows > 0 && cols > 0 ? walk_words(rows, cols) : 0;
 }
@@ -298,7 +303,8 @@ int day_batched_impl(const SolweigScene* scene, const SolweigSkyLayout* layout, 
     if (cfg.gvf_hours == 1 && !S.has_water && first_steps == 1 && second_steps >= 2 && second_steps <= kWkMaxSteps &&
         day_walk_args(gvf_dxdy, second_steps, &wa)) {
         uint32_t* walks = reinterpret_cast<uint32_t*>(wb + w.walks);
-        const bool statics = S.gvf_walks && S.gvf_nosh && ((uintptr_t)S.gvf_walks & 15) == 0;
+        const bool statics = S.gvf_walks && S.gvf_nosh && ((uintptr_t)S.gvf_walks & 15) == 0 &&
+                             S.gvf_table == gvf_table_key(gvf_dxdy, first_steps, second_steps);
         if (!statics) {
             const int rc = launch_gvf_walks(S, gvf_dxdy, second_steps, nullptr, walks, nosh, st);
             if (rc) return rc;

@@ -18,6 +18,18 @@ constexpr uint32_t kWkWallBits = (1u << kWkMaxSteps) - 1u;
 constexpr int kWkLimShift = 22;
 constexpr uint32_t kWkFrozen = 1u << 27, kWkFace = 1u << 28;
 
+// Key of a step table (FNV-1a over 32-bit words, 1 us): words and lengths are read only with the
+// table that they were made for.  Under another one a step past its end or a
+// sample outside the raster would be read.
+inline uint64_t gvf_table_key(const int32_t* dxdy, int first, int second) {
+    uint64_t key = 0xcbf29ce484222325ull;
+    auto add = [&](int32_t v) { key = (key ^ (uint32_t)v) * 0x100000001b3ull; };
+    add(first);
+    add(second);
+    for (int i = 0; i < 2 * kWkDirs * second; ++i) add(dxdy[i]);
+    return key ? key : 1u;
+}
+
 __host__ __device__ __forceinline__ long long walk_words(int rows, int cols) {
     return (long long)((rows + kWkTile - 1) / kWkTile) * ((cols + kWkTile - 1) / kWkTile) * kWkTileWords;
 }

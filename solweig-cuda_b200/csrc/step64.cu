@@ -603,8 +603,9 @@ extern "C" int solweig_step64_hours(const SolweigScene* scene, const double* svf
         tab.offs[i] = make_int2(gvf_dxdy[2 * i], gvf_dxdy[2 * i + 1]);
         tab.ahead[i] = (long long)gvf_dxdy[2 * i] * S.cols + gvf_dxdy[2 * i + 1];
     }
-    // the scene's walk lengths are those of these steps (they come with its walk words)
-    const bool hits = S.gvf_hits && first_steps == 1 && second_steps <= 22 && !S.has_water;
+    // the scene's walk lengths and words, if they are those of this table
+    const bool hits = S.gvf_hits && first_steps == 1 && second_steps <= 22 && !S.has_water &&
+                      S.gvf_table == gvf_table_key(gvf_dxdy, first_steps, second_steps);
     const bool words = hits && S.gvf_walks && ((uintptr_t)S.gvf_walks & 3) == 0;
     cudaStream_t st = as_stream(stream);
     const SolweigHour* hr = hours + hour;

@@ -585,6 +585,7 @@ class Scene:
         self.struct.gvf_hits = self.gvf_hits.data_ptr()
         self.struct.gvf_nosh = self.gvf_nosh.data_ptr()
         self.struct.gvf_walks = self.gvf_walks.data_ptr()
+        self.struct.gvf_table = L.solweig_gvf_table_key(self.gvf_host_ptr, self.first_steps, self.second_steps)
 
     def _make_struct(self):
         s = _lib.SolweigScene()
