@@ -153,8 +153,6 @@ def sky_layout(patch_option):
 def svf_ray_tables(patch_option, shape, amaxvalue, scale, device, stream=None):
     """The patches' visibility rays on the device (``solweig_svf_ray_tables``):
     (dxdy [P, capacity, 2], dz [P, capacity], lengths [P], capacity)."""
-    if not amaxvalue == amaxvalue:
-        raise ValueError("amaxvalue is not a number")
     trig, ymajor = rays.svf_ray_constants(patch_option)
     P = ymajor.size
     cap = rays.svf_ray_capacity(patch_option, shape, amaxvalue, scale)

@@ -117,11 +117,14 @@ def svf_ray_constants(patch_option):
 
 def svf_ray_capacity(patch_option, shape, amaxvalue, scale):
     """Steps that hold the longest ray of :func:`svf_rays`: heights grow linearly
-    with the step, so a ray ends within two steps past amaxvalue / rise."""
+    with the step, so a ray ends within two steps past amaxvalue / rise (at the
+    raster's edge when amaxvalue is not a number)."""
     (s, c, _, rise), ymajor = svf_ray_constants(patch_option)
     capacity = max(shape) + 1
     if amaxvalue < 0:
         return 1
+    if np.isnan(amaxvalue):
+        return capacity
     slope = np.abs(1 / np.where(ymajor, s, c)) * (rise / scale)
     bound = np.where(slope > 0, np.ceil(amaxvalue / np.where(slope > 0, slope, 1.0)) + 2, capacity)
     return int(max(1, min(capacity, bound.max())))
