@@ -34,6 +34,7 @@
 namespace solweig {
 
 constexpr int kStep64BX = 32, kStep64BY = 4;
+static_assert(SOLWEIG_SCRATCH64_PLANES % 2 == 0, "an hour's planes keep the next hour's sample pairs aligned");
 
 // Scratch planes of an hour [SOLWEIG_SCRATCH64_PLANES][pixels] float64.
 enum Scratch64 : int {
@@ -63,7 +64,7 @@ __device__ __forceinline__ int first_day_hour(const SolweigHour* __restrict__ ho
 }
 
 __global__ void __launch_bounds__(kStep64BX* kStep64BY) step64_fields_kernel(
-    SolweigScene S, const SolweigHour* __restrict__ hours, double* __restrict__ scratch) {
+    SolweigScene S, const SolweigHour* __restrict__ hours, double* __restrict__ scratch, bool pairs) {
     const SolweigHour& h = hours[blockIdx.z];
     if (!h.daytime) return;
     const int c = blockIdx.x * kStep64BX + threadIdx.x;
@@ -106,8 +107,14 @@ __global__ void __launch_bounds__(kStep64BX* kStep64BY) step64_fields_kernel(
         if (fl & 4) tg = h.twater - h.ta;
     }
     sc[kS64Shadow * n + p] = shadow;
-    reinterpret_cast<double2*>(sc + kS64Sample * n)[p] =
-        make_double2(lup_excess(emis, tg, shadow, h.ta), (double)S.alb[p] * shadow);
+    const double2 v = make_double2(lup_excess(emis, tg, shadow, h.ta), (double)S.alb[p] * shadow);
+    double* sample = sc + kS64Sample * n + 2 * p;
+    if (pairs) {
+        *reinterpret_cast<double2*>(sample) = v;
+    } else {
+        sample[0] = v.x;
+        sample[1] = v.y;
+    }
     reinterpret_cast<uint8_t*>(sc + kS64Bits * n)[p] = sunwall;
 }
 
@@ -120,18 +127,24 @@ __global__ void __launch_bounds__(kStep64BX* kStep64BY) step64_fields_kernel(
 // sample; its walk lengths (kWalkHits) leave a sunlit-wall byte per step; else
 // the ground bits are read first.  The albedo without shadow is the same in
 // every hour of a launch: NOSH (the first daytime hour) sums its five planes.
+// PAIRS: a sample is one 16-byte load, else (scratch on an odd multiple of 8
+// bytes, with the ground bits alone) two.
 // What bounds it: the latency of the samples' loads through L1 and the FP64
 // pipe; 64 registers (8 blocks per SM).  17 hours of 300 x 280 pixels: 1.13 ->
 // 0.68 ms against lengths, a byte and an albedo per step and hour (5 or 6 blocks
 // per SM: 0.78, 0.76 against 0.75 before the offsets came ready).
 enum Walk64 { kWalkGround, kWalkHits, kWalkWords };
 
-template <int WALK, bool NOSH>
+template <int WALK, bool NOSH, bool PAIRS>
 __device__ __forceinline__ void gvf64_pixel(const SolweigScene& S, const SolweigHour& h, const GvfOffsets64& tab,
                                             int first, int second, int r, int c, double* __restrict__ sc) {
     const long long n = (long long)S.rows * S.cols;
     const long long p = (long long)r * S.cols + c;
-    const double2* sample = reinterpret_cast<const double2*>(sc + kS64Sample * n) + p;
+    const double* samples = sc + kS64Sample * n + 2 * p;
+    auto sample = [&](long long ahead) {
+        const double* at = samples + 2 * ahead;
+        return PAIRS ? *reinterpret_cast<const double2*>(at) : make_double2(at[0], at[1]);
+    };
     const double* lup1p = sc + kS64LupFirst * n + p;
     const uint8_t* sunp = reinterpret_cast<const uint8_t*>(sc + kS64Bits * n) + p;
     const uint8_t* flagp = S.flags + p;
@@ -142,7 +155,7 @@ __device__ __forceinline__ void gvf64_pixel(const SolweigScene& S, const Solweig
     const bool own_ground = *flagp & 1;
     const double own_b = own_ground ? 1.0 : 0.0, ground = 1.0 - own_b;
     const double own_sh = sc[kS64Shadow * n + p], own_alb = (double)*albp;
-    const double own_lup = sample->x;
+    const double own_lup = sample(0).x;
     const uint32_t face = S.gvf_face[p];
     const double dfirst = first, dsecond = second;
     const double by_first = 1.0 / dfirst, by_first1 = 1.0 / (dfirst + 1.0);
@@ -197,7 +210,7 @@ __device__ __forceinline__ void gvf64_pixel(const SolweigScene& S, const Solweig
         }
         for (int k = 0; k < lim; ++k) {
             const long long q = ahead[k];
-            t = sample[q];
+            t = sample(q);
             if (WALK != kWalkWords) {
                 if (j == 0 && S.has_water) t.x = lup1p[q];
                 if (sunp[q] && sun == second) sun = k;
@@ -261,7 +274,7 @@ __device__ __forceinline__ void gvf64_pixel(const SolweigScene& S, const Solweig
     }
 }
 
-template <int WALK>
+template <int WALK, bool PAIRS>
 __global__ void __launch_bounds__(kStep64BX* kStep64BY, 8) step64_gvf_kernel(
     SolweigScene S, const SolweigHour* __restrict__ hours, const __grid_constant__ GvfOffsets64 tab, int first,
     int second, double* __restrict__ scratch) {
@@ -271,8 +284,8 @@ __global__ void __launch_bounds__(kStep64BX* kStep64BY, 8) step64_gvf_kernel(
     const int r = blockIdx.y * kStep64BY + threadIdx.y;
     if (r >= S.rows || c >= S.cols) return;
     double* sc = hour_scratch(scratch, (long long)S.rows * S.cols);
-    if (first_day_hour(hours) == (int)blockIdx.z) gvf64_pixel<WALK, true>(S, h, tab, first, second, r, c, sc);
-    else gvf64_pixel<WALK, false>(S, h, tab, first, second, r, c, sc);
+    if (first_day_hour(hours) == (int)blockIdx.z) gvf64_pixel<WALK, true, PAIRS>(S, h, tab, first, second, r, c, sc);
+    else gvf64_pixel<WALK, false, PAIRS>(S, h, tab, first, second, r, c, sc);
 }
 
 // Per-patch and per-band values of one hour (float64), staged in shared memory.
@@ -597,7 +610,6 @@ extern "C" int solweig_step64_hours(const SolweigScene* scene, const double* svf
     SOLWEIG_CHECK_ARG(second_steps >= 1 && second_steps <= SOLWEIG_GVF_MAX_STEPS && first_steps >= 1 &&
                           first_steps <= second_steps,
                       "solweig_step64: GVF steps first=%d second=%d", first_steps, second_steps);
-    SOLWEIG_CHECK_ARG(((uintptr_t)scratch & 15) == 0, "solweig_step64: scratch not 16-byte aligned");
     GvfOffsets64 tab;
     for (int i = 0; i < SOLWEIG_GVF_DIRECTIONS * second_steps; ++i) {
         tab.offs[i] = make_int2(gvf_dxdy[2 * i], gvf_dxdy[2 * i + 1]);
@@ -607,15 +619,18 @@ extern "C" int solweig_step64_hours(const SolweigScene* scene, const double* svf
     const bool hits = S.gvf_hits && first_steps == 1 && second_steps <= 22 && !S.has_water &&
                       S.gvf_table == gvf_table_key(gvf_dxdy, first_steps, second_steps);
     const bool words = hits && S.gvf_walks && ((uintptr_t)S.gvf_walks & 3) == 0;
+    const bool pairs = ((uintptr_t)scratch & 15) == 0;  // an hour's planes are an even number of doubles
     cudaStream_t st = as_stream(stream);
     const SolweigHour* hr = hours + hour;
     dim3 block(kStep64BX, kStep64BY);
     dim3 grid(blocks_for(S.cols, kStep64BX), blocks_for(S.rows, kStep64BY), count);
-    step64_fields_kernel<<<grid, block, 0, st>>>(S, hr, scratch);
+    step64_fields_kernel<<<grid, block, 0, st>>>(S, hr, scratch, pairs);
     SOLWEIG_CHECK_LAUNCH("step64_fields_kernel");
-    if (words) step64_gvf_kernel<kWalkWords><<<grid, block, 0, st>>>(S, hr, tab, first_steps, second_steps, scratch);
-    else if (hits) step64_gvf_kernel<kWalkHits><<<grid, block, 0, st>>>(S, hr, tab, first_steps, second_steps, scratch);
-    else step64_gvf_kernel<kWalkGround><<<grid, block, 0, st>>>(S, hr, tab, first_steps, second_steps, scratch);
+    auto gvf = !pairs ? step64_gvf_kernel<kWalkGround, false>
+               : words ? step64_gvf_kernel<kWalkWords, true>
+               : hits  ? step64_gvf_kernel<kWalkHits, true>
+                       : step64_gvf_kernel<kWalkGround, true>;
+    gvf<<<grid, block, 0, st>>>(S, hr, tab, first_steps, second_steps, scratch);
     SOLWEIG_CHECK_LAUNCH("step64_gvf_kernel");
     step64_wave_kernel<<<blocks_for((long long)S.rows * S.cols, 128), 128, 0, st>>>(S, hr, count, *state, *out,
                                                                                    hour_stride, scratch);
