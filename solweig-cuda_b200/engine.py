@@ -16,6 +16,7 @@ from __future__ import annotations
 
 import ctypes
 import math
+from collections.abc import Sequence
 from dataclasses import dataclass
 from functools import lru_cache
 
@@ -684,7 +685,7 @@ def _plan_scene(scene, latitude):
     return s
 
 
-class DayPlan:
+class DayPlan(Sequence):
     """FP64 host plan of consecutive hours (``solweig_plan_hours``): a sequence of
     (SolweigHour, ShadowRay or None, HourScalars), backed by
 
@@ -731,8 +732,16 @@ class DayPlan:
         rec, sc = self.records[i], self.scalars[i]
         hour = _lib.SolweigHour.from_buffer_copy(self.records, i * HOUR_DTYPE.itemsize)
         ray = lv = None
+    def __add__(self, other):
+        return list(self) + list(other)
+
+    def __radd__(self, other):
+        return list(other) + list(self)
+
         if rec["daytime"]:
             k = int(rec["steps"])
+        if isinstance(i, range):
+            return [self[k] for k in i]
             ray = rays.ShadowRay(self.rays[i, :k], self.dz[i, :k], float(rec["ray_low"]), float(rec["ray_high"]),
                                  int(rec["ray_middle"]))
             L = self.layout
@@ -864,6 +873,11 @@ def plan_rows(met, sol):
     rows = np.zeros((len(met), len(_lib.PLAN_ROW)))
     _sun_columns(rows, sol.altitude, sol.azimuth, sol.zen)
     for name, v in (("jday", sol.jday), ("dectime", sol.dectime), ("altmax", sol.altmax), ("ta", met[:, 11]),
+def plan_hours(scene, met, latitude, longitude, site_altitude, utc):
+    """The hours of :func:`plan_day` one by one."""
+    yield from plan_day(scene, met, latitude, longitude, site_altitude, utc)
+
+
                     ("rh", met[:, 10]), ("rad_g", met[:, 14]), ("rad_d", met[:, 21]), ("rad_i", met[:, 22]),
                     ("p_kpa", met[:, 12]), ("ws", met[:, 9]), ("psi", [_leaf_psi(doy) for doy in met[:, 1]]),
                     ("new_day", sol.dectime == np.floor(sol.dectime))):

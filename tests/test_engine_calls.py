@@ -1,0 +1,33 @@
+"""Calls of the engine that its own day runners do not make: the plan of a day as a
+list and hour by hour, host work beside the wall aspect, the rays' step count."""
+import types
+
+import numpy as np
+import pytest
+
+
+def _plans():
+    from solweig_cuda_b200 import engine, synthetic
+    scene = types.SimpleNamespace(layout=engine.SkyLayout(2), tgk_wall=0.37, tstart_wall=-3.41, tmaxlst_wall=15.0,
+                                  scale=1.0, amaxvalue=20.0, shape=(40, 60), landcover=1)
+    met = synthetic.make_met(doy=172, latitude=53.0, longitude=0.0, seed=4)
+    args = (scene, met, 53.0, 0.0, 3.0, 0.0)
+    return engine.plan_day(*args), engine.plan_hours(*args)
+
+
+def _key(hour):
+    h, ray, scal = hour
+    return h.daytime, h.rad_tot, h.lum[7], None if ray is None else ray.dz.tobytes(), scal.esky
+
+
+def test_a_plan_reads_like_a_list_of_its_hours():
+    plan, hours = _plans()
+    whole = [_key(h) for h in plan]
+    assert len(whole) == len(plan) == 24 and [_key(h) for h in hours] == whole
+    for part in (slice(2, 9), slice(None, None, 5), slice(-3, None), slice(5, 5)):
+        assert [_key(h) for h in plan[part]] == whole[part]
+    assert _key(plan[-1]) == whole[-1] and [_key(h) for h in reversed(plan)] == whole[::-1]
+    assert [_key(h) for h in plan + plan[:2]] == whole + whole[:2]
+    assert [_key(h) for h in plan[:2] + plan] == whole[:2] + whole
+    with pytest.raises(IndexError):
+        plan[24]
