@@ -285,10 +285,11 @@ def wall_aspect(dsm_host, dsm_dev, walls_dev, pixel_size, stream=None):
     return aspect, walls
 
 
-def wall_aspect_device(dsm_host, dsm_dev, walls_dev, pixel_size, stream=None):
+def wall_aspect_device(dsm_host, dsm_dev, walls_dev, pixel_size, stream=None, host_work=None):
     """Wall aspect in degrees as a float64 device tensor (``src/walls.py:83-129``):
     the template kernel on the device, the gradient fall-back only at the few
-    wall pixels the templates leave unresolved (from ``dsm_host`` when given)."""
+    wall pixels the templates leave unresolved (from ``dsm_host`` when given).
+    ``host_work`` (optional) runs on the host while the template kernel runs."""
     rows, cols = dsm_dev.shape
     key = float(pixel_size)
     if key not in _TEMPLATE_CACHE:
@@ -297,6 +298,8 @@ def wall_aspect_device(dsm_host, dsm_dev, walls_dev, pixel_size, stream=None):
     mask = walls_dev > 0
     aspect = torch.zeros_like(dsm_dev)
     if not bool(mask.any()):
+        if host_work is not None:
+            host_work()
         return aspect
     if rows > 2 * radius + 2 and cols > 2 * radius + 2:
         dev = dsm_dev.device
@@ -305,6 +308,8 @@ def wall_aspect_device(dsm_host, dsm_dev, walls_dev, pixel_size, stream=None):
             device_ptr(dsm_dev), device_ptr(walls_dev), device_ptr(aspect), rows, cols, radius,
             device_ptr(t[0][0]), device_ptr(t[0][1]), device_ptr(t[1][0]), device_ptr(t[1][1]),
             device_ptr(t[2][0]), device_ptr(t[2][1]), stream_handle(stream)), "solweig_wall_aspect")
+    if host_work is not None:
+        host_work()
     unresolved = torch.nonzero((mask & (aspect == 0)).flatten()).flatten()
     if unresolved.numel():
         host = dsm_host if dsm_host is not None else dsm_dev.cpu().numpy()

@@ -31,3 +31,17 @@ def test_a_plan_reads_like_a_list_of_its_hours():
     assert [_key(h) for h in plan[:2] + plan] == whole[:2] + whole
     with pytest.raises(IndexError):
         plan[24]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("walls", [True, False])
+def test_host_work_runs_once_beside_the_aspect(cuda, walls):
+    import torch
+    from solweig_cuda_b200 import engine, synthetic
+    dsm = synthetic.make_scene(60, 70, seed=3).dsm.astype(np.float64) if walls else np.zeros((60, 70))
+    dev = torch.from_numpy(dsm).to(cuda)
+    heights = engine.wall_heights_device(dev, 3.0)
+    done = []
+    got = engine.wall_aspect_device(dsm, dev, heights, 1.0, host_work=lambda: done.append(1))
+    assert done == [1]
+    assert torch.equal(got, engine.wall_aspect_device(dsm, dev, heights, 1.0))
