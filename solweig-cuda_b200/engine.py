@@ -692,7 +692,8 @@ def _plan_scene(scene, latitude):
 
 class DayPlan(Sequence):
     """FP64 host plan of consecutive hours (``solweig_plan_hours``): a sequence of
-    (SolweigHour, ShadowRay or None, HourScalars), backed by
+    (SolweigHour, ShadowRay or None, HourScalars), made when asked for (slices and
+    sums are lists of them), backed by
 
     ``records``    [n] SolweigHour records (without their ray pointers),
     ``rays``/``dz``  [n, capacity, 2] int32 / [n, capacity] float64 sun rays,
@@ -732,21 +733,21 @@ class DayPlan(Sequence):
         """Band sky emittances [n, MAX_BANDS] float64."""
         return self.scalars[:, _BAND0:]
 
-    def __getitem__(self, i):
-        i = range(len(self))[i]
-        rec, sc = self.records[i], self.scalars[i]
-        hour = _lib.SolweigHour.from_buffer_copy(self.records, i * HOUR_DTYPE.itemsize)
-        ray = lv = None
     def __add__(self, other):
         return list(self) + list(other)
 
     def __radd__(self, other):
         return list(other) + list(self)
 
-        if rec["daytime"]:
-            k = int(rec["steps"])
+    def __getitem__(self, i):
+        i = range(len(self))[i]
         if isinstance(i, range):
             return [self[k] for k in i]
+        rec, sc = self.records[i], self.scalars[i]
+        hour = _lib.SolweigHour.from_buffer_copy(self.records, i * HOUR_DTYPE.itemsize)
+        ray = lv = None
+        if rec["daytime"]:
+            k = int(rec["steps"])
             ray = rays.ShadowRay(self.rays[i, :k], self.dz[i, :k], float(rec["ray_low"]), float(rec["ray_high"]),
                                  int(rec["ray_middle"]))
             L = self.layout
@@ -873,16 +874,16 @@ def plan_day(scene, met, latitude, longitude, site_altitude, utc, sol=None):
                    (1.0, 1.0, 0.0))
 
 
-def plan_rows(met, sol):
-    """Rows of the host plan [n, len(PLAN_ROW)] from forcing rows and their sun positions."""
-    rows = np.zeros((len(met), len(_lib.PLAN_ROW)))
-    _sun_columns(rows, sol.altitude, sol.azimuth, sol.zen)
-    for name, v in (("jday", sol.jday), ("dectime", sol.dectime), ("altmax", sol.altmax), ("ta", met[:, 11]),
 def plan_hours(scene, met, latitude, longitude, site_altitude, utc):
     """The hours of :func:`plan_day` one by one."""
     yield from plan_day(scene, met, latitude, longitude, site_altitude, utc)
 
 
+def plan_rows(met, sol):
+    """Rows of the host plan [n, len(PLAN_ROW)] from forcing rows and their sun positions."""
+    rows = np.zeros((len(met), len(_lib.PLAN_ROW)))
+    _sun_columns(rows, sol.altitude, sol.azimuth, sol.zen)
+    for name, v in (("jday", sol.jday), ("dectime", sol.dectime), ("altmax", sol.altmax), ("ta", met[:, 11]),
                     ("rh", met[:, 10]), ("rad_g", met[:, 14]), ("rad_d", met[:, 21]), ("rad_i", met[:, 22]),
                     ("p_kpa", met[:, 12]), ("ws", met[:, 9]), ("psi", [_leaf_psi(doy) for doy in met[:, 1]]),
                     ("new_day", sol.dectime == np.floor(sol.dectime))):
