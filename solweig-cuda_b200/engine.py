@@ -55,6 +55,32 @@ def stream_handle(stream=None):
     return ctypes.c_void_p(s.cuda_stream)
 
 
+def _as_stream(stream):
+    return stream if isinstance(stream, torch.cuda.Stream) else torch.cuda.ExternalStream(stream.cuda_stream)
+
+
+def fork(stream=None):
+    """Handle of the stream that kernels go to: the current one, or ``stream`` once it
+    waits for the current one, whose uploads and torch kernels made their inputs
+    (and whose memory pool their outputs come from)."""
+    if stream is not None:
+        _as_stream(stream).wait_stream(torch.cuda.current_stream())
+    return stream_handle(stream)
+
+
+def join(stream=None):
+    """Let the current stream, which reads what kernels on ``stream`` wrote, wait for them."""
+    if stream is not None:
+        torch.cuda.current_stream().wait_stream(_as_stream(stream))
+
+
+def lend(stream, *tensors):
+    """Keep the memory of ``tensors``, about to be freed, until kernels on ``stream`` are done."""
+    if stream is not None:
+        for t in tensors:
+            t.record_stream(_as_stream(stream))
+
+
 def device_ptr(t):
     return ctypes.c_void_p(t.data_ptr()) if t is not None else None
 
@@ -164,7 +190,7 @@ def svf_ray_tables(patch_option, shape, amaxvalue, scale, device, stream=None):
     host = [ctypes.c_void_p(a.ctypes.data) for a in (trig[0], trig[1], trig[2], rise, ymajor)]
     _lib.check(_lib.lib().solweig_svf_ray_tables(
         *host, P, shape[0], shape[1], float(amaxvalue), cap, device_ptr(dxdy), device_ptr(dz), device_ptr(lengths),
-        stream_handle(stream)), "solweig_svf_ray_tables")
+        fork(stream)), "solweig_svf_ray_tables")
     return dxdy, dz, lengths, cap
 
 
@@ -253,8 +279,9 @@ def wall_heights_device(dsm_dev, threshold, stream=None):
     rows, cols = dsm_dev.shape
     walls = torch.empty_like(dsm_dev)
     _lib.check(_lib.lib().solweig_wall_heights(device_ptr(dsm_dev), device_ptr(walls), rows, cols,
-                                                float(threshold), stream_handle(stream)),
+                                                float(threshold), fork(stream)),
                "solweig_wall_heights")
+    join(stream)
     return walls
 
 
@@ -277,7 +304,8 @@ def wall_aspect(dsm_host, dsm_dev, walls_dev, pixel_size, stream=None):
         _lib.check(_lib.lib().solweig_wall_aspect(
             device_ptr(dsm_dev), device_ptr(walls_dev), device_ptr(out), rows, cols, radius,
             device_ptr(t[0][0]), device_ptr(t[0][1]), device_ptr(t[1][0]), device_ptr(t[1][1]),
-            device_ptr(t[2][0]), device_ptr(t[2][1]), stream_handle(stream)), "solweig_wall_aspect")
+            device_ptr(t[2][0]), device_ptr(t[2][1]), fork(stream)), "solweig_wall_aspect")
+        join(stream)
         aspect = out.cpu().numpy()
     unresolved = np.flatnonzero(mask & (aspect == 0))
     if unresolved.size:
@@ -307,7 +335,8 @@ def wall_aspect_device(dsm_host, dsm_dev, walls_dev, pixel_size, stream=None, ho
         _lib.check(_lib.lib().solweig_wall_aspect(
             device_ptr(dsm_dev), device_ptr(walls_dev), device_ptr(aspect), rows, cols, radius,
             device_ptr(t[0][0]), device_ptr(t[0][1]), device_ptr(t[1][0]), device_ptr(t[1][1]),
-            device_ptr(t[2][0]), device_ptr(t[2][1]), stream_handle(stream)), "solweig_wall_aspect")
+            device_ptr(t[2][0]), device_ptr(t[2][1]), fork(stream)), "solweig_wall_aspect")
+        join(stream)
     if host_work is not None:
         host_work()
     unresolved = torch.nonzero((mask & (aspect == 0)).flatten()).flatten()
@@ -346,7 +375,9 @@ def _gradient_aspect(dsm, pixel_size, flat_idx):
 
 
 class Scene:
-    """Static geometry and per-pixel statics of one tile, resident on the device."""
+    """Static geometry and per-pixel statics of one tile, resident on the device.
+    Its kernels go to ``stream`` (the current one when None); work on another stream
+    waits for that one first."""
 
     def __init__(self, dsm, trees, dem, pixel_size=1.0, landcover=None, wall_threshold=3.0,
                  patch_option=2, device="cuda", walls=None, aspect=None, stream=None,
@@ -370,7 +401,6 @@ class Scene:
         self.layout = sky_layout(int(patch_option))
         self.patch_option = int(patch_option)
         L = _lib.lib()
-        st = stream_handle(stream)
         n = self.pixels
         # Raise / clip semantics of src/series.py:252-291 (one host sync).
         dsm_lo, dsm_hi, dem_lo, trees_hi = torch.stack(
@@ -415,7 +445,8 @@ class Scene:
             defaults.ctypes.data_as(ctypes.c_void_p), device_ptr(self.dsm), device_ptr(self.vegdem),
             device_ptr(self.vegdem2), device_ptr(self.flags), device_ptr(self.alb),
             device_ptr(self.emis), device_ptr(self.tgk), device_ptr(self.tstart),
-            device_ptr(self.tmaxlst), device_ptr(self.lc_grid), st), "solweig_scene_build")
+            device_ptr(self.tmaxlst), device_ptr(self.lc_grid), fork(stream)), "solweig_scene_build")
+        join(stream)
         if landcover is not None:
             wall_row = LANDCOVER_CLASSES[LANDCOVER_CLASSES[:, 0] == 99][0]
             self.tgk_wall, self.tstart_wall, self.tmaxlst_wall = (float(wall_row[3]),
@@ -426,8 +457,6 @@ class Scene:
         del dsm_in, trees_in, dem_in, lc_in
         self.has_water = int(bool(((self.flags & 4) != 0).any().item())) if landcover is not None else 0
         # Sky view factor: bit-packed visibility + the 16 reduce planes.
-        t_dxdy, t_dz, t_len, cap = svf_ray_tables(patch_option, self.shape, self.amaxvalue, self.scale, dev, stream)
-        self._svf_lengths = t_len
         nb = self.layout.struct.nbands
         self.masks = torch.empty((2 * _lib.MASK_WORDS, self.rows, self.cols), dtype=torch.int32,
                                  device=dev)
@@ -443,8 +472,10 @@ class Scene:
         self.gvf_dxdy_host, self.first_steps, self.second_steps = rays.gvf_offsets(self.scale)
         self.gvf_dxdy = _upload(self.gvf_dxdy_host, np.int32, dev)
         self.gvf_host_ptr = self.gvf_dxdy_host.ctypes.data_as(ctypes.c_void_p)
+        t_dxdy, t_dz, t_len, cap = svf_ray_tables(patch_option, self.shape, self.amaxvalue, self.scale, dev, stream)
         # ray ceilings and exit tables of one patch word (solweig_svf_ex2)
         svf_work = torch.empty(int(L.solweig_svf_work_bytes(self.rows, self.cols)), dtype=torch.uint8, device=dev)
+        st = fork(stream)  # from here on the current stream gets no work
         _lib.check(L.solweig_svf_ex2(
             device_ptr(self.dsm), device_ptr(self.vegdem), device_ptr(self.vegdem2), device_ptr(self.geo32),
             device_ptr(self.flags), self.rows, self.cols, lay.struct.patches, cap,
@@ -453,7 +484,8 @@ class Scene:
             lay.sectors.ctypes.data_as(ctypes.c_void_p), CONSTANTS["transVeg"],
             device_ptr(self.masks), device_ptr(planes), device_ptr(self.veg_sums),
             device_ptr(self.sky_band_counts), device_ptr(svf_work), svf_work.numel(), st), "solweig_svf")
-        del t_dxdy, t_dz, svf_work
+        lend(stream, t_dxdy, t_dz, t_len, svf_work, planes)
+        del t_dxdy, t_dz, t_len, svf_work
         # Derived statics after the float32 round trip of the SVF planes.
         self.svf32 = torch.empty((15, self.rows, self.cols), **f32)
         self.svfbuveg = torch.empty(self.shape, **f32)
@@ -490,7 +522,6 @@ class Scene:
         self.patch_option = int(inputs.get("patch_option", 2))
         self.layout = sky_layout(self.patch_option)
         L = _lib.lib()
-        st = stream_handle(stream)
 
         def f64(x):
             return _as_device(x, torch.float64, dev, self.shape)
@@ -533,7 +564,7 @@ class Scene:
                  for k in ("shmat", "vegshmat", "vbshvegshmat")]
         self.masks = torch.empty((2 * _lib.MASK_WORDS, rows, cols), dtype=torch.int32, device=dev)
         _lib.check(L.solweig_svf_pack(device_ptr(cubes[0]), device_ptr(cubes[1]), device_ptr(cubes[2]),
-                                      self.pixels, P, device_ptr(self.masks), st), "solweig_svf_pack")
+                                      self.pixels, P, device_ptr(self.masks), fork(stream)), "solweig_svf_pack")
         nb = self.layout.struct.nbands
         planes = torch.empty((16, rows, cols), dtype=torch.float64, device=dev)
         self.veg_sums = torch.empty((4, rows, cols), dtype=torch.float32, device=dev)
@@ -543,7 +574,7 @@ class Scene:
             device_ptr(self.masks), device_ptr(self.vegdem2), self.pixels, ctypes.byref(lay.struct),
             lay.band_weights.ctypes.data_as(ctypes.c_void_p), lay.sectors.ctypes.data_as(ctypes.c_void_p),
             CONSTANTS["transVeg"], device_ptr(planes), device_ptr(self.veg_sums),
-            device_ptr(self.sky_band_counts), st), "solweig_svf_reduce")
+            device_ptr(self.sky_band_counts), fork(stream)), "solweig_svf_reduce")
         self.planes = None
         svf_names = cls.SVF_ORDER
         self.svf32 = torch.stack([f32(inputs[k]) for k in svf_names])
@@ -557,14 +588,15 @@ class Scene:
             device_ptr(planes), device_ptr(self.walls), device_ptr(self.aspect), self.pixels,
             CONSTANTS["transVeg"], lo.ctypes.data_as(ctypes.c_void_p), hi.ctypes.data_as(ctypes.c_void_p),
             mid.ctypes.data_as(ctypes.c_void_p), None, device_ptr(scratch["svfbuveg"]),
-            device_ptr(scratch["svfalfa"]), device_ptr(scratch["tan"]), device_ptr(self.gvf_face), st),
+            device_ptr(scratch["svfalfa"]), device_ptr(scratch["tan"]), device_ptr(self.gvf_face), fork(stream)),
             "solweig_scene_finalize")
+        lend(stream, planes, *cubes, *scratch.values())
         first, second = float(inputs.get("first", 1.0)), float(inputs.get("second", 22.0))
         self.gvf_dxdy_host, self.first_steps, self.second_steps = rays.gvf_offsets(self.scale, first, second)
         self.gvf_dxdy = _upload(self.gvf_dxdy_host, np.int32, dev)
         self.gvf_host_ptr = self.gvf_dxdy_host.ctypes.data_as(ctypes.c_void_p)
         self.struct = self._make_struct()
-        self._gvf_statics(st)
+        self._gvf_statics(fork(stream))
         return self
 
     def _gvf_statics(self, st):
@@ -623,8 +655,8 @@ class Scene:
 
     @property
     def svf_steps(self):
-        """Steps of the 153 visibility rays together."""
-        return int(self._svf_lengths.sum())
+        """Steps of the visibility rays together."""
+        return int(rays.svf_rays(self.patch_option, self.shape, self.amaxvalue, self.scale)[2].sum())
 
     @property
     def walls_host(self):
@@ -947,7 +979,8 @@ class DayRunner:
         return outputs_struct(res, index)
 
     def run_day(self, met, outputs=("tmrt", "utci"), stream=None):
-        """Run the rows of one calendar day; returns {name: tensor [H, rows, cols]}."""
+        """Run the rows of one calendar day; returns {name: tensor [H, rows, cols]},
+        which kernels on ``stream`` (the current one when None) write."""
         met = np.asarray(met, dtype=np.float64)
         if len(met) > self.buffers.hours:
             raise ValueError(f"at most {self.buffers.hours} rows per day")
@@ -956,6 +989,7 @@ class DayRunner:
         self.buffers.wait_free()
         self._stage(plan)
         self.reset_state()
+        fork(stream)
         self._launch_day(len(plan), res, stream)
         self.buffers.mark()
         self.last_plan = plan

@@ -45,3 +45,48 @@ def test_host_work_runs_once_beside_the_aspect(cuda, walls):
     got = engine.wall_aspect_device(dsm, dev, heights, 1.0, host_work=lambda: done.append(1))
     assert done == [1]
     assert torch.equal(got, engine.wall_aspect_device(dsm, dev, heights, 1.0))
+
+
+@pytest.mark.gpu
+def test_svf_steps_counts_the_rays(cuda):
+    from solweig_cuda_b200 import engine, rays, synthetic
+    c = synthetic.make_scene(48, 64, seed=3)
+    scene = engine.Scene(c.dsm, c.trees, c.dem, 1.0, landcover=c.landcover)
+    assert scene.svf_steps == rays.svf_rays(2, scene.shape, scene.amaxvalue, 1.0)[2].sum()
+
+
+@pytest.mark.gpu
+def test_a_scene_and_its_days_on_another_stream_are_the_same(cuda):
+    """Statics of a scene built on a side stream and days run on one, while the
+    current stream is idle and while it is not."""
+    import torch
+    from solweig_cuda_b200 import engine, synthetic
+    c = synthetic.make_scene(150, 131, seed=5)
+    met = synthetic.make_met(doy=172, latitude=53.0, longitude=0.0, seed=4)
+    busy = torch.zeros(1 << 26, device=cuda)
+
+    def build(stream, work):
+        res = {}
+        torch.cuda.synchronize()
+        for _ in range(work):
+            busy.add_(1.0)
+        scene = engine.Scene(c.dsm, c.trees, c.dem, 1.0, landcover=c.landcover, stream=stream)
+        torch.cuda.synchronize()
+        for name in ("walls", "aspect", "masks", "svf32", "gvf_face", "gvf_walks", "gvf_nosh"):
+            res[name] = getattr(scene, name).cpu().numpy()
+        for runner in (engine.DayRunner, engine.DayRunner64):
+            run = runner(scene, 53.0, 0.0, 3.0, 0.0)
+            torch.cuda.synchronize()
+            for _ in range(work):
+                busy.add_(1.0)
+            out = run.run_day(met, stream=stream)
+            torch.cuda.synchronize()
+            res.update({(runner.__name__, k): v.cpu().numpy() for k, v in out.items()})
+        return res
+
+    want = build(None, 0)
+    side = torch.cuda.Stream()
+    for work in (0, 0, 50):
+        got = build(side, work)
+        for name, v in want.items():
+            assert np.array_equal(got[name], v, equal_nan=True), (name, work)
