@@ -172,7 +172,11 @@ __device__ __forceinline__ void warp_tile_pixel(int bx, int by, int& r, int& c) 
 }
 
 // TABLES: the packed geometry with the hours' tables (exits, step records of
-// kpitch entries per hour, plane of H), else the rasters step by step.
+// kpitch entries per hour, plane of H), else the rasters step by step.  Eight
+// blocks per SM for both: the step-by-step walk is bound by the latency of its
+// loads, and its few spills at 32 registers cost less than the occupancy of 40
+// (2000 x 2000 px with relief, heights not exact in float32: 7.21 against 7.89 ms
+// a day, 1000 x 1000 px 1.83 against 1.96).
 template <bool TABLES>
 __global__ void __launch_bounds__(256, 8) day_shadow_kernel(SolweigScene S, const SolweigHour* __restrict__ hours,
                                                             float4* __restrict__ quads,
