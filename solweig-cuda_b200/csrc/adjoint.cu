@@ -1159,7 +1159,7 @@ __global__ void __launch_bounds__(32 * kLumWarps, 2) lum_grad_kernel(SolweigScen
 struct GradWork {
     long long day_total;  // the batched-day work (quads0 = its quads)
     long long quads1, sv, gvf, lam_gl, lam_ga, lam_gn, lam_s, lam_sums, lam_lup, lam_albsh, lam_alb, d_emis_direct;
-    long long codes, words;  // of the GVF walks: samples' codes and the transpose's words
+    long long walks, codes, words;  // of the GVF walks: walk words (read until the transpose), samples' codes, the transpose's words
     long long total;
 };
 
@@ -1182,6 +1182,7 @@ GradWork grad_work_layout(int rows, int cols, int nhours) {
     g.lam_alb = o; o = align256(o + 4LL * px);
     g.d_emis_direct = o; o = align256(o + 4LL * px);
     const long long passes = (nhours + kWkHours - 1) / kWkHours;
+    g.walks = o; o = align256(o + 4LL * walk_words(rows, cols));
     g.codes = o; o = align256(o + 4LL * px * passes);
     g.words = o; o = align256(o + 4LL * 2 * kTrGroups * px * passes);
     g.total = o;
@@ -1252,7 +1253,7 @@ static int grad_prepare(const SolweigScene* scene, const SolweigSkyLayout* layou
     // 0.60 ms instead of 1.22 ms with one block per tile and hour).
     walk_words = day_walk_args(gvf_dxdy, second_steps, &wa);
     if (walk_words) {
-        uint32_t* walks = reinterpret_cast<uint32_t*>(wb + dw.walks);
+        uint32_t* walks = reinterpret_cast<uint32_t*>(wb + gw.walks);
         rc = launch_gvf_walks(Sp, gvf_dxdy, second_steps, nullptr, walks, nosh, st);
         if (rc) return rc;
         wa.walks = walks;

@@ -1035,8 +1035,15 @@ DayWork day_work_layout(int rows, int cols, int nhours, bool water) {
     // per 16 x 16 tile maxima of the heights (ceil(rows/16) * ceil(cols/16)
     // floats, bounded here from the pixel count alone: <= px/256 + (rows + cols)/16 + 1)
     w.tilemax = o; o = align256(o + 4LL * (px / 256 + (px + 1) / 16 + 4));
-    // GVF walk words, for scenes that come without them, and the tiles' distinct samples
-    w.walks = o; o = align256(o + (water ? 0 : 4LL * walk_words(rows, cols)));
+    // GVF walk words, for scenes that come without them: in the patch-sum region
+    // behind the samples' codes, free until the contraction (72 bytes per pixel that
+    // most scenes bring along); days too short for that (four hours and less) keep a
+    // region of their own
+    const long long words = water ? 0 : 4LL * walk_words(rows, cols);
+    const long long codes = align256(4LL * px * ((nhours + kWkHours - 1) / kWkHours));
+    w.walks = w.sums + codes;
+    if (codes + words > 4LL * px * 2 * ncols) { w.walks = o; o = align256(o + words); }
+    // the tiles' distinct samples
     w.dict = o;
     o = align256(o + (water ? 0 : walk_words(rows, cols) / kWkTileWords * 8 * kWkDictKeys * ((nhours + 3) / kWkHours)));
     // per hour the first-outside steps of the rows and columns, and the ray's step records
