@@ -152,9 +152,6 @@ def day_launches(scene, config, sweep_parts=1):
     return sweep_parts * (2 + c) + c + win + walk + 7
 
 
-PIPELINE_HOURS = (2, 2, 2, 2, 4, 4, 8)
-
-
 class ChosenDay(BatchedDay):
     """The batched form: every hour of a day in a few launches
     (``solweig_day_batched``: ray ceilings and shadow sweep, GVF over all hours,
@@ -168,18 +165,18 @@ class ChosenDay(BatchedDay):
     CARDINAL = ("keast", "ksouth", "kwest", "knorth", "least", "lsouth", "lwest", "lnorth")
 
     def __init__(self, scene, latitude, longitude, site_altitude=3.0, utc=0.0, hours=24,
-                 outputs=("tmrt", "utci"), use_graph=True, pipeline_hours=PIPELINE_HOURS):
+                 outputs=("tmrt", "utci"), use_graph=True, pipeline_hours=0):
         bad = [o for o in outputs if o in self.CARDINAL]
         if bad:
             raise ValueError(f"the batched form does not produce {bad}")
         super().__init__(scene, latitude, longitude, site_altitude, utc, hours, outputs, use_graph)
         self.scratch = None
         # pipeline_hours: an int or a sequence of range lengths (the last one
-        # repeats) issues the sweep stage in ranges of hours with a graph each; 0
-        # and the default issue it as a whole.  Ranges let the GPU start before
-        # the last hours are planned, but planning a day takes 0.2 ms after the
-        # sun positions, less than seven sweep launches cost a small raster.
-        self.ranges = None if pipeline_hours is PIPELINE_HOURS else self._ranges(hours, pipeline_hours)
+        # repeats) issues the sweep stage in ranges of hours with a graph each, 0
+        # as a whole.  The day is planned before either: that takes 0.2 ms after
+        # the sun positions, less than seven more sweep launches cost a small
+        # raster, so ranges only bound the sweep stage's single launches.
+        self.ranges = self._ranges(hours, pipeline_hours)
         self.part_graphs = None
         L = _lib.lib()
         self.work_bytes = int(L.solweig_day_batched_work_bytes(scene.rows, scene.cols, hours,
