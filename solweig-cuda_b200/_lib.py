@@ -18,6 +18,7 @@ MAX_PATCHES = 160
 MASK_WORDS = 5
 MAX_BANDS = 8
 GVF_DIRECTIONS = 18
+PACKED_MAX_PIXELS = 1 << 28  # largest raster of the packed shadow walk
 GVF_MAX_STEPS = 64
 SCRATCH_PLANES = 20  # quad (4) + first-direction Lup (1) + 15 GVF planes
 SCRATCH64_PLANES = 20  # float64 step: 5 per-pixel GVF inputs + 15 GVF planes

@@ -141,15 +141,21 @@ class BatchedDay:
 def day_launches(scene, config, sweep_parts=1):
     """Kernel launches of one batched day for this scene and launch shapes,
     with the sweep stage issued in ``sweep_parts`` hour ranges: per range the
-    ray exits, the ceilings and the sweep; once the height dilation (and the
-    tile maxima of the window sweep); then the GVF (sample codes and the walk
-    kernel, or the per-hour kernel), weights, two splits (sky and vegetation
-    weights), tables, contraction and radiation."""
-    c = int(not config.no_ceiling)
-    walk = int(config.gvf_hours == 1 and scene.first_steps == 1 and 2 <= scene.second_steps <= 22
-               and not scene.struct.has_water)
-    win = int(config.sweep_window != 0 and scene.geo32 is not None and not scene.struct.has_water)
-    return sweep_parts * (2 + c) + c + win + walk + 7
+    ray exits, the ceilings and the sweep; once the height dilation, for the
+    ceilings or the raster sweep's plane of heights (and the tile maxima of the
+    window sweep); then the GVF (the walk words where the scene has none for
+    its step table, sample codes and the walk kernel, or the per-hour kernel),
+    weights, two splits (sky and vegetation weights), tables, contraction and
+    radiation."""
+    s = scene.struct
+    ceiling = int(not config.no_ceiling)
+    window = int(config.sweep_window != 0 and scene.geo32 is not None and not s.has_water)
+    height = scene.geo32 is not None and not window and scene.pixels <= _lib.PACKED_MAX_PIXELS
+    walk = config.gvf_hours == 1 and scene.first_steps == 1 and 2 <= scene.second_steps <= 22 and not s.has_water
+    statics = s.gvf_walks and s.gvf_nosh and s.gvf_table == _lib.lib().solweig_gvf_table_key(
+        scene.gvf_host_ptr, scene.first_steps, scene.second_steps)
+    gvf = (2 if statics else 3) if walk else 1
+    return sweep_parts * (2 + ceiling) + int(ceiling or height) + window + gvf + 6
 
 
 class ChosenDay(BatchedDay):

@@ -244,8 +244,10 @@ int day_batched_impl(const SolweigScene* scene, const SolweigSkyLayout* layout, 
                 SOLWEIG_CHECK_LAUNCH("sweep_tile_max_kernel");
             }
         }
-        // the plane of H lives in the albedo-without-shadow plane, free until the GVF
-        float* height = S.geo32 ? nosh : nullptr;
+        // the raster sweep on the packed geometry reads tables; its plane of H lives
+        // in the albedo-without-shadow plane, free until the GVF
+        const bool packed = S.geo32 && !window && px <= kPackedMaxPixels;
+        float* height = packed ? nosh : nullptr;
         if ((ceiling || height) && h0 == 0) {
             dim3 dgrid(blocks_for(S.cols, kDilTile), blocks_for(S.rows, kDilTile));
             if (S.geo32) ceiling_dilate_kernel<true><<<dgrid, dim3(32, 8), 0, st>>>(S, dil, height);
@@ -283,7 +285,7 @@ int day_batched_impl(const SolweigScene* scene, const SolweigSkyLayout* layout, 
             return SOLWEIG_OK;
         }
         dim3 grid(blocks_for(S.cols, cfg.shadow_bx), blocks_for(S.rows, cfg.shadow_by), nh);
-        if (S.geo32 && px <= kPackedMaxPixels)
+        if (packed)
             day_shadow_kernel<true><<<grid, dim3(cfg.shadow_bx, cfg.shadow_by), 0, st>>>(
                 S, hours + h0, quads + h0 * px, lup_first ? lup_first + h0 * px : nullptr,
                 ceiling ? ceiling + h0 * px : nullptr, exits, rec, kpitch, height);
