@@ -21,9 +21,10 @@
 // the window can change any lane's outputs and the warp jumps to the first
 // step outside the window together.
 //
-// The per-step recurrences are those of shadow_walk_packed (shadow.cuh), in
-// the same float64 operations: every output is bit-identical.  The raster
-// must carry the packed float32 geometry (SolweigScene::geo32).
+// The per-step recurrences and exits are those of shadow_walk_geo (shadow.cuh),
+// in the same float64 operations; shadow_walk_packed, which the raster sweep
+// takes, screens its samples in float32 and skips others, but every output of
+// the three is the same.  The raster must carry the packed float32 geometry (SolweigScene::geo32).
 #pragma once
 #include <cuda.h>
 
@@ -156,7 +157,7 @@ __device__ __forceinline__ ShadowResult shadow_walk_window(
         }
         return s.shadowed && (!is_wall || s.f - a >= wall);
     };
-    // true: nothing further can change (the exits of shadow_walk_packed)
+    // true: nothing further can change (the exits of shadow_walk_geo)
     auto settled = [&](long long q, int k, double dzk) {
         if (dz_prev >= clear && (!is_wall || (s.topmax >= 0.0 && hmax - dzk <= s.topmax))) return true;
         if (ceiling != nullptr && k >= 4 && (k & 3) == 0) {
