@@ -104,15 +104,21 @@ def svf_patch_directions(patch_option):
     return azimuth, altitude, counts
 
 
-@lru_cache(maxsize=4)
 def svf_ray_constants(patch_option):
     """Per patch (sin, cos, tan) of the azimuth, tan of the altitude and whether
     the columns are the ray's major axis: what the device builds the rays of
     :func:`svf_rays` from (``solweig_svf_ray_tables``)."""
+    return _svf_ray_constants(int(patch_option))
+
+
+@lru_cache(maxsize=4)
+def _svf_ray_constants(patch_option):
     azimuth, altitude, _ = svf_patch_directions(patch_option)
     az = [a * (np.pi / 180.) for a in azimuth]
     trig = np.array([[np.sin(a), np.cos(a), np.tan(a), np.tan(e * (np.pi / 180.))] for a, e in zip(az, altitude)])
-    return np.ascontiguousarray(trig.T), np.array([_ymajor(a) for a in az], dtype=np.uint8)
+    trig, ymajor = np.ascontiguousarray(trig.T), np.array([_ymajor(a) for a in az], dtype=np.uint8)
+    trig.flags.writeable = ymajor.flags.writeable = False  # shared by every caller
+    return trig, ymajor
 
 
 def svf_ray_capacity(patch_option, shape, amaxvalue, scale):
