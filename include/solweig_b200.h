@@ -371,9 +371,9 @@ int solweig_step64_hours(const SolweigScene* scene, const double* svfbuveg, cons
                          double* scratch, void* stream);
 
 /* Batched day ----------------------------------------------------------------
- * All nhours (<= 64) hours of one day (src/series.py:445-491) in seven
- * launches: shadow sweep and ground view factors for every hour (one launch
- * each), the luminance-weighted sky / vegetation patch sums of all hours as
+ * All nhours (<= 64) hours of one day (src/series.py:445-491) in a dozen
+ * launches: ray ceilings and shadow sweep of every hour, ground view factors of
+ * all hours (walk words, or one launch slice per hour), the luminance-weighted sky / vegetation patch sums of all hours as
  * one BF16 tensor-core contraction (tcgen05, FP32 accumulation, weights split
  * into BF16 hi + lo), per-hour sunlit/shaded tables, and one radiation launch
  * whose threads loop over the hours with the wave-delay state in registers.
@@ -397,9 +397,9 @@ typedef struct SolweigDayConfig {
     int32_t gvf_rows;              /* GVF tile rows per block: 4, 8 or 16 (32 columns) */
     int32_t rad_threads;           /* radiation block: 128 or 256 pixels */
     int32_t gemm_ctas_per_sm;      /* contraction CTAs per SM: 0 = as many as fit, 1, 2 */
-    int32_t gvf_hours;             /* 1: 32x32 tiles walk all daytime hours in one block, 4
-                                      hours per pass (1 m walk, no water); 0: one launch slice
-                                      per hour everywhere */
+    int32_t gvf_hours;             /* 1: GVF by walk words, four daytime hours per block of a
+                                      32x32 tile (walks of 2 to 22 steps with first_steps 1,
+                                      no water); 0: one launch slice per hour everywhere */
     int32_t no_ceiling;            /* 0: the sweep stops on the per-hour ray ceilings
                                       (same results, fewer steps); 1: every ray walks
                                       to its global clearance */

@@ -2,10 +2,11 @@
 
 All hours of a day are planned on the host first (FP64 solar geometry,
 Perez luminance, patch weights, sun rays: ``engine.plan_day``), written into
-pinned memory and replayed as one captured graph: the hour-record and ray uploads, the state
-reset and the 2 kernels of every hour (``solweig_day``).  The graph is
-captured once per scene and replays for any forcing of the same length,
-because every kernel reads its hour record from device memory.
+pinned memory and replayed as one captured graph: the hour-record and ray
+uploads, the state reset and the three kernels of every hour (``solweig_day``),
+or the few launches of the whole day (:class:`ChosenDay`).  The graph is
+captured once per scene, on its second day, and replays for any forcing of the
+same length, because every kernel reads its hour record from device memory.
 """
 from __future__ import annotations
 
@@ -283,20 +284,21 @@ class ChosenDay(BatchedDay):
     def stage_bytes(pixels, hours, day_hours):
         """Algorithmic HBM bytes of each stage of one day.
 
-        shadow (with the ray ceilings): per daytime pixel-hour 16 B packed
-        geometry read and a 4 B ceiling written and read back, 40 B float64
-        geometry + 1 B flags + 20 B float32 fields read, 16 B quad written
-        (101 B); GVF: 16 B quad + 4 B face
-        bits + 4 B emissivity read, 3 planes + the albedo-without-shadow plane
-        written (40 B); tables: per-hour tables (negligible); contraction: 40 B
+        shadow (with the ray ceilings): per daytime pixel-hour 4 B of the plane
+        of heights and the pixel's own 16 B sample read, 8 B ceiling and window
+        maximum written and read back, 8 B wall height + 1 B flags + 20 B
+        float32 fields read, 16 B quad written (81 B); GVF (walk words): 16 B
+        quad + 4 B emissivity read, a quarter of 4 B codes written and read
+        back and of 72 B words read, 3 planes written (52 B) and the
+        albedo-without-shadow plane once; tables: per-hour tables (negligible); contraction: 40 B
         of mask words per pixel read, 2 sums per pixel-hour written (8 B: sky
         plus transmitted vegetation, luminance and luminance*cos*omega);
         radiation: 109 B of per-pixel statics and 16 B of state per day, 20 B
         per daytime pixel-hour (3 GVF planes, 2 sums) and 8 B per pixel-hour
         written (Tmrt, UTCI)."""
         return {
-            "day_shadow_kernel": pixels * day_hours * 101,
-            "day_gvf_kernel": pixels * day_hours * 40,
+            "day_shadow_kernel": pixels * day_hours * 81,
+            "day_gvf_kernel": pixels * (52 * day_hours + 4),
             "day_tables_kernel": hours * 9680,
             "patch_gemm_kernel": pixels * (40 + 8 * hours),
             "day_radiation_kernel": pixels * (125 + 20 * day_hours + 8 * hours),

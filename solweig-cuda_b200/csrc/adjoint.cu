@@ -91,7 +91,6 @@ __global__ void param_quads_kernel(SolweigScene S, const SolweigHour* __restrict
     if (!h.daytime) return;
     const float4 q = q0[idx];
     const float s0 = q.x;
-    const float psi = (float)h.psi;
     if (*error) {  // a ray longer than the sweep's records: no result rather than a wrong one
         const float nan = __int_as_float(0x7fffffff);
         sv[idx] = 0;
@@ -104,7 +103,6 @@ __global__ void param_quads_kernel(SolweigScene S, const SolweigHour* __restrict
     else if (s0 == 0.0f) { sh = 0; vegsh = 1; }
     else if (s0 == (float)(1.0 - (1.0 - h.psi))) { sh = 1; vegsh = 0; }
     else { sh = 0; vegsh = 0; }
-    (void)psi;
     sv[idx] = (uint8_t)(sh | (vegsh << 1));
     const double t = tau[p];
     const double shadow = (double)(float)((double)sh - (1.0 - vegsh) * (1.0 - t));

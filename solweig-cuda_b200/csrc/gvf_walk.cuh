@@ -9,14 +9,18 @@
 //
 // A sample is the pair (Lup, albedo * shadow).  Both come from a few land-cover
 // classes and shadow values, so within a tile an hour has few distinct pairs
-// (six for two ground classes under sun, building and tree shadow), whatever
-// the rasters hold elsewhere.  With at most kWkValues of them the walk counts
+// (five for two ground classes: each in the sun and under trees, and (0, 0) in
+// a building's shadow), whatever the rasters hold elsewhere.  With at most kWkValues of them the walk counts
 // instead of adding: a sample is one 32-bit word with a one in the 5-bit field
 // of its value (a walk has at most 22 samples), four hours are one 16-byte
 // load and four integer additions, and the counts meet the values once per
 // pixel and hour.  That halves the shared-memory traffic that bounds the walk
 // (4 instead of 8 bytes per sample and hour) and leaves nothing to round until
-// the end.  A tile with more values adds the pairs, two hours at a time.
+// the end.  A tile with more values (three ground classes give seven) adds the
+// pairs, two hours at a time: 2000 x 2000 px with two classes 3.56 ms a day, with
+// three 6.50, with an albedo of its own per pixel 7.08, where one thread per pixel
+// adding the pairs of four hours took 6.70 whatever the values; 500 x 500 px at
+// 2 m 0.24, 0.41 and 0.47 against 1.18 ms.
 // gvf_codes_kernel finds each tile's values and writes the number of every
 // sample's value once; a tile's walk merges its own and its neighbours' values
 // and stages 4 bytes per pixel and pass instead of the four 16-byte quads

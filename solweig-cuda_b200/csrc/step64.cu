@@ -23,7 +23,12 @@
 // fewer roundings than they replace: the steps after a walk's end, which all
 // add the same, come as one product, and sums of solid-angle weights over a
 // set of patches, equal within an altitude band, are band counts times the
-// band's weight.  This file is compiled with --fmad=false (as the reference
+// band's weight.  The means over a walk's steps are products with rounded
+// reciprocals (true divisions: 2.00 instead of 1.67 ms per day of 300 x 280 px).
+// Against longer precision the sum of a pixel's 18 walks has an rms error of 1.05
+// to 1.15e-16 for 22 steps (1.13 to 1.78e-16 with one addition per step and
+// divisions), 1.08 to 1.15 for 11 steps (1.06 to 1.15), 1.08 to 1.16 for 6 (1.04
+// to 1.15).  This file is compiled with --fmad=false (as the reference
 // compiles its kernels, src/runtime.py:11), so no multiply-add is contracted.
 // UTCI is evaluated from the float32-rounded Tmrt and air temperature, as
 // utci_calculator casts its inputs (src/utci.py:8-12).
