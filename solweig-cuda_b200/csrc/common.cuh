@@ -39,6 +39,14 @@ inline unsigned blocks_for(long long n, int threads) {
     return static_cast<unsigned>((n + threads - 1) / threads);
 }
 
+// Lets a kernel without static shared memory take any dynamic size.  The limit
+// belongs to the kernel and is shared by all threads: a launch's own size, set by
+// one thread between another's setting and its launch, fails that launch when it
+// is smaller ("invalid argument"), so it is always the largest.
+inline void allow_shared(const void* kernel) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+}
+
 // Steps covered by the window maximum of the ray-ceiling planes (ceiling.cuh):
 // a walk may skip that many steps at once on it (shadow.cuh).
 constexpr int kCeilSkip = 8;

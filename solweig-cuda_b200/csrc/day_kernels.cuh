@@ -1053,6 +1053,7 @@ DayWork day_work_layout(int rows, int cols, int nhours, bool water) {
     return w;
 }
 
+// For kernels that always take the same size (allow_shared for the others).
 void set_smem_attr(const void* kernel, size_t bytes) {
     // Not a stream operation; cheap after the first call.
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
@@ -1100,7 +1101,7 @@ int launch_day_walk(const SolweigScene& S, const SolweigHour* hours, int nhours,
                                                       nosh);
     SOLWEIG_CHECK_LAUNCH("gvf_codes_kernel");
     const size_t smem = day_walk_smem_bytes(wa.width);
-    set_smem_attr((const void*)day_gvf_walk_kernel, smem);
+    allow_shared((const void*)day_gvf_walk_kernel);
     day_gvf_walk_kernel<<<grid, kWkThreads, smem, st>>>(S, hours, nhours, wa, quads, gvf);
     SOLWEIG_CHECK_LAUNCH("day_gvf_walk_kernel");
     return SOLWEIG_OK;
@@ -1114,11 +1115,11 @@ void launch_day_gvf_ty(const SolweigScene& S, const SolweigHour* hours, int nhou
     dim3 grid(blocks_for(S.cols, 32), blocks_for(S.rows, TY), nhours);
     if (S.has_water) {
         auto k = day_gvf_kernel<TY, FIRST, SECOND, TABLE, true>;
-        set_smem_attr((const void*)k, smem);
+        allow_shared((const void*)k);
         k<<<grid, dim3(32, TY), smem, st>>>(S, hours, ga, tab, quads, lup_first, gvf, nosh);
     } else {
         auto k = day_gvf_kernel<TY, FIRST, SECOND, TABLE, false>;
-        set_smem_attr((const void*)k, smem);
+        allow_shared((const void*)k);
         k<<<grid, dim3(32, TY), smem, st>>>(S, hours, ga, tab, quads, lup_first, gvf, nosh);
     }
 }
@@ -1137,7 +1138,7 @@ int launch_gemm(const uint32_t* masks, long long px, int patches, const __nv_bfl
     if (combined && gemm_pipe_smem_bytes(nb) <= 227 * 1024) {
         // the pipelined kernel: one CTA per SM (its shared memory)
         const size_t smem = gemm_pipe_smem_bytes(nb);
-        set_smem_attr((const void*)patch_gemm_pipe_kernel, smem);
+        allow_shared((const void*)patch_gemm_pipe_kernel);
         int dev = 0, sms = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1152,7 +1153,7 @@ int launch_gemm(const uint32_t* masks, long long px, int patches, const __nv_bfl
     const size_t smem = gemm_smem_bytes(nb, combined);
     SOLWEIG_CHECK_ARG(smem <= 227 * 1024, "patch contraction: %d weight columns need %zu bytes of shared memory",
                       ncols, smem);
-    set_smem_attr((const void*)patch_gemm_kernel, smem);
+    allow_shared((const void*)patch_gemm_kernel);
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -94,7 +94,7 @@ extern "C" int solweig_gvf(const SolweigScene* scene, const float* shadow, const
     gs.first = first_steps;
     gs.second = second_steps;
     dim3 block(kGvfBX, kGvfBY), grid(blocks_for(S.cols, kGvfBX), blocks_for(S.rows, kGvfBY));
-    cudaFuncSetAttribute(gvf_planes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_shared((const void*)gvf_planes_kernel);
     gvf_planes_kernel<<<grid, block, smem, st>>>(quad, lup_first, S.gvf_face, S.emis, S.rows, S.cols,
                                                  reinterpret_cast<const int2*>(gvf_dxdy), gs,
                                                  S.has_water, ta, planes);

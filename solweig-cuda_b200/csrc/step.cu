@@ -320,27 +320,6 @@ static int check_scene(const SolweigScene* S) {
     return SOLWEIG_OK;
 }
 
-static void set_smem_once(const void* kernel, size_t bytes) {
-    // cudaFuncSetAttribute is not a stream operation; remember the largest
-    // size set per kernel so steady-state launches (and graph capture) skip it.
-    static thread_local const void* which[32] = {};
-    static thread_local size_t done[32] = {};
-    int slot = -1;
-    for (int i = 0; i < 32; ++i) {
-        if (which[i] == kernel) {
-            if (done[i] >= bytes) return;
-            slot = i;
-            break;
-        }
-        if (!which[i] && slot < 0) slot = i;
-    }
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (slot >= 0) {
-        which[slot] = kernel;
-        done[slot] = bytes;
-    }
-}
-
 extern "C" int solweig_step_shadow(const SolweigScene* scene, const SolweigHour* hours, int hour,
                                    float* scratch, void* stream) {
     int rc = check_scene(scene);
@@ -369,12 +348,12 @@ static void launch_gvf(const SolweigScene& S, const SolweigHour* hours, int hour
     dim3 grid(blocks_for(S.cols, 32), blocks_for(S.rows, TY));
     if (S.has_water) {
         auto k = step_gvf_kernel<TY, FIRST, SECOND, TABLE, true>;
-        set_smem_once((const void*)k, smem);
+        allow_shared((const void*)k);
         k<<<grid, dim3(32, TY), smem, st>>>(S, hours, hour, ga, tab, scratch_quad(scratch), lup_first,
                                             scratch_gvf(scratch, n));
     } else {
         auto k = step_gvf_kernel<TY, FIRST, SECOND, TABLE, false>;
-        set_smem_once((const void*)k, smem);
+        allow_shared((const void*)k);
         k<<<grid, dim3(32, TY), smem, st>>>(S, hours, hour, ga, tab, scratch_quad(scratch), lup_first,
                                             scratch_gvf(scratch, n));
     }
